@@ -81,7 +81,7 @@ int Ctx::tune_batch(const BatchLaunch& base, int n, size_t total_px, uint64_t ke
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const int occ = half_sweep_batch_occupancy(base.max_s, base.mand);
-    const int bt = half_sweep_block_threads(base.max_s);
+    const int bt = half_sweep_block_threads();
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     int rc = HPM_OK;
     BatchShape best;
@@ -218,6 +218,12 @@ int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int
         if (rc) return rc;
         off += (size_t)views[r].w * views[r].h;
     }
+    if ((e = ensure_dev(b_weights, b_weights_cap, (size_t)n * kWeightTable)) != cudaSuccess)
+        return cuda_fail(e, "alloc weight tables");
+    for (int k = 0; k < n; ++k) {
+        const int rc = take_whole_levels(refs[k], src_ids + src_off[k], b_weights + (size_t)k * kWeightTable, h_bargs[k]);
+        if (rc) return rc;
+    }
 
     // prior mode: work lists of every run (confidences and prior masks are fixed during the pass and the
     // initialisation does not change them), computed before the launches that a graph may replay
@@ -240,7 +246,7 @@ int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int
     }
 
     // tile tables: initialisation (16 x 8 pixel blocks), then the half-sweep's
-    const int bt = half_sweep_block_threads(max_s);
+    const int bt = half_sweep_block_threads();
     const uint64_t key = (uint64_t)max_s | ((uint64_t)mand << 8) |
                          ((uint64_t)(total ? (int)std::log2((double)total) : 0) << 16);
     BatchShape shape;
@@ -327,7 +333,7 @@ int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int
     if (use_graph && have_shape && !shape.perview)
         for (auto& g : batch_graphs)
             if (g.n == n && g.init_tiles == bi.tiles && g.sweep_tiles == bs.tiles && g.max_s == max_s &&
-                g.mand == mand && g.iters == iters && g.bx == bs.bx && g.grid == bs.grid_blocks &&
+                g.mand == mand && g.listed == listed && g.iters == iters && g.bx == bs.bx && g.grid == bs.grid_blocks &&
                 g.perview == shape.perview)
                 graph = &g;
     if (graph) {
@@ -368,6 +374,7 @@ int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int
             if (e != cudaSuccess) return cuda_fail(e, "batch graph instantiate");
             BatchGraph bg;
             bg.n = n; bg.init_tiles = bi.tiles; bg.sweep_tiles = bs.tiles; bg.max_s = max_s; bg.mand = mand;
+            bg.listed = listed;
             bg.iters = iters; bg.bx = bs.bx; bg.grid = bs.grid_blocks; bg.perview = shape.perview; bg.exec = ex;
             batch_graphs.push_back(bg);
         }

@@ -57,13 +57,19 @@ cudaError_t Ctx::ensure_map(int view, int kind, int w, int h) {
 }
 
 cudaError_t Ctx::ensure_run(size_t n) {
-    cudaError_t e;
-    if ((e = ensure(planes, run_cap_planes, n)) != cudaSuccess) return e;
-    if ((e = ensure(costs, run_cap_costs, n)) != cudaSuccess) return e;
-    if ((e = ensure(pre_costs, run_cap_pre, n)) != cudaSuccess) return e;
-    if ((e = ensure(sel, run_cap_sel, n)) != cudaSuccess) return e;
-    if ((e = ensure(rng, run_cap_rng, n)) != cudaSuccess) return e;
-    if ((e = ensure(conf, run_cap_conf, n)) != cudaSuccess) return e;
+    if (n <= run_px && run_mem) return cudaSuccess;
+    const size_t px = (n + 63) & ~size_t(63);  // every part starts on a 256-byte boundary
+    run_px = 0;
+    cudaError_t e = ensure(run_mem, run_mem_cap, px * (sizeof(float4) + 5 * 4) + kWeightTable * sizeof(float));
+    if (e != cudaSuccess) return e;
+    planes = reinterpret_cast<float4*>(run_mem);
+    costs = reinterpret_cast<float*>(planes + px);
+    pre_costs = costs + px;
+    sel = reinterpret_cast<uint32_t*>(pre_costs + px);
+    rng = sel + px;
+    conf = reinterpret_cast<float*>(rng + px);
+    weights = conf + px;
+    run_px = n;
     return cudaSuccess;
 }
 
@@ -71,6 +77,9 @@ Ctx::~Ctx() {
     for (auto& v : views) {
         if (v.tex) cudaDestroyTextureObject(v.tex);
         if (v.arr) cudaFreeArray(v.arr);
+        if (v.bytes) cudaFree(v.bytes);
+        if (v.tex8) cudaDestroyTextureObject(v.tex8);
+        if (v.arr8) cudaFreeArray(v.arr8);
         if (v.gray) cudaFree(v.gray);
         for (auto& m : v.maps) if (m.ptr) cudaFree(m.ptr);
         if (v.canny) cudaFree(v.canny);
@@ -82,11 +91,11 @@ Ctx::~Ctx() {
     for (auto& g : batch_graphs)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     for (void* p : { (void*)b_planes, (void*)b_costs, (void*)b_pre, (void*)b_sel, (void*)b_rng, (void*)b_conf,
-                     (void*)b_scaled, (void*)d_bargs, (void*)d_btiles })
+                     (void*)b_scaled, (void*)b_weights, (void*)d_bargs, (void*)d_btiles })
         if (p) cudaFree(p);
     if (h_bargs) cudaFreeHost(h_bargs);
     if (h_btiles) cudaFreeHost(h_btiles);
-    for (void* p : { (void*)planes, (void*)costs, (void*)pre_costs, (void*)sel, (void*)rng, (void*)conf,
+    for (void* p : { (void*)run_mem,
                      (void*)active_px, (void*)active_n, (void*)b_active,
                      (void*)scaled, (void*)scratch, (void*)scan_state, (void*)scan_work, (void*)points,
                      (void*)prior_small, (void*)prior_tris, (void*)prior_label, (void*)prior_work,
@@ -98,6 +107,7 @@ Ctx::~Ctx() {
     }
     if (prof_hyp) cudaFree(prof_hyp);
     if (half_stage) cudaFree(half_stage);
+    if (level_flags) cudaFree(level_flags);
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -221,6 +231,7 @@ int hpm_set_view(hpm_ctx* ctx, int view, const float* gray, int w, int h, const 
     if (e != cudaSuccess) return c->cuda_fail(e, "alloc grey image");
     e = cudaMemcpyAsync(v.gray, gray, sizeof(float) * w * h, cudaMemcpyHostToDevice, c->stream);
     if (e != cudaSuccess) return c->cuda_fail(e, "upload grey image");
+    v.whole_levels = -1;
     v.w = w; v.h = h; v.cam = *cam;
     v.cam.width = w; v.cam.height = h;
     return c->bind_texture(view);

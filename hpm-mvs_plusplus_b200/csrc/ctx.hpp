@@ -29,9 +29,17 @@ struct ViewState {
     hpm_camera cam{};
     float* gray = nullptr;
     size_t gray_cap = 0;
+    int whole_levels = 0;  // the grey image holds whole levels 0..255 only (-1: not looked at yet)
     cudaArray_t arr = nullptr;
     cudaTextureObject_t tex = 0;
     int arr_w = 0, arr_h = 0, arr_mode = -1, arr_fmt = -1;
+    uint8_t* bytes = nullptr;  // an image of whole levels as bytes (whole_levels == 1)
+    size_t bytes_cap = 0;
+    // 8-bit texture of an F32 image of whole levels, which the half-sweeps sample (Ctx::bind_bytes)
+    cudaArray_t arr8 = nullptr;
+    cudaTextureObject_t tex8 = 0;
+    int arr8_w = 0, arr8_h = 0, arr8_mode = -1;
+    bool bytes_bound = false;  // tex8 holds the current image
     DevMap maps[kNumMaps];
     uint8_t* canny = nullptr;
     size_t canny_cap = 0;
@@ -81,16 +89,22 @@ struct Ctx {
     int addr_mode = 0;
     int tex_format = 0;  // HPM_TEX_F32, HPM_TEX_F16 or HPM_TEX_U8: texel type of the source-image textures
     int ncc_mode = 0;    // HPM_NCC_PLAIN or HPM_NCC_SHIFTED
+    int* level_flags = nullptr; size_t level_flags_cap = 0;  // per view, results of k_whole_levels
     uint16_t* half_stage = nullptr; size_t half_stage_cap = 0;
     int64_t launches = 0;
 
     // work buffers of one PatchMatch run (sized for the largest reference view)
-    float4* planes = nullptr; size_t run_cap_planes = 0;
-    float* costs = nullptr; size_t run_cap_costs = 0;
-    float* pre_costs = nullptr; size_t run_cap_pre = 0;
-    uint32_t* sel = nullptr; size_t run_cap_sel = 0;
-    uint32_t* rng = nullptr; size_t run_cap_rng = 0;
-    float* conf = nullptr; size_t run_cap_conf = 0;
+    // (one allocation, carved by ensure_run)
+    uint8_t* run_mem = nullptr; size_t run_mem_cap = 0;
+    size_t run_px = 0;
+    float4* planes = nullptr;
+    float* costs = nullptr;
+    float* pre_costs = nullptr;
+    uint32_t* sel = nullptr;
+    uint32_t* rng = nullptr;
+    float* conf = nullptr;
+    float* weights = nullptr;                            // bilateral weights of whole-level references
+    float* b_weights = nullptr; size_t b_weights_cap = 0;
     int* active_px = nullptr; size_t active_px_cap = 0;  // prior-mode compaction (k_prior_active)
     int* active_n = nullptr; size_t active_n_cap = 0;
     int* b_active = nullptr; size_t b_active_cap = 0;    // the same for every run of a prior-mode batch
@@ -126,7 +140,7 @@ struct Ctx {
     std::vector<std::pair<uint64_t, BatchShape>> batch_shapes;  // autotuner cache: key -> shape
     struct BatchGraph {
         int n = 0, init_tiles = 0, sweep_tiles = 0, max_s = 0, iters = 0, bx = 0, grid = 0;
-        bool mand = false, perview = false;
+        bool mand = false, perview = false, listed = false;
         cudaGraphExec_t exec = nullptr;
     };
     std::vector<BatchGraph> batch_graphs;
@@ -147,6 +161,9 @@ struct Ctx {
     cudaError_t ensure_map(int view, int kind, int w, int h);
     cudaError_t ensure_run(size_t n);
     int bind_texture(int view);
+    int bind_bytes(int view);
+    int take_whole_levels(int ref, const int32_t* srcs, float* weights, RunArgs& a);
+    int look_at_levels(int ref, const int32_t* srcs, int n_src);
     int fill_run_args(int ref, const int32_t* srcs, int n_src, const hpm_params* params, RunArgs& a);
     int prepare_run(int ref, const int32_t* srcs, int n_src, const hpm_params* params, int texture_level,
                     uint64_t seed, RunArgs& a);

@@ -19,24 +19,35 @@ constexpr int kPatchRadius = 5;
 constexpr int kPatchStep = 2;
 constexpr int kMarsagliaMaxTries = 4096;
 
+// Code size.  The half-sweep's NCC is some 13 KB of straight-line code (its patch lives in registers),
+// and the warps of an SM stand at different places of the kernel: everything around the NCC that is
+// inlined or unrolled adds to what they fetch from the instruction caches.  The parts that run once a
+// pixel are therefore loops and calls, not copies.
+
+// One block of the pixel's random stream, out of line.
+static __device__ __noinline__ uint4 philox_block(uint64_t seed, uint32_t view, uint32_t x, uint32_t y, uint32_t b) {
+    hpm_u32x4 c;
+    c.v[0] = b; c.v[1] = x; c.v[2] = y; c.v[3] = view;
+    const hpm_u32x4 r = hpm_philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
+    return make_uint4(r.v[0], r.v[1], r.v[2], r.v[3]);
+}
+
 struct PixelRng {
     uint64_t seed;
     uint32_t view, x, y, draw;
     uint32_t block_id;  // draw >> 2 of the cached block, or 0xffffffff
-    uint32_t w[4];
+    uint4 w;
     __device__ __forceinline__ void init(uint64_t s, uint32_t v, uint32_t px, uint32_t py, uint32_t d) {
         seed = s; view = v; x = px; y = py; draw = d; block_id = 0xffffffffu;
     }
     __device__ __forceinline__ float uniform() {
         const uint32_t b = draw >> 2;
         if (b != block_id) {
-            hpm_u32x4 c;
-            c.v[0] = b; c.v[1] = x; c.v[2] = y; c.v[3] = view;
-            const hpm_u32x4 r = hpm_philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
-            w[0] = r.v[0]; w[1] = r.v[1]; w[2] = r.v[2]; w[3] = r.v[3];
+            w = philox_block(seed, view, x, y, b);
             block_id = b;
         }
-        const uint32_t bits = w[draw & 3u];
+        const uint32_t k = draw & 3u;
+        const uint32_t bits = k < 2 ? (k == 0 ? w.x : w.y) : (k == 2 ? w.z : w.w);
         ++draw;
         return hpm_bits_to_uniform(bits);
     }
@@ -85,7 +96,7 @@ __device__ __forceinline__ void normalize3(float4& v) {
     v.x *= inv; v.y *= inv; v.z *= inv;
 }
 
-__device__ __forceinline__ float4 random_normal(const hpm_camera& c, int px, int py, PixelRng& rng, float depth) {
+static __device__ __noinline__ float4 random_normal(const hpm_camera& c, int px, int py, PixelRng& rng, float depth) {
     float q1 = 1.0f, q2 = 1.0f, s = 2.0f;
     int tries = 0;
     while (s >= 1.0f && tries < kMarsagliaMaxTries) {
@@ -103,7 +114,7 @@ __device__ __forceinline__ float4 random_normal(const hpm_camera& c, int px, int
     return n;
 }
 
-__device__ __forceinline__ float4 perturbed_normal(const hpm_camera& c, int px, int py, float4 normal,
+static __device__ __noinline__ float4 perturbed_normal(const hpm_camera& c, int px, int py, float4 normal,
                                                    PixelRng& rng, float perturbation) {
     const float4 vd = view_direction(c, px, py, 1.0f);
     const float a1 = (rng.uniform() - 0.5f) * perturbation;
@@ -131,15 +142,19 @@ __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? l
 // clamped point fetch at (int)x, (int)y) and carried back; the cost is the
 // reprojection distance, at most 3.  The two transfers use the per-view bases
 // of hpm_view_transfer (include/hpm_geometry.h).
-__device__ __forceinline__ float geom_cost(const float* __restrict__ sdepth, int sw, int sh, const float* Gf,
-                                           const float* gf, const float* Gb, const float* gb, float depth, int px,
-                                           int py) {
-    const float max_cost = 3.0f;
-    float sx, sy;
+// In two parts, so that a caller can have several gathers of the first in flight.
+__device__ __forceinline__ float geom_source_depth(const float* __restrict__ sdepth, int sw, int sh, const float* Gf,
+                                                   const float* gf, float depth, int px, int py, float& sx,
+                                                   float& sy) {
     hpm_transfer(Gf, gf, (float)px, (float)py, depth, &sx, &sy);
     const int ix = clampi(__float2int_rz(sx), 0, sw - 1);
     const int iy = clampi(__float2int_rz(sy), 0, sh - 1);
-    const float d = __ldg(sdepth + (size_t)iy * sw + ix);
+    return __ldg(sdepth + (size_t)iy * sw + ix);
+}
+
+__device__ __forceinline__ float geom_back_cost(const float* Gb, const float* gb, float sx, float sy, float d, int px,
+                                                int py) {
+    const float max_cost = 3.0f;
     if (d == 0.0f) return max_cost;
     float bx, by;
     hpm_transfer(Gb, gb, sx, sy, d, &bx, &by);
@@ -149,9 +164,9 @@ __device__ __forceinline__ float geom_cost(const float* __restrict__ sdepth, int
 
 // Edge-density texture term (HPM.cu:349-373); the ratio is evaluated in double
 // as in the reference (double literals).
-__device__ __forceinline__ float texture_term(const uint8_t* __restrict__ canny, int W, int H, int px, int py) {
+static __device__ __noinline__ float texture_term(const uint8_t* __restrict__ canny, int W, int H, int px, int py) {
     int total = 0, edges = 0;
-#pragma unroll
+#pragma unroll 1
     for (int i = -5; i < 6; i += 2)
 #pragma unroll
         for (int j = -5; j < 6; j += 2) {

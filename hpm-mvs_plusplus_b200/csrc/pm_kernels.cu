@@ -5,16 +5,35 @@
 // Algorithm: HPM-MVS++ HPM.cu:567-842 (init, refinement), 843-1873 (standard
 // propagation), 1875-2791 (mandatory consistency), 2793-2842 (schedule,
 // export).  The kernels are laid out differently:
-//   * one thread per pixel of the active colour, block 32 x (BLK/32) over
-//     (x, row pair) so a warp covers a 32 x 2 strip (coherent texture reads);
+//   * one thread per pixel of the active colour, block 32 x 4 over (x, row
+//     pair) so a warp covers a 32 x 2 strip (coherent texture reads);
 //   * the pixel's reference patch (weights and weighted texels) lives in
 //     registers and is built once per launch instead of once per NCC;
-//   * per-pixel cost rows, view weights, final costs and positions live in a
-//     per-thread column of shared memory (stride BLK, conflict-free);
+//   * images of whole grey levels are sampled from 8-bit textures with the same
+//     bits as float ones (Ctx::bind_bytes), and their weights come from a table;
 //   * NCCs whose view weight is zero are not evaluated (their product with the
 //     zero weight is exactly 0 because the NCC is never NaN), and a reference
 //     patch with variance < 1e-5 yields cost 2 for every hypothesis without
-//     sampling (exactly the reference's result).
+//     sampling (exactly the reference's result);
+//   * a refinement candidate is dropped at the view where its partial cost
+//     already rules it out.
+//
+// What bounds a half-sweep.  Three things compete on an SM: the texture data
+// pipe (36 fetches per NCC; a quad of lanes that samples apart takes up to four
+// passes), instruction fetch (the NCC is straight-line code, since its patch is
+// in registers, and the warps stand at different places), and the latency of
+// the serial parts around the NCCs.  Six half-sweeps of one run, ms, S = 10,
+// before and after each change, all with the same bits:
+//   code size 291 -> 105 KB (loops and calls outside the NCC):
+//                      1600x1200 mandatory 48.5 -> 42.0, prior 31.2 -> 22.8
+//   8-bit textures:    800x600 photometric 13.4 -> 11.0 (2.2 -> 1.4 passes a quad)
+//   pairs of samples in one instruction (f32x2):  mandatory 42.0 -> 39.0
+//   weight table, candidate planes gathered at once:  mandatory 39.0 -> 37.5
+//   candidates dropped early:  800x600 photometric 11.4 -> 11.0
+//   the next 12 fetches issued before these are summed:  mandatory 37.3 -> 36.2
+// Twelve warps per SM at 168 registers and sixteen at 128 (texels of the patch
+// packed in bytes) ran alike; eight at 220 registers were 15-25 % slower, and
+// blocks of 64 threads up to 15 % slower while the code was large.
 // Arithmetic follows include/hpm_fp.h (IEEE fp32, explicit fused multiply-adds),
 // which the CPU oracle shares, so the two differ only where the texture unit's
 // filtered sample does (about 0.6 % of samples, by one ulp).
@@ -26,20 +45,45 @@
 namespace hpm {
 
 
-// CNT: the counting build of a kernel (profiling); the timed build has it off
-// so the counters do not change its code.
-template <int NS, int BLK, bool CNT = false>
-struct Scratch {
+// Per-thread columns of shared memory of the initialisation: the costs of one
+// hypothesis by view, and the same sorted.
+template <int NS, int BLK>
+struct InitScratch {
     float* base;  // smem + threadIdx linear
-    static constexpr bool kCount = CNT;
-    // cost rows 0-7 (directions), row 8 (the hypothesis costed against the
-    // selected views), view weights, final costs, candidate positions
-    static constexpr int kWords = 10 * NS + 16;
+    static constexpr int kWords = 2 * NS;
     __device__ __forceinline__ float& ca(int d, int j) const { return base[(d * NS + j) * BLK]; }
-    __device__ __forceinline__ float& vw(int j) const { return base[(9 * NS + j) * BLK]; }
-    __device__ __forceinline__ float& fc(int d) const { return base[(10 * NS + d) * BLK]; }
-    __device__ __forceinline__ int& pos(int d) const { return reinterpret_cast<int*>(base)[(10 * NS + 8 + d) * BLK]; }
 };
+
+// Per-thread scratch of a half-sweep.  The cost rows of the eight directions are written once, an NCC
+// apart, and read once, by view selection: they stream through the thread's local memory, so that
+// shared memory (view weights, final costs, candidate positions) leaves the L1 to the textures and
+// the registers alone bound the resident warps.  After view selection the rows' words hold the
+// refinement's candidates and the state they are tested against, which would otherwise sit in
+// registers across every NCC.
+template <int NS, int BLK>
+struct Scratch {
+    float* base;   // smem + threadIdx linear
+    float* rows;   // local memory, kRowWords
+    float4* cand;  // local memory: plane_m of the eight directions' planes and their depth at the pixel
+    static constexpr int kWords = NS + 16;
+    static constexpr int kRowWords = 8 * NS < 72 ? 72 : 8 * NS;  // at least a patch's texels and weights
+    __device__ __forceinline__ float& ca(int d, int j) const { return rows[d * NS + j]; }
+    __device__ __forceinline__ float4 held(int i) const {
+        return make_float4(rows[4 * i], rows[4 * i + 1], rows[4 * i + 2], rows[4 * i + 3]);
+    }
+    __device__ __forceinline__ void hold(int i, float4 v) const {
+        rows[4 * i] = v.x; rows[4 * i + 1] = v.y; rows[4 * i + 2] = v.z; rows[4 * i + 3] = v.w;
+    }
+    __device__ __forceinline__ float& vw(int j) const { return base[j * BLK]; }
+    __device__ __forceinline__ float& fc(int d) const { return base[(NS + d) * BLK]; }
+    __device__ __forceinline__ int& pos(int d) const { return reinterpret_cast<int*>(base)[(NS + 8 + d) * BLK]; }
+};
+
+constexpr int kWeightRows = 6;
+static_assert(kWeightRows * 256 == kWeightTable, "RunArgs::weights");
+
+constexpr int kSweepThreads = 128;
+constexpr int kSweepBlocks = 3;  // resident blocks per SM: at most 168 registers a thread
 
 // Statistics of a pixel's reference patch (the view-independent part of the NCC).
 struct RefStats {
@@ -48,39 +92,135 @@ struct RefStats {
     float inv_w;  // 1 / weight_sum
 };
 
+// Two floats in a register pair; one instruction works on both, each rounded as the scalar one.  The
+// NCC takes two patch columns at a time, whose sums are separate, so pairing them changes no order.
+using Pair = unsigned long long;
+
+__device__ __forceinline__ Pair pair_of(float lo, float hi) {
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 halves(Pair a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ Pair add2(Pair a, Pair b) {
+    Pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// A pixel's reference patch in registers: the bilateral weights w_k and the weighted texels w_k r_k of
+// samples k = 6 i + j (column-major), those of columns i and i + 1 (i even) in row j as a pair.
 struct Patch {
-    float2 p[kPatchSamples];  // (w_k, w_k * r_k)
+    Pair w[kPatchSamples / 2], wr[kPatchSamples / 2];
     RefStats rs;
+    __device__ __forceinline__ Pair w2(int i, int j) const { return w[3 * i + j]; }
+    __device__ __forceinline__ Pair wr2(int i, int j) const { return wr[3 * i + j]; }
 };
 
-__device__ __forceinline__ void build_patch(const RunArgs& a, int px, int py, Patch& P) {
-    const float* __restrict__ ref = a.ref_img;
+// The bilateral weight of a patch texel |dx|, |dy| = 5, 3 or 1 away and `d` grey levels off the centre.
+__device__ __forceinline__ float bilateral_weight(int dx, int dy, float d, float two_ss, float two_sc) {
+    const float sd = sqrtf((float)(dx * dx + dy * dy));
+    return hpm_expf(-sd / two_ss - d / two_sc);
+}
+
+// Rows of the weight table: the six distances of a patch sample, by (|dx|, |dy|) in either order.
+__host__ __device__ constexpr int weight_row(int dx, int dy) {
+    const int a = dx < 0 ? -dx : dx, b = dy < 0 ? -dy : dy;
+    const int hi = a > b ? a : b, lo = a > b ? b : a;
+    return hi == 5 ? (lo - 1) / 2 + 3 : (hi == 3 ? (lo - 1) / 2 + 1 : 0);
+}
+
+#ifndef HPM_NS
+// The weights of a reference of whole levels: kWeightRows x 256 values, one per distance and level
+// difference (RunArgs::weights).
+__global__ void k_weight_table(float two_ss, float two_sc, float* __restrict__ out) {
+    const int row = blockIdx.x, d = threadIdx.x;
+    const int hi = row < 1 ? 1 : (row < 3 ? 3 : 5), lo = row < 1 ? 1 : (row < 3 ? 2 * (row - 1) + 1 : 2 * (row - 3) + 1);
+    out[row * 256 + d] = bilateral_weight(hi, lo, (float)d, two_ss, two_sc);
+}
+#endif
+
+// The patch in two ways with the same bits.  A reference of whole levels reads bytes and takes its
+// weights from the table: 36 loads of each, all in flight, instead of 36 exponentials and 72 divisions.
+// Any other forms the weights in a loop, through kPatchWords words of the thread's local memory.
+constexpr int kPatchWords = 2 * kPatchSamples;
+
+__device__ __forceinline__ void build_patch(const RunArgs& a, int px, int py, Patch& P, float* tmp) {
     const int W = a.W, H = a.H;
-    const float center = __ldg(ref + (size_t)clampi(py, 0, H - 1) * W + clampi(px, 0, W - 1));
-    const float two_ss = 2.0f * a.prm.sigma_spatial * a.prm.sigma_spatial;
-    const float two_sc = 2.0f * a.prm.sigma_color * a.prm.sigma_color;
+    const int at = clampi(py, 0, H - 1) * W + clampi(px, 0, W - 1);
+    float r[kPatchSamples], w[kPatchSamples];
+    float center;
+    if (a.whole_levels) {
+        const int c = __ldg(a.ref_bytes + at);
+        center = (float)c;
+        int t[kPatchSamples];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+            const uint8_t* row = a.ref_bytes + (size_t)clampi(py - kPatchRadius + kPatchStep * j, 0, H - 1) * W;
+#pragma unroll
+            for (int i = 0; i < 6; ++i)
+                t[i * 6 + j] = __ldg(row + clampi(px - kPatchRadius + kPatchStep * i, 0, W - 1));
+        }
+#pragma unroll
+        for (int k = 0; k < kPatchSamples; ++k) {
+            const int dx = -kPatchRadius + kPatchStep * (k / 6), dy = -kPatchRadius + kPatchStep * (k % 6);
+            w[k] = __ldg(a.weights + weight_row(dx, dy) * 256 + abs(t[k] - c));
+            // a byte as the low mantissa bits of 2^23, less 2^23: exact
+            r[k] = __uint_as_float(0x4B000000u | (uint32_t)t[k]) - 8388608.0f;
+        }
+    } else {
+        center = __ldg(a.ref_img + at);
+        const float two_ss = 2.0f * a.prm.sigma_spatial * a.prm.sigma_spatial;
+        const float two_sc = 2.0f * a.prm.sigma_color * a.prm.sigma_color;
+#pragma unroll 1
+        for (int k = 0; k < kPatchSamples; ++k) {
+            const int dx = -kPatchRadius + kPatchStep * (k / 6), dy = -kPatchRadius + kPatchStep * (k % 6);
+            const float t = __ldg(a.ref_img + (size_t)clampi(py + dy, 0, H - 1) * W + clampi(px + dx, 0, W - 1));
+            tmp[k] = t;
+            tmp[kPatchSamples + k] = bilateral_weight(dx, dy, fabsf(t - center), two_ss, two_sc);
+        }
+#pragma unroll
+        for (int k = 0; k < kPatchSamples; ++k) {
+            r[k] = tmp[k];
+            w[k] = tmp[kPatchSamples + k];
+        }
+    }
     // shifted moments (precision form): the patch relative to its centre texel; shift 0 is the plain arithmetic
     const float cs = a.ncc_shift ? center : 0.0f;
     float s_r = 0.f, s_rr = 0.f, s_w = 0.f;
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
         float r_r = 0.f, r_rr = 0.f, r_w = 0.f;
-        const int dx = -kPatchRadius + kPatchStep * i;
-        const int x = clampi(px + dx, 0, W - 1);
 #pragma unroll
         for (int j = 0; j < 6; ++j) {
-            const int dy = -kPatchRadius + kPatchStep * j;
-            const float r = __ldg(ref + (size_t)clampi(py + dy, 0, H - 1) * W + x);
-            const float sd = sqrtf((float)(dx * dx + dy * dy));
-            const float w = hpm_expf(-sd / two_ss - fabsf(r - center) / two_sc);
-            const float rs = r - cs;
-            const float wr = w * rs;
-            P.p[i * 6 + j] = make_float2(w, wr);
-            r_r += wr;
-            r_rr = hpm_fma(wr, rs, r_rr);
-            r_w += w;
+            const int k = i * 6 + j;
+            const float rs = r[k] - cs;
+            r[k] = w[k] * rs;
+            r_r += r[k];
+            r_rr = hpm_fma(r[k], rs, r_rr);
+            r_w += w[k];
         }
         s_r += r_r; s_rr += r_rr; s_w += r_w;
+    }
+#pragma unroll
+    for (int q = 0; q < kPatchSamples / 2; ++q) {
+        const int k = 12 * (q / 6) + q % 6;
+        P.w[q] = pair_of(w[k], w[k + 6]);
+        P.wr[q] = pair_of(r[k], r[k + 6]);
     }
     P.rs.inv_w = 1.0f / s_w;
     P.rs.mean = s_r * P.rs.inv_w;
@@ -101,7 +241,7 @@ __device__ __forceinline__ PlaneM plane_m(const RunArgs& a, float4 pl) {
 
 // One bilateral NCC (HPM.cu:375-448) with the patch in registers.  CNT: the
 // counting build also counts the NCCs that sample the source (hyp_count[2]).
-template <bool CNT = false>
+template <bool CNT>
 __device__ __forceinline__ float ncc_view(const RunArgs& a, const Patch& P, int px, int py, const PlaneM& pm, int j) {
     const float cost_max = 2.0f;
     if (P.rs.var < 1e-5f) return cost_max;
@@ -127,41 +267,55 @@ __device__ __forceinline__ float ncc_view(const RunArgs& a, const Patch& P, int 
     }
     const cudaTextureObject_t tex = a.tex[j + 1];
     float s_s = 0.f, s_ss = 0.f, s_rs = 0.f;
-    float vshift = 0.0f;  // shifted moments: the source patch relative to its first sample
-    // two patch columns (12 fetches) are issued before their moments are summed: more fetches in
-    // flight per warp at the same register budget; the summation order is the oracle's
+    // Every fetch is carried through RunArgs::tex_scale and tex_bias; taken off are the bias or, for
+    // shifted moments, the patch's first sample.
+    float vshift = -a.tex_bias;
+    const Pair one = pair_of(1.0f, 1.0f), izc = pair_of(iz_c, iz_c);
+    const Pair h0 = pair_of(H[0], H[0]), h3 = pair_of(H[3], H[3]), h6 = pair_of(-H[6], -H[6]);
+    // Two patch columns make 12 fetches; the next two columns' are issued before the moments of these
+    // are summed, so the texture unit has work while the sums run.  The summation order is the oracle's.
+    float v[2][2][6];
+    auto fetch = [&](int i0, float (&o)[2][6]) {
+        const float x = (float)(px - kPatchRadius + kPatchStep * i0);
+        const Pair xx = pair_of(x, x + (float)kPatchStep);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            const float y = (float)(py - kPatchRadius + kPatchStep * k);
+            const float tx = hpm_fma(H[1], y, H[2]), ty = hpm_fma(H[4], y, H[5]), tz = hpm_fma(-H[7], y, -H[8]);
+            const float2 qx = halves(fma2(h0, xx, pair_of(tx, tx)));
+            const float2 qy = halves(fma2(h3, xx, pair_of(ty, ty)));
+            const Pair nqz = fma2(h6, xx, pair_of(tz, tz));  // -q_z
+            // hpm_recip_near(q_z, iz_c) of both
+            Pair r = fma2(izc, fma2(nqz, izc, one), izc);
+            r = fma2(r, fma2(nqz, r, one), r);
+            const float2 iz = halves(r);
+            o[0][k] = tex2D<float>(tex, hpm_fma(qx.x, iz.x, 0.5f), hpm_fma(qy.x, iz.x, 0.5f));
+            o[1][k] = tex2D<float>(tex, hpm_fma(qx.y, iz.y, 0.5f), hpm_fma(qy.y, iz.y, 0.5f));
+        }
+    };
+    fetch(0, v[0]);
 #pragma unroll
     for (int i0 = 0; i0 < 6; i0 += 2) {
-        float v[2][6];
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-            const float x = (float)(px - kPatchRadius + kPatchStep * (i0 + g));
-#pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                const float y = (float)(py - kPatchRadius + kPatchStep * k);
-                const float qx = hpm_fma(H[0], x, hpm_fma(H[1], y, H[2]));
-                const float qy = hpm_fma(H[3], x, hpm_fma(H[4], y, H[5]));
-                const float qz = hpm_fma(H[6], x, hpm_fma(H[7], y, H[8]));
-                const float iz = hpm_recip_near(qz, iz_c);
-                v[g][k] = tex2D<float>(tex, hpm_fma(qx, iz, 0.5f), hpm_fma(qy, iz, 0.5f));
-            }
+        const float (&vc)[2][6] = v[(i0 >> 1) & 1];
+        if (i0 < 4) {
+            fetch(i0 + 2, v[((i0 >> 1) + 1) & 1]);
+            asm volatile("" ::: "memory");  // the compiler keeps these fetches ahead of the sums below
         }
+        Pair r_s = 0, r_ss = 0, r_rs = 0;
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
-            const int i = i0 + g;
-            if (i == 0 && a.ncc_shift) vshift = v[0][0];
-            float r_s = 0.f, r_ss = 0.f, r_rs = 0.f;
-#pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                const float2 w = P.p[i * 6 + k];
-                const float vk = v[g][k] - vshift;
-                const float ws = w.x * vk;
-                r_s += ws;
-                r_ss = hpm_fma(ws, vk, r_ss);
-                r_rs = hpm_fma(w.y, vk, r_rs);
-            }
-            s_s += r_s; s_ss += r_ss; s_rs += r_rs;
+        for (int k = 0; k < 6; ++k) {
+            Pair vk = pair_of(vc[0][k], vc[1][k]);
+            vk = fma2(vk, pair_of(a.tex_scale, a.tex_scale), pair_of(a.tex_bias, a.tex_bias));
+            if (i0 == 0 && k == 0 && a.ncc_shift) vshift = -halves(vk).x;
+            vk = add2(vk, pair_of(vshift, vshift));
+            const Pair ws = mul2(P.w2(i0, k), vk);
+            r_s = add2(r_s, ws);
+            r_ss = fma2(ws, vk, r_ss);
+            r_rs = fma2(P.wr2(i0, k), vk, r_rs);
         }
+        const float2 c_s = halves(r_s), c_ss = halves(r_ss), c_rs = halves(r_rs);
+        s_s += c_s.x; s_ss += c_ss.x; s_rs += c_rs.x;
+        s_s += c_s.y; s_ss += c_ss.y; s_rs += c_rs.y;
     }
     s_s *= P.rs.inv_w; s_ss *= P.rs.inv_w; s_rs *= P.rs.inv_w;
     const float var_s = s_ss - s_s * s_s;
@@ -174,8 +328,8 @@ __device__ __forceinline__ float ncc_view(const RunArgs& a, const Patch& P, int 
 // ---------------------------------------------------------------- init
 
 template <int NS, int BLK, bool CNT>
-__device__ float initial_cost(const RunArgs& a, const Patch& P, int px, int py, float4 pl, uint32_t* sel_out,
-                              const Scratch<NS, BLK, CNT>& s) {
+__device__ __forceinline__ float initial_cost(const RunArgs& a, const Patch& P, int px, int py, float4 pl, uint32_t* sel_out,
+                              const InitScratch<NS, BLK>& s) {
     const float cost_max = 2.0f;
     const int S = a.S;
     int valid = 0;
@@ -183,7 +337,7 @@ __device__ float initial_cost(const RunArgs& a, const Patch& P, int px, int py, 
     const PlaneM pm = plane_m(a, pl);
 #pragma unroll 1
     for (int j = 0; j < S; ++j) {
-        const float c = ncc_view(a, P, px, py, pm, j);
+        const float c = ncc_view<false>(a, P, px, py, pm, j);
         s.ca(0, j) = c;
         s.ca(1, j) = c;
         if (c < cost_max) ++valid;
@@ -221,7 +375,7 @@ __device__ __forceinline__ float range_gauss(float x, float sigma) {
 }
 
 template <int NS, int BLK, bool CNT>
-__device__ __forceinline__ void init_pixel(const RunArgs& a, const Scratch<NS, BLK, CNT>& s, int px, int py) {
+__device__ __forceinline__ void init_pixel(const RunArgs& a, const InitScratch<NS, BLK>& s, int px, int py) {
     const int W = a.W, H = a.H;
     if (px >= W || py >= H) return;
     const int center = py * W + px;
@@ -234,23 +388,21 @@ __device__ __forceinline__ void init_pixel(const RunArgs& a, const Scratch<NS, B
 
     if (!prior && !mand) a.texture[center] = texture_term(a.canny, W, H, px, py);
 
-    Patch P;
-    build_patch(a, px, py, P);
-    uint32_t sel = 0;
+    // What the pixel starts from: the plane to store, and the hypothesis to cost against all sources,
+    // if any.  Every mode meets in one costing loop, so the kernel carries one copy of the NCC.
+    bool store = true, cost = true;
+    float4 pl = a.planes[center];
+    float pre_depth = 0.0f;  // upsample mode: offset of the pre-cost hypothesis
     if (!geom && !hier && !prior) {
         const float depth = rng.uniform() * (a.prm.depth_max - a.prm.depth_min) + a.prm.depth_min;
-        float4 pl = random_normal(c0, px, py, rng, depth);
-        pl.w = distance_to_origin(c0, px, py, depth, pl);
-        a.planes[center] = pl;
-        a.costs[center] = initial_cost(a, P, px, py, pl, &sel, s);
-        a.sel[center] = sel;
+        pl = random_normal(c0, px, py, rng, depth);
+        pl.w = depth;
     } else if (prior) {
+        const bool sure = a.conf[center] > 0.3;
         if (a.pmask[center] > 0) {
-            if (a.conf[center] > 0.3) {
-                float4 pl = a.planes[center];
-                pl.w = distance_to_origin(c0, px, py, pl.w, pl);
-                a.planes[center] = pl;
+            if (sure) {
                 a.costs[center] = 0.1f;
+                cost = false;
             } else if (a.costs[center] > 0.1f) {
                 const float perturbation = 0.02f;
                 const float4 pp = a.prior[center];
@@ -258,23 +410,14 @@ __device__ __forceinline__ void init_pixel(const RunArgs& a, const Scratch<NS, B
                 const float dmin_p = (1 - 3 * perturbation) * dp;
                 const float dmax_p = (1 + 3 * perturbation) * dp;
                 dp = rng.uniform() * (dmax_p - dmin_p) + dmin_p;
-                float4 pl = perturbed_normal(c0, px, py, pp, rng, (float)(3 * perturbation * 3.14159265358979323846));
+                pl = perturbed_normal(c0, px, py, pp, rng, (float)(3 * perturbation * 3.14159265358979323846));
                 pl.w = dp;
+                store = false;
                 a.planes[center] = pl;
-                a.costs[center] = initial_cost(a, P, px, py, pl, &sel, s);
-                a.sel[center] = sel;
-            } else {
-                float4 pl = a.planes[center];
-                pl.w = distance_to_origin(c0, px, py, pl.w, pl);
-                a.planes[center] = pl;
-                a.costs[center] = initial_cost(a, P, px, py, pl, &sel, s);
-                a.sel[center] = sel;
             }
         } else {
-            float4 pl = a.planes[center];
-            pl.w = distance_to_origin(c0, px, py, pl.w, pl);
-            a.planes[center] = pl;
-            if (a.conf[center] > 0.3) a.costs[center] = 0.1f;
+            cost = false;
+            if (sure) a.costs[center] = 0.1f;
         }
     } else if (ups) {
         const int scols = a.prm.scaled_cols, srows = a.prm.scaled_rows;
@@ -291,6 +434,7 @@ __device__ __forceinline__ void init_pixel(const RunArgs& a, const Scratch<NS, B
             int r_y = __float2int_rz(o_y + j);
             r_y = (r_y > 0 ? (r_y < sr_f ? r_y : srows - 1) : 0);
             const int r_ys = clampi(py + j, 0, H - 1);
+#pragma unroll 1
             for (int i = -nn; i <= nn; ++i) {
                 int r_x = __float2int_rz(o_x + i);
                 r_x = (r_x > 0 ? (r_x < sc_f ? r_x : scols - 1) : 0);
@@ -305,36 +449,46 @@ __device__ __forceinline__ void init_pixel(const RunArgs& a, const Scratch<NS, B
         }
         float4 nt = make_float4(n0 / nf, n1 / nf, n2 / nf, 0.0f);
         normalize3(nt);
-        const float4 cur = a.planes[center];
-        // pre-cost plane: zero normal, upsampled depth as offset (HPM.cu:689, HPM.cpp:894-901)
-        const float pre = initial_cost(a, P, px, py, make_float4(0.f, 0.f, 0.f, cur.w), &sel, s);
-        a.pre_costs[center] = pre;
-        float4 pl = rotate_to_cam(c0, nt);
-        pl.w = distance_to_origin(c0, px, py, cur.w, pl);
-        a.planes[center] = pl;
-        a.costs[center] = initial_cost(a, P, px, py, pl, &sel, s);
-        a.sel[center] = sel;
+        pre_depth = pl.w;
+        pl = rotate_to_cam(c0, nt);
+        pl.w = pre_depth;
     } else {
         if (mand && !(a.conf[center] >= 0.3)) {
             if (texture_term(a.canny, W, H, px, py) > 0.5) a.conf[center] = 0.1f;
         }
-        float4 pl = hier ? a.scaled[center] : a.planes[center];
+        if (hier) pl = a.scaled[center];
         pl = rotate_to_cam(c0, pl);
+    }
+    if (store) {
+        // pl.w is the depth here; the perturbed prior keeps its depth as the offset (HPM.cu:603-604)
         pl.w = distance_to_origin(c0, px, py, pl.w, pl);
         a.planes[center] = pl;
-        a.costs[center] = initial_cost(a, P, px, py, pl, &sel, s);
-        a.sel[center] = sel;
     }
     a.rng[center] = rng.draw;
+    if (!cost) return;
+
+    float tmp[kPatchWords];
+    Patch P;
+    build_patch(a, px, py, P, tmp);
+    uint32_t sel = 0;
+    // upsample mode costs the pre-cost plane first: zero normal, upsampled depth as offset (HPM.cu:689,
+    // HPM.cpp:894-901)
+#pragma unroll 1
+    for (int h = ups ? 0 : 1; h < 2; ++h) {
+        const float4 hyp = h ? pl : make_float4(0.f, 0.f, 0.f, pre_depth);
+        const float c = initial_cost<NS, BLK, CNT>(a, P, px, py, hyp, &sel, s);
+        (h ? a.costs : a.pre_costs)[center] = c;
+    }
+    a.sel[center] = sel;
 }
 
+// 32 x 4 blocks, 12 warps per SM: 1.10 ms per 1600x1200 geometric initialisation with one costing loop,
+// byte textures and the weight table, against 1.50 with an inlined copy of the NCC per mode
 template <int NS, int BLK, bool CNT>
-// 3 blocks per SM (at most 168 registers): 12 warps, against 8 at the unbounded 174 registers; 1.5 ms
-// instead of 1.8 ms per 1600x1200 initialisation with 32 x 4 blocks
-__global__ void __launch_bounds__(BLK, 3) k_random_init(const __grid_constant__ RunArgs a) {
+__global__ void __launch_bounds__(BLK, kSweepBlocks) k_random_init(const __grid_constant__ RunArgs a) {
     extern __shared__ float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    const Scratch<NS, BLK, CNT> s{ smem + tid };
+    const InitScratch<NS, BLK> s{ smem + tid };
     init_pixel<NS, BLK, CNT>(a, s, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y);
 }
 
@@ -362,11 +516,11 @@ __device__ __forceinline__ int batch_run_of(const int* __restrict__ tile_start, 
 }
 
 template <int NS, int BLK, bool CNT>
-__global__ void __launch_bounds__(BLK) k_random_init_batch(const RunArgs* __restrict__ args,
+__global__ void __launch_bounds__(BLK, kSweepBlocks) k_random_init_batch(const RunArgs* __restrict__ args,
                                                            const int* __restrict__ tile_start, int n) {
     extern __shared__ float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    const Scratch<NS, BLK, CNT> s{ smem + tid };
+    const InitScratch<NS, BLK> s{ smem + tid };
     const int total = __ldg(tile_start + n);
     for (int b = blockIdx.x; b < total; b += gridDim.x) {
         const int k = batch_run_of(tile_start, n, b);
@@ -379,323 +533,305 @@ __global__ void __launch_bounds__(BLK) k_random_init_batch(const RunArgs* __rest
 
 // ---------------------------------------------------------------- propagation
 
-// Costs of one hypothesis (its PlaneM) against the source views in `mask`,
-// into scratch row `row` (ComputeMultiViewCostVector, HPM.cu:490-495).  The
-// only place a half-sweep evaluates the NCC, so the kernel carries one copy.
-// The loop runs over view indices, the same for every lane: a variant in which
-// each lane took its own k-th selected view ran three times slower on B200,
-// because texture fetches with different texture objects across a warp
-// serialise.
-template <int NS, int BLK, bool CNT>
-__device__ __forceinline__ void eval_row(const RunArgs& a, const Patch& P, int px, int py, const PlaneM& pm,
-                                         uint32_t mask, int row, const Scratch<NS, BLK, CNT>& s) {
-#pragma unroll 1
-    for (int j = 0; j < a.S; ++j)
-        if ((mask >> j) & 1u) s.ca(row, j) = ncc_view<CNT>(a, P, px, py, pm, j);
-}
-
-__device__ __forceinline__ void v_path_scan(const float* __restrict__ costs, int W, int H, int x, int y, int ax,
-                                            int ay, int bx, int by, float& bc, int& best) {
+// The lowest-cost position of a diagonal path: `start`, then up to seven more, steps (ax, ay) and
+// (bx, by) in turn from (x, y), while inside the image.
+static __device__ __noinline__ int v_path_best(const float* __restrict__ costs, int W, int H, int x, int y, int ax,
+                                               int ay, int bx, int by, int start) {
+    int best = start;
+    float bc = costs[best];
+    float c[7];
+    int q[7];
+    bool in = true;
 #pragma unroll
     for (int i = 0; i < 7; ++i) {
         if (i % 2 == 0) { x += ax; y += ay; } else { x += bx; y += by; }
-        if (x >= 0 && x < W && y < H && y >= 0) {
-            const int q = y * W + x;
-            const float c = costs[q];
-            if (c < bc) { bc = c; best = q; }
-        } else break;
+        in = in && x >= 0 && x < W && y < H && y >= 0;  // the path ends where it leaves the image
+        q[i] = in ? y * W + x : start;
+        c[i] = costs[q[i]];
     }
-}
-
-// First candidate 5 px away along (dx, dy), then up to 4 more every 2 px while
-// inside the image (HPM.cu:1385-1475).  right_far keeps the maximum (HPM.cu:1464).
-__device__ __forceinline__ bool far_search(const float* __restrict__ costs, int W, int H, int px, int py, int dx,
-                                           int dy, bool keep_max, int& pos) {
-    const int x = px + 5 * dx, y = py + 5 * dy;
-    if (x < 0 || x >= W || y < 0 || y >= H) return false;
-    int best = y * W + x;
-    float bc = costs[best];
 #pragma unroll
-    for (int i = 1; i < 5; ++i) {
-        const int xi = px + (5 + 2 * i) * dx, yi = py + (5 + 2 * i) * dy;
-        if (xi < 0 || xi >= W || yi < 0 || yi >= H) break;
-        const int q = yi * W + xi;
-        const float c = costs[q];
-        if (keep_max ? (bc < c) : (c < bc)) { bc = c; best = q; }
-    }
-    pos = best;
-    return true;
+    for (int i = 0; i < 7; ++i)
+        if (c[i] < bc) { bc = c[i]; best = q[i]; }
+    return best;
 }
 
 // Non-local candidate positions of the eight directions (HPM.cu:1367-1608);
 // returns the bitmask of valid directions and leaves the positions in scratch.
-template <int NS, int BLK, bool CNT>
-__device__ __forceinline__ uint32_t direction_search(const RunArgs& a, int px, int py,
-                                                     const Scratch<NS, BLK, CNT>& s) {
+// Odd directions (up, down, left, right): the first candidate 5 px away, then up
+// to 4 more every 2 px while inside the image (HPM.cu:1385-1475); the last
+// keeps the maximum (HPM.cu:1464).  Even ones (left-up, right-up, right-down,
+// left-down): a diagonal path from 5 or 6 px away.
+template <int NS, int BLK>
+__device__ __forceinline__ uint32_t direction_search(const RunArgs& a, int px, int py, const Scratch<NS, BLK>& s) {
     const int W = a.W, H = a.H;
-    const int center = py * W + px;
     const float* __restrict__ costs = a.costs;
     uint32_t flags = 0;
-    int pos[8];
-    pos[0] = center - 5 - 6 * W; pos[1] = center - 5 * W; pos[2] = center + 6 - 5 * W; pos[3] = center + 5 * W;
-    pos[4] = center + 5 + 6 * W; pos[5] = center - 5; pos[6] = center - 6 + 5 * W; pos[7] = center + 5;
-    if (far_search(costs, W, H, px, py, 0, -1, false, pos[1])) flags |= 1u << 1;
-    if (far_search(costs, W, H, px, py, 0, 1, false, pos[3])) flags |= 1u << 3;
-    if (far_search(costs, W, H, px, py, -1, 0, false, pos[5])) flags |= 1u << 5;
-    if (far_search(costs, W, H, px, py, 1, 0, true, pos[7])) flags |= 1u << 7;
-    if (px > 4 && py > 5) {
-        flags |= 1u << 0;
-        float bc = costs[pos[0]]; int best = pos[0];
-        v_path_scan(costs, W, H, px - 5, py - 6, -2, 0, 0, -2, bc, best);
-        pos[0] = best;
-    }
-    if (px < W - 6 && py > 4) {
-        flags |= 1u << 2;
-        float bc = costs[pos[2]]; int best = pos[2];
-        v_path_scan(costs, W, H, px + 6, py - 5, 0, -2, 2, 0, bc, best);
-        pos[2] = best;
-    }
-    if (px < W - 5 && py < H - 6) {
-        flags |= 1u << 4;
-        float bc = costs[pos[4]]; int best = pos[4];
-        v_path_scan(costs, W, H, px + 5, py + 6, 2, 0, 0, 2, bc, best);
-        pos[4] = best;
-    }
-    if (px > 5 && py < H - 5) {
-        flags |= 1u << 6;
-        float bc = costs[pos[6]]; int best = pos[6];
-        v_path_scan(costs, W, H, px - 6, py + 5, 0, 2, -2, 0, bc, best);
-        pos[6] = best;
-    }
+    // one straight and one diagonal direction a turn, their loads in flight together
+#pragma unroll 1
+    for (int d = 0; d < 8; d += 2) {
+        const int dx = d == 4 ? -1 : (d == 6 ? 1 : 0), dy = d == 0 ? -1 : (d == 2 ? 1 : 0);
+        const int x = px + 5 * dx, y = py + 5 * dy;
+        const bool straight = !(x < 0 || x >= W || y < 0 || y >= H);
+        float far_cost[5];
+        bool far_in[5];
 #pragma unroll
-    for (int d = 0; d < 8; ++d) s.pos(d) = pos[d];
+        for (int i = 0; i < 5; ++i) {
+            const int xi = px + (5 + 2 * i) * dx, yi = py + (5 + 2 * i) * dy;
+            far_in[i] = !(xi < 0 || xi >= W || yi < 0 || yi >= H);
+            far_cost[i] = far_in[i] ? costs[yi * W + xi] : 0.0f;
+        }
+        const int sx = px + (d == 0 ? -5 : d == 2 ? 6 : d == 4 ? 5 : -6);
+        const int sy = py + (d == 0 ? -6 : d == 2 ? -5 : d == 4 ? 6 : 5);
+        if (!(sx < 0 || sx >= W || sy < 0 || sy >= H)) {
+            // left-up: (-2, 0) (0, -2); right-up: (0, -2) (2, 0); right-down: (2, 0) (0, 2); left-down: (0, 2) (-2, 0)
+            const bool x_first = d == 0 || d == 4;
+            const int ex = d == 0 || d == 6 ? -2 : 2, ey = d == 0 || d == 2 ? -2 : 2;
+            s.pos(d) = v_path_best(costs, W, H, sx, sy, x_first ? ex : 0, x_first ? 0 : ey, x_first ? 0 : ex,
+                                   x_first ? ey : 0, sy * W + sx);
+            flags |= 1u << d;
+        }
+        if (straight) {
+            int best = 0;
+            float bc = far_cost[0];
+#pragma unroll
+            for (int i = 1; i < 5; ++i)
+                if (far_in[i] && (d == 6 ? (bc < far_cost[i]) : (far_cost[i] < bc))) { bc = far_cost[i]; best = i; }
+            s.pos(d + 1) = (py + (5 + 2 * best) * dy) * W + px + (5 + 2 * best) * dx;
+            flags |= 2u << d;
+        }
+    }
     return flags;
 }
 
 struct Selection {
     uint32_t temp_selected;
-    int num_selected;
     float weight_norm;
 };
 
 // Joint view selection and the eight final costs (HPM.cu:1686-1771), from the
 // cost rows of the directions; weights to scratch vw, final costs to fc.
-template <int NS, int BLK, bool CNT>
+template <int NS, int BLK>
 __device__ __forceinline__ Selection view_selection(const RunArgs& a, int px, int py, int iter, uint32_t flags,
-                                                    PixelRng& rng, const Scratch<NS, BLK, CNT>& s) {
+                                                    PixelRng& rng, const Scratch<NS, BLK>& s) {
     const int W = a.W, S = a.S;
     const int center = py * W + px;
     const bool geom = a.prm.mode & HPM_MODE_GEOM;
-    float priors[NS];
-#pragma unroll
-    for (int j = 0; j < NS; ++j) priors[j] = 0.0f;
     const int nbr[4] = { center - W * 5, center + W * 5, center - 5, center + 5 };
+    uint32_t near[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        if (flags & (1u << (2 * i + 1))) {
-            const uint32_t m = a.sel[nbr[i]];
-#pragma unroll
-            for (int j = 0; j < NS; ++j)
-                if (j < S) priors[j] += ((m >> j) & 1u) ? 0.9f : 0.1f;
-        }
-    }
+    for (int i = 0; i < 4; ++i) near[i] = (flags & (1u << (2 * i + 1))) ? a.sel[nbr[i]] : 0u;
     const float cost_thr = (float)(0.8 * hpm_expf((float)(iter * iter) / (-90.0f)));
-    float probs[NS];
+    float sum = 0.0f;
+#pragma unroll 1
+    for (int j = 0; j < S; ++j) {
+        float prior = 0.0f;
 #pragma unroll
-    for (int j = 0; j < NS; ++j) {
-        probs[j] = 0.0f;
-        if (j < S) {
-            float count = 0.0f, tmpw = 0.0f;
-            int count_false = 0;
+        for (int i = 0; i < 4; ++i)
+            if (flags & (1u << (2 * i + 1))) prior += ((near[i] >> j) & 1u) ? 0.9f : 0.1f;
+        float count = 0.0f, tmpw = 0.0f, prob = 0.0f;
+        int count_false = 0;
+        float c[8];
 #pragma unroll
-            for (int d = 0; d < 8; ++d) {
-                const float c = s.ca(d, j);
-                if (c < cost_thr) { tmpw += hpm_expf(c * c / (-0.18f)); count += 1.0f; }
-                if (c > 1.2f) ++count_false;
-            }
-            if (count > 2 && count_false < 3) probs[j] = tmpw / count;
-            else if (count_false < 3) probs[j] = hpm_expf(cost_thr * cost_thr / (-0.32f));
-            probs[j] = probs[j] * priors[j];
+        for (int d = 0; d < 8; ++d) c[d] = s.ca(d, j);
+#pragma unroll 4
+        for (int d = 0; d < 8; ++d) {
+            const float e = hpm_expf(c[d] * c[d] / (-0.18f));
+            if (c[d] < cost_thr) { tmpw += e; count += 1.0f; }
+            if (c[d] > 1.2f) ++count_false;
         }
+        if (count > 2 && count_false < 3) prob = tmpw / count;
+        else if (count_false < 3) prob = hpm_expf(cost_thr * cost_thr / (-0.32f));
+        prob = prob * prior;
+        s.vw(j) = prob;
+        sum += prob;
     }
+    // 15 draws from the cumulative distribution, counted in 4 bits per view: a draw takes the first
+    // view whose sum is above it.  The sums do not fall, so that is the view numbered by how many are
+    // not above it (no view when the probabilities are all zero and the sums NaN).
+    float cum[NS];
     {
-        float sum = 0.0f;
-#pragma unroll
-        for (int j = 0; j < NS; ++j) if (j < S) sum += probs[j];
         const float inv = 1.0f / sum;
-        float cum = 0.0f;
+        float acc = 0.0f;
 #pragma unroll
-        for (int j = 0; j < NS; ++j) if (j < S) { cum += probs[j] * inv; probs[j] = cum; }
+        for (int j = 0; j < NS; ++j)
+            if (j < S) { acc += s.vw(j) * inv; cum[j] = acc; }
     }
-    float vw[NS];
+    uint32_t hits[(NS + 7) / 8];
 #pragma unroll
-    for (int j = 0; j < NS; ++j) vw[j] = 0.0f;
+    for (int k = 0; k < (NS + 7) / 8; ++k) hits[k] = 0;
+#pragma unroll 1
     for (int smp = 0; smp < 15; ++smp) {
         const float rp = rng.uniform() - FLT_EPSILON;
-        bool done = false;
+        int first = 0;
 #pragma unroll
-        for (int j = 0; j < NS; ++j) {
-            if (!done && j < S && probs[j] > rp) { vw[j] += 1.0f; done = true; }
-        }
+        for (int j = 0; j < NS; ++j)
+            if (j < S && !(cum[j] > rp)) ++first;
+#pragma unroll
+        for (int k = 0; k < (NS + 7) / 8; ++k)
+            if (first < S && (first >> 3) == k) hits[k] += 1u << (4 * (first & 7));
     }
     Selection o;
-    o.temp_selected = 0; o.num_selected = 0; o.weight_norm = 0.0f;
+    o.temp_selected = 0; o.weight_norm = 0.0f;
 #pragma unroll
     for (int j = 0; j < NS; ++j) {
-        s.vw(j) = vw[j];
-        if (j < S && vw[j] > 0) {
+        const uint32_t n = (hits[j >> 3] >> (4 * (j & 7))) & 15u;
+        const float w = (float)n;
+        s.vw(j) = w;
+        if (n > 0) {
             o.temp_selected |= 1u << j;
-            o.weight_norm += vw[j];
-            o.num_selected++;
+            o.weight_norm += w;
         }
     }
+    // Final costs of the directions (HPM.cu:1752-1771): sums over the selected views in their order.
+    // View after view, so that the eight directions' depth gathers of the geometric cost are in
+    // flight together.
+    float fc[8];
+#pragma unroll
+    for (int d = 0; d < 8; ++d) fc[d] = s.fc(d) = 0.0f;
 #pragma unroll 1
-    for (int d = 0; d < 8; ++d) {
-        float fc = 0.0f;
-        const bool valid = flags & (1u << d);
-        float depth = 0.0f;
-        if (geom && valid) depth = depth_from_plane(a.cams[0], a.planes[s.pos(d)], px, py);
-        for (int j = 0; j < S; ++j) {
-            const float w = s.vw(j);
-            if (w > 0) {
-                if (geom) {
-                    if (valid)
-                        fc += w * (s.ca(d, j) + 0.2f * geom_cost(a.depth_src[j + 1], a.dsw[j + 1], a.dsh[j + 1],
-                                                                   a.fwd[j + 1].A, a.fwd[j + 1].b, a.bwd[j + 1].A,
-                                                                   a.bwd[j + 1].b, depth, px, py));
-                    else
-                        fc += w * (s.ca(d, j) + 0.1f * 3.0f);
-                } else {
-                    fc += w * s.ca(d, j);
+    for (int j = 0; j < S; ++j) {
+        const float w = s.vw(j);
+        if (!(w > 0)) continue;
+        if (!geom) {
+#pragma unroll
+            for (int d = 0; d < 8; ++d) fc[d] += w * s.ca(d, j);
+        } else {
+#pragma unroll 1
+            for (int h = 0; h < 8; h += 4) {
+                float sx[4], sy[4], sd[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float depth = (flags >> (h + k)) & 1u ? s.cand[h + k].w : 0.0f;
+                    sd[k] = geom_source_depth(a.depth_src[j + 1], a.dsw[j + 1], a.dsh[j + 1], a.fwd[j + 1].A,
+                                              a.fwd[j + 1].b, depth, px, py, sx[k], sy[k]);
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float g = (flags >> (h + k)) & 1u
+                                        ? 0.2f * geom_back_cost(a.bwd[j + 1].A, a.bwd[j + 1].b, sx[k], sy[k], sd[k], px, py)
+                                        : 0.1f * 3.0f;
+                    s.fc(h + k) += w * (s.ca(h + k, j) + g);
                 }
             }
         }
-        s.fc(d) = fc / o.weight_norm;
     }
+#pragma unroll
+    for (int d = 0; d < 8; ++d) s.fc(d) = (geom ? s.fc(d) : fc[d]) / o.weight_norm;
     return o;
 }
 
-// Weighted cost over the selected views of the hypothesis whose NCCs are in
-// scratch row 8 (HPM.cu:1775-1786, 805-817).
-template <int NS, int BLK, bool CNT>
-__device__ __forceinline__ float selected_cost(const RunArgs& a, int px, int py, float4 pl, uint32_t selmask,
-                                               float weight_norm, const Scratch<NS, BLK, CNT>& s) {
-    const bool geom = a.prm.mode & HPM_MODE_GEOM;
-    const float depth = geom ? depth_from_plane(a.cams[0], pl, px, py) : 0.0f;
-    float c = 0.0f;
-#pragma unroll 1
-    for (int j = 0; j < a.S; ++j) {
-        if (!((selmask >> j) & 1u)) continue;
-        const float w = s.vw(j);
-        const float n = s.ca(8, j);
-        if (geom) c += w * (n + 0.2f * geom_cost(a.depth_src[j + 1], a.dsw[j + 1], a.dsh[j + 1], a.fwd[j + 1].A,
-                                                  a.fwd[j + 1].b, a.bwd[j + 1].A, a.bwd[j + 1].b, depth, px,
-                                                  py));
-        else c += w * n;
-    }
-    return c / weight_norm;
-}
+constexpr float kPriorBeta = 0.18f;
 
-__device__ __forceinline__ int find_min_index8(const float* v) {  // ties -> last (HPM.cu:41-52)
-    float m = v[0]; int idx = 0;
-#pragma unroll
-    for (int i = 1; i < 8; ++i) if (v[i] <= m) { m = v[i]; idx = i; }
-    return idx;
-}
-
-__device__ __forceinline__ int find_max_index8(const float* v) {  // ties -> last (HPM.cu:54-65)
-    float m = v[0]; int idx = 0;
-#pragma unroll
-    for (int i = 1; i < 8; ++i) if (v[i] >= m) { m = v[i]; idx = i; }
-    return idx;
-}
-
-__device__ __forceinline__ float prior_score(float final_cost, float depth_now, float depth_prior, float4 pp,
-                                             float4 pl, float texture, float two_dss, float two_ass) {
-    const float gamma = 0.5f, beta = 0.18f;
+// The prior's factor of the score: how near the hypothesis is to the prior plane.
+static __device__ __noinline__ float prior_factor(float depth_now, float depth_prior, float4 pp, float4 pl, float texture,
+                                              float two_dss, float two_ass) {
+    const float gamma = 0.5f;
     const float dd = depth_now - depth_prior;
     const float nd = fabsf(pp.x - pl.x) + fabsf(pp.y - pl.y) + fabsf(pp.z - pl.z);
-    const float prior = (float)(gamma * (1.2 - 0.2 * texture) + (double)(hpm_expf(-dd * dd / two_dss) * hpm_expf(-nd * nd / two_ass)));
-    return (float)(exp(-final_cost * final_cost / beta * (1 + 0.2 * texture)) * (double)prior);
+    return (float)(gamma * (1.2 - 0.2 * texture) + (double)(hpm_expf(-dd * dd / two_dss) * hpm_expf(-nd * nd / two_ass)));
 }
+
+static __device__ __noinline__ float prior_score(float final_cost, float depth_now, float depth_prior, float4 pp,
+                                             float4 pl, float texture, float two_dss, float two_ass) {
+    const float prior = prior_factor(depth_now, depth_prior, pp, pl, texture, two_dss, two_ass);
+    return (float)(exp(-final_cost * final_cost / kPriorBeta * (1 + 0.2 * texture)) * (double)prior);
+}
+
+// Threshold of a good cost in round `it` of the extension (HPM.cu:1063-1126).
+static __device__ __noinline__ float good_threshold(int iter, int it) {
+    return (float)(0.8 * exp(-iter * iter * (3 - it) / 90.0));
+}
+
+// Margins of the refinement's rejection limits.  A candidate is accepted when its weighted mean cost
+// is below the current one (or, under a prior, when its score is above the current one, which falls
+// with the cost).  The terms of the sum are not negative and rounded addition and division are
+// monotone, so a partial sum above the limit is a rejection; the margins cover the rounding of the
+// limit itself (a few units of 2^-24, and the logarithm's), ten and a hundred times over.
+constexpr float kLimitMargin = 1.000002f;
+constexpr float kLogMargin = 1e-5f;
 
 // One pixel of a black or red half-sweep: CheckerboardPropagation (HPM.cu:1347-1873)
 // or, with MAND, CheckerboardPropagation_MandatoryConsistency (HPM.cu:1875-2791).
 //
 // The NCC work runs in one loop of 17 slots, each costing at most one
-// hypothesis through eval_row:
-//   slots 0-7    the eight direction candidates, against all sources;
-//   slots 8-10   the three rounds of the left-up extension (HPM.cu:1063-1126);
+// hypothesis:
+//   slot  0      the left-up direction's candidate, against all sources;
+//   slots 1-3    the three rounds of its extension (HPM.cu:1063-1126);
+//   slots 4-10   the candidates of directions 1-7;
 //   slot  11     view selection, then the current plane against the selected views;
 //   slots 12-16  the five PlaneHypothesisRefinement candidates (HPM.cu:765-841),
 //                built from the state at entry and accepted greedily in order.
 // The decisions between slots are the reference's, in its order, and the
 // random draws happen in the same sequence.
-#ifndef HPM_SWEEP_MIN_BLOCKS
-#define HPM_SWEEP_MIN_BLOCKS 3  // 3 blocks of 128 threads per SM: at most 170 registers
-#endif
-
 template <int NS, int BLK, bool MAND, bool CNT>
-__device__ __forceinline__ void sweep_pixel(const RunArgs& a, const Scratch<NS, BLK, CNT>& s, int px, int pair,
-                                            int color, int iter) {
+__device__ __forceinline__ void sweep_pixel(const RunArgs& a, float* smem_column, int px, int pair, int color,
+                                            int iter) {
     const int py = 2 * pair + ((px & 1) ^ color);
     const int W = a.W, H = a.H, S = a.S;
     if (px >= W || py >= H || pair >= a.cover_pairs) return;
     const int center = py * W + px;
     const hpm_camera& c0 = a.cams[0];
     const uint32_t mode = a.prm.mode;
-    const bool prior = mode & HPM_MODE_PRIOR, hier = mode & HPM_MODE_HIERARCHY;
+    const bool prior = mode & HPM_MODE_PRIOR, hier = mode & HPM_MODE_HIERARCHY, geom = mode & HPM_MODE_GEOM;
     const float dmin = a.prm.depth_min, dmax = a.prm.depth_max;
 
     if (!MAND && prior) {
         if (a.conf[center] > 0.3) return;
         if (a.pmask[center] == 0) return;
     }
-    PixelRng rng;
-    rng.init(a.seed, a.view_id, px, py, a.rng[center]);
+    float rows[Scratch<NS, BLK>::kRowWords];
+    float4 cand[8];
+    const Scratch<NS, BLK> s{ smem_column, rows, cand };
     Patch P;
-    build_patch(a, px, py, P);
-    const bool reliable = MAND ? (a.conf[center] >= 0.3) : true;
+    build_patch(a, px, py, P, rows);
     const uint32_t all_views = (S >= 32) ? 0xffffffffu : ((1u << S) - 1u);
 
-    // `float cost_array[8][32] = { 2.0f }` (HPM.cu:1378): only [0][0] is 2, the rest 0.
-    for (int d = 0; d < 8; ++d)
-        for (int j = 0; j < S; ++j) s.ca(d, j) = 0.0f;
-    s.ca(0, 0) = 2.0f;
     const uint32_t flags = direction_search(a, px, py, s);
+    auto candidate = [&](int at) {
+        const float4 p = a.planes[at];
+        const PlaneM m = plane_m(a, p);
+        return make_float4(m.m[0], m.m[1], m.m[2], geom ? depth_from_plane(c0, p, px, py) : 0.0f);
+    };
+#pragma unroll 4
+    for (int d = 0; d < 8; ++d)  // the gathers in flight together, not one at each slot's head
+        if ((flags >> d) & 1u) cand[d] = candidate(s.pos(d));
+    // `float cost_array[8][32] = { 2.0f }` (HPM.cu:1378): the row of a direction outside the image is
+    // 0, but [0][0] is 2.
+    if (flags != 0xffu) {
+        for (int d = 0; d < 8; ++d)
+            if (!((flags >> d) & 1u))
+                for (int j = 0; j < S; ++j) s.ca(d, j) = d + j == 0 ? 2.0f : 0.0f;
+    }
 
     // state carried across slots
     bool extending = flags & 1u;  // left-up extension still active
-    Selection sel{ 0u, 0, 0.0f };
     bool refine = false;          // slots 12-16 run
-    bool use_prior = false;
-    float4 cur = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 plane_now = cur;
-    float depth_now = 0.0f, cost_now = 0.0f, restricted_cost = 0.0f, texture = 0.0f, depth_prior = 0.0f;
-    float4 pp = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 plane0 = cur, plane_rand = cur, plane_pert = cur;
-    float depth0 = 0.0f, depth_rand = 0.0f, depth_pert = 0.0f;
+    uint32_t selected = 0;        // views of the selection, and the sum of their weights
+    float weight_norm = 0.0f;
+    float cost_now = 0.0f, restricted_cost = 0.0f;
     const float depth_sigma = (dmax - dmin) / 64.0f;
     const float two_dss = 2 * depth_sigma * depth_sigma;
     const float angle_sigma = (float)(3.14159265358979323846 * (5.0f / 180.0f));
     const float two_ass = 2 * angle_sigma * angle_sigma;
-
+    // words of the scratch rows after view selection: 0-4 the candidates (normal, depth), 5 the plane
+    // of the pixel, 6 the prior plane, 7 (prior depth, texture, prior used)
+    constexpr int kHeldNow = 5, kHeldPrior = 6, kHeldTerms = 7;
 #pragma unroll 1
     for (int t = 0; t < 17; ++t) {
         bool run = false;
         float4 pl = make_float4(0.f, 0.f, 0.f, 0.f);
         uint32_t mask = all_views;
-        int row = 8;
-        if (t < 8) {
-            run = (flags >> t) & 1u;
-            if (run) pl = a.planes[s.pos(t)];
-            row = t;
-        } else if (t < 11) {
+        int row = 0;
+        float depth = 0.0f;       // slots 11-16: the hypothesis' depth at the pixel (geometric cost)
+        float limit = INFINITY;   // slots 12-16: a weighted cost sum above it is rejected
+        if (t == 0) {
+            run = flags & 1u;
+        } else if (t < 4) {
             // Extended propagation: only orientation 0 (left_up) is active because
             // `bool symbol_eight_orientations[10] = { true }` (HPM.cu:1612, 1063-1126).
-            const int it = t - 8;
+            const int it = t - 1;
             if (extending) {
-                const float good_thr = (float)(0.8 * exp(-iter * iter * (3 - it) / 90.0));
+                const float good_thr = good_threshold(iter, it);
                 int good = 0, bad = 0;
                 for (int j = 0; j < S; ++j) {
                     const float c = s.ca(0, j);
@@ -707,55 +843,108 @@ __device__ __forceinline__ void sweep_pixel(const RunArgs& a, const Scratch<NS, 
                 } else if (px > 4 + 8 * it && py > 5 + 8 * it) {
                     const int sx = px - 5 - 8 * it, sy = py - 6 - 8 * it;
                     int best = sy * W + sx;
-                    float bc = a.costs[best];
-                    v_path_scan(a.costs, W, H, sx, sy, -2, 0, 0, -2, bc, best);
+                    best = v_path_best(a.costs, W, H, sx, sy, -2, 0, 0, -2, best);
                     const int prev = s.pos(0);
-                    if (bc > a.costs[prev]) {
+                    if (a.costs[best] > a.costs[prev]) {
                         best = prev;
                     } else if (best != prev) {
                         run = true;
-                        pl = a.planes[best];
-                        row = 0;
+                        cand[0] = candidate(best);
                     }
                     // best == prev recomputes the same row in the reference: identical values
-                    s.pos(0) = best;
+                    if (run) s.pos(0) = best;
                 }
             }
+        } else if (t < 11) {
+            row = t - 3;
+            run = (flags >> row) & 1u;
         } else if (t == 11) {
-            sel = view_selection(a, px, py, iter, flags, rng, s);
-            cur = a.planes[center];
+            PixelRng rng;
+            rng.init(a.seed, a.view_id, px, py, a.rng[center]);
+            const Selection sel = view_selection(a, px, py, iter, flags, rng, s);
+            a.rng[center] = rng.draw;
+            selected = sel.temp_selected;
+            weight_norm = sel.weight_norm;
             run = true;
-            pl = cur;
-            mask = sel.temp_selected;
+            pl = a.planes[center];
+            mask = selected;
+            if (geom) depth = depth_from_plane(c0, pl, px, py);
         } else if (refine) {
-            const int i = t - 12;
             // candidates (depth, normal): (rand, entry) (entry, rand) (rand, rand) (entry, perturbed) (perturbed, entry)
-            pl = (i == 1 || i == 2) ? plane_rand : (i == 3 ? plane_pert : plane0);
-            const float dc = (i == 0 || i == 2) ? depth_rand : (i == 4 ? depth_pert : depth0);
+            pl = s.held(t - 12);
+            const float dc = pl.w;
             pl.w = distance_to_origin(c0, px, py, dc, pl);
             run = true;
-            mask = sel.temp_selected;
+            mask = selected;
+            depth = depth_from_plane(c0, pl, px, py);
+            const float4 terms = s.held(kHeldTerms);
+            if (!(depth >= dmin && depth <= dmax)) {
+                mask = 0;
+            } else if (terms.z == 0.0f) {
+                limit = cost_now * weight_norm * kLimitMargin;
+            } else if (restricted_cost > 0.0f) {
+                const float lead = logf(prior_factor(dc, terms.x, s.held(kHeldPrior), pl, terms.y, two_dss, two_ass) /
+                                        restricted_cost) + kLogMargin;
+                if (lead > 0.0f)
+                    limit = sqrtf(lead * kPriorBeta / (1.0f + 0.2f * terms.y)) * weight_norm * kLimitMargin;
+                else
+                    mask = 0, limit = -1.0f;
+            }
         }
 
+        // The hypothesis against the views in `mask`: cost rows of the directions (slots 0-10,
+        // ComputeMultiViewCostVector, HPM.cu:490-495), or the weighted cost sum over the selected
+        // views (HPM.cu:1775-1786, 805-817).  The only place a half-sweep evaluates the NCC, so the
+        // kernel carries one copy.  The loop runs over view indices, the same for every lane: a
+        // variant in which each lane took its own k-th selected view ran three times slower on B200,
+        // because texture fetches with different texture objects across a warp serialise.
+        float wcost = 0.0f;
         if (run) {
             if (CNT) atomicAdd(a.hyp_count + 1, (unsigned long long)S);
-            const PlaneM pm = plane_m(a, pl);
-            eval_row(a, P, px, py, pm, mask, row, s);
+            PlaneM pm;
+            if (t < 11) {
+                const float4 m = cand[row];
+                pm.m[0] = m.x; pm.m[1] = m.y; pm.m[2] = m.z;
+            } else {
+                pm = plane_m(a, pl);
+            }
+#pragma unroll 1
+            for (int j = 0; j < S; ++j) {
+                if (!((mask >> j) & 1u)) continue;
+                const bool weighted = t >= 11;
+                const float c = ncc_view<CNT>(a, P, px, py, pm, j);
+                if (!weighted) {
+                    s.ca(row, j) = c;
+                } else {
+                    const float w = s.vw(j);
+                    float sx = 0.0f, sy = 0.0f, sd = 0.0f;
+                    if (geom)
+                        sd = geom_source_depth(a.depth_src[j + 1], a.dsw[j + 1], a.dsh[j + 1], a.fwd[j + 1].A,
+                                               a.fwd[j + 1].b, depth, px, py, sx, sy);
+                    if (geom)
+                        wcost += w * (c + 0.2f * geom_back_cost(a.bwd[j + 1].A, a.bwd[j + 1].b, sx, sy, sd, px, py));
+                    else
+                        wcost += w * c;
+                    if (wcost > limit) mask = 0;
+                }
+            }
         }
 
         if (t == 11) {
-            float fcl[8];
-#pragma unroll
-            for (int d = 0; d < 8; ++d) fcl[d] = s.fc(d);
-            if (!MAND || reliable) {
-                const int min_idx = find_min_index8(fcl);
+            float4 cur = pl;
+            if (!MAND || a.conf[center] >= 0.3) {
+                int min_idx = 0;  // ties: the last (HPM.cu:41-52)
+                float min_cost = s.fc(0);
+#pragma unroll 1
+                for (int d = 1; d < 8; ++d)
+                    if (s.fc(d) <= min_cost) { min_cost = s.fc(d); min_idx = d; }
                 const bool min_valid = flags & (1u << min_idx);
-                cost_now = selected_cost(a, px, py, cur, sel.temp_selected, sel.weight_norm, s);
+                cost_now = wcost / weight_norm;
                 a.costs[center] = cost_now;
                 const float cost_chk = cost_now;  // costs[center] as read by the NaN test
-                depth_now = depth_from_plane(c0, cur, px, py);
-                restricted_cost = 0.0f;
-                texture = 0.0f;
+                float depth_now = depth_from_plane(c0, cur, px, py);
+                float texture = 0.0f, depth_prior = 0.0f;
+                float4 pp = make_float4(0.f, 0.f, 0.f, 0.f);
                 float4 prior_pick = cur;  // prior mode: the maximum-score neighbour's plane, when valid
                 bool has_pick = false;
                 if (!MAND && prior) {
@@ -763,17 +952,18 @@ __device__ __forceinline__ void sweep_pixel(const RunArgs& a, const Scratch<NS, 
                     depth_prior = depth_from_plane(c0, pp, px, py);
                     texture = texture_term(a.canny, W, H, px, py);
                     if (a.pmask[center] > 0) {
-                        float rfc[8];
-#pragma unroll
+                        int max_idx = 0;  // ties: the last (HPM.cu:54-65)
+                        float max_score = 0.0f;
+#pragma unroll 1
                         for (int d = 0; d < 8; ++d) {
-                            rfc[d] = 0.0f;
+                            float score = 0.0f;
                             if (flags & (1u << d)) {
                                 const float4 pd = a.planes[s.pos(d)];
                                 const float dn = depth_from_plane(c0, pd, px, py);
-                                rfc[d] = prior_score(fcl[d], dn, depth_prior, pp, pd, texture, two_dss, two_ass);
+                                score = prior_score(s.fc(d), dn, depth_prior, pp, pd, texture, two_dss, two_ass);
                             }
+                            if (d == 0 || score >= max_score) { max_score = score; max_idx = d; }
                         }
-                        const int max_idx = find_max_index8(rfc);
                         const float rnow = prior_score(cost_now, depth_now, depth_prior, pp, cur, texture, two_dss,
                                                        two_ass);
                         if (flags & (1u << max_idx)) {
@@ -781,24 +971,24 @@ __device__ __forceinline__ void sweep_pixel(const RunArgs& a, const Scratch<NS, 
                             const float db = depth_from_plane(c0, pd, px, py);
                             prior_pick = pd;
                             has_pick = true;
-                            if (db >= dmin && db <= dmax && rfc[max_idx] > rnow) {
+                            if (db >= dmin && db <= dmax && max_score > rnow) {
                                 // depth_now is left alone: HPM.cu:1815 shadows it in this block, so
                                 // the refinement receives the pre-acceptance depth
                                 cur = pd;
                                 a.planes[center] = pd;
-                                a.costs[center] = fcl[max_idx];
-                                restricted_cost = rfc[max_idx];
-                                a.sel[center] = sel.temp_selected;
+                                a.costs[center] = s.fc(max_idx);
+                                restricted_cost = max_score;
+                                a.sel[center] = selected;
                             }
                         }
                     } else if (min_valid) {
                         const float4 pd = a.planes[s.pos(min_idx)];
                         const float db = depth_from_plane(c0, pd, px, py);
-                        if (db >= dmin && db <= dmax && fcl[min_idx] < cost_now) {
+                        if (db >= dmin && db <= dmax && min_cost < cost_now) {
                             depth_now = db;
                             cur = pd;
                             a.planes[center] = pd;
-                            a.costs[center] = fcl[min_idx];
+                            a.costs[center] = min_cost;
                         }
                     }
                 }
@@ -807,25 +997,29 @@ __device__ __forceinline__ void sweep_pixel(const RunArgs& a, const Scratch<NS, 
                 // whenever that direction is valid; prior mode never assigns it and holds the
                 // maximum-score neighbour's plane when valid.  Otherwise it starts as the
                 // pixel's current plane.
-                plane_now = (!MAND && prior && has_pick) ? prior_pick : cur;
+                float4 plane_now = (!MAND && prior && has_pick) ? prior_pick : cur;
                 if ((MAND || !prior) && min_valid) {
                     const float4 pd = a.planes[s.pos(min_idx)];
                     const float db = depth_from_plane(c0, pd, px, py);
                     plane_now = pd;
-                    if (db >= dmin && db <= dmax && fcl[min_idx] < cost_now) {
-                        depth_now = db; plane_now = pd; cost_now = fcl[min_idx];
-                        a.sel[center] = sel.temp_selected;
+                    if (db >= dmin && db <= dmax && min_cost < cost_now) {
+                        depth_now = db; plane_now = pd; cost_now = min_cost;
+                        a.sel[center] = selected;
                     }
                     if (cost_chk != cost_chk) {
                         if (!MAND) depth_now = db;
-                        plane_now = pd; cost_now = fcl[min_idx];
-                        a.sel[center] = sel.temp_selected;
+                        plane_now = pd; cost_now = min_cost;
+                        a.sel[center] = selected;
                     }
                 }
                 // PlaneHypothesisRefinement's random draws (HPM.cu:765-799), before any candidate is costed
                 refine = true;
-                use_prior = prior && a.pmask[center] > 0;
+                const bool use_prior = prior && a.pmask[center] > 0;
                 const float perturbation = 0.02f;
+                float4 plane_rand;
+                float depth_rand;
+                PixelRng rng;
+                rng.init(a.seed, a.view_id, px, py, a.rng[center]);
                 if (use_prior) {
                     depth_rand = rng.uniform() * 6 * depth_sigma + (depth_prior - 3 * depth_sigma);
                     plane_rand = perturbed_normal(c0, px, py, pp, rng, angle_sigma);
@@ -835,36 +1029,47 @@ __device__ __forceinline__ void sweep_pixel(const RunArgs& a, const Scratch<NS, 
                 }
                 const float dmin_p = (1 - perturbation) * depth_now;
                 const float dmax_p = (1 + perturbation) * depth_now;
-                depth_pert = rng.uniform() * (dmax_p - dmin_p) + dmin_p;
-                plane_pert = perturbed_normal(c0, px, py, plane_now, rng,
-                                              (float)(perturbation * 3.14159265358979323846));
-                plane0 = plane_now;
-                depth0 = depth_now;
+                const float depth_pert = rng.uniform() * (dmax_p - dmin_p) + dmin_p;
+                const float4 plane_pert = perturbed_normal(c0, px, py, plane_now, rng,
+                                                           (float)(perturbation * 3.14159265358979323846));
+                a.rng[center] = rng.draw;
+                s.hold(0, make_float4(plane_now.x, plane_now.y, plane_now.z, depth_rand));
+                s.hold(1, make_float4(plane_rand.x, plane_rand.y, plane_rand.z, depth_now));
+                s.hold(2, make_float4(plane_rand.x, plane_rand.y, plane_rand.z, depth_rand));
+                s.hold(3, make_float4(plane_pert.x, plane_pert.y, plane_pert.z, depth_now));
+                s.hold(4, make_float4(plane_now.x, plane_now.y, plane_now.z, depth_pert));
+                s.hold(kHeldNow, plane_now);
+                s.hold(kHeldPrior, pp);
+                s.hold(kHeldTerms, make_float4(depth_prior, texture, use_prior ? 1.0f : 0.0f, 0.0f));
             } else {
                 // mandatory consistency, unreliable pixel (HPM.cu:2684-2789)
                 const float beta = 0.18f;
-                float rfc[8];
-                const float mmc = sel.num_selected * 0.5f;
-#pragma unroll
-                for (int d = 0; d < 8; ++d) {
-                    rfc[d] = 0.0f;
-                    if (flags & (1u << d)) {
-                        const float cp = a.conf[s.pos(d)];
-                        const float gce = hpm_expf(-fcl[d] * fcl[d] / beta);
-                        const float dm = fmaxf(0.0f, mmc - cp);
-                        const float mce = (float)(0.5f + exp(-dm * dm / (mmc * mmc * 1.0)));
-                        rfc[d] = (cp > 0) ? fmaxf(3.0f, mce) * gce : mce * gce;
-                        if (cp > 0) fcl[d] = (float)(fcl[d] * fmin((double)hpm_expf(-cp * 2), 0.35));
-                    }
-                }
-                const int max_idx = find_max_index8(rfc);
-                float cost_u = selected_cost(a, px, py, cur, sel.temp_selected, sel.weight_norm, s);
+                const float mmc = __popc(selected) * 0.5f;
+                // score of a cost under a confidence (HPM.cu:2691-2716)
+                auto score_of = [&](float cost, float conf) {
+                    const float gce = hpm_expf(-cost * cost / beta);
+                    const float dm = fmaxf(0.0f, mmc - conf);
+                    const float mce = (float)(0.5f + exp(-dm * dm / (mmc * mmc * 1.0)));
+                    return (conf > 0) ? fmaxf(3.0f, mce) * gce : mce * gce;
+                };
+                float cost_u = wcost / weight_norm;
                 const float cost_chk = cost_u;
                 const float cc = a.conf[center];
-                const float gce = hpm_expf(-cost_u * cost_u / beta);
-                const float dm = fmaxf(0.0f, mmc - cc);
-                const float mce = (float)(0.5f + exp(-dm * dm / (mmc * mmc * 1.0)));
-                const float rnow = (cc > 0) ? fmaxf(3.0f, mce) * gce : mce * gce;
+                // the eight directions, then the pixel's own plane (d = 8)
+                int max_idx = 0;  // ties: the last (HPM.cu:54-65)
+                float max_score = 0.0f, max_cost = 0.0f, rnow = 0.0f;
+#pragma unroll 1
+                for (int d = 0; d < 9; ++d) {
+                    const bool own = d == 8;
+                    float score = 0.0f, cost = own ? cost_u : s.fc(d);
+                    if (own || (flags & (1u << d))) {
+                        const float cp = own ? cc : a.conf[s.pos(d)];
+                        score = score_of(cost, cp);
+                        if (!own && cp > 0) cost = (float)(cost * fmin((double)hpm_expf(-cp * 2), 0.35));
+                    }
+                    if (own) rnow = score;
+                    else if (d == 0 || score >= max_score) { max_score = score; max_idx = d; max_cost = cost; }
+                }
                 if (cc < 0.3) cost_u = (float)(cost_u * exp(0.2 + cc * 2));
                 else cost_u = cost_u * hpm_expf(-cc * 2);
                 float4 pu = cur;  // HPM.cu:2761: the neighbour's plane whenever that direction is valid
@@ -873,14 +1078,14 @@ __device__ __forceinline__ void sweep_pixel(const RunArgs& a, const Scratch<NS, 
                     const float4 pd = a.planes[pm];
                     pu = pd;
                     const float db = depth_from_plane(c0, pd, px, py);
-                    if (db >= dmin && db <= dmax && rfc[max_idx] > rnow) {
-                        pu = pd; cost_u = fcl[max_idx];
-                        a.sel[center] = sel.temp_selected;
+                    if (db >= dmin && db <= dmax && max_score > rnow) {
+                        pu = pd; cost_u = max_cost;
+                        a.sel[center] = selected;
                         a.conf[center] = (float)(0.5 * a.conf[pm]);
                     }
                     if (cost_chk != cost_chk) {
-                        pu = pd; cost_u = fcl[max_idx];
-                        a.sel[center] = sel.temp_selected;
+                        pu = pd; cost_u = max_cost;
+                        a.sel[center] = selected;
                         a.conf[center] = (float)(0.5 * a.conf[pm]);
                     }
                 }
@@ -888,41 +1093,39 @@ __device__ __forceinline__ void sweep_pixel(const RunArgs& a, const Scratch<NS, 
                 a.planes[center] = pu;
             }
         } else if (t >= 12 && refine) {
-            const int i = t - 12;
-            const float dc = (i == 0 || i == 2) ? depth_rand : (i == 4 ? depth_pert : depth0);
-            const float tc = selected_cost(a, px, py, pl, sel.temp_selected, sel.weight_norm, s);
-            const float db = depth_from_plane(c0, pl, px, py);
-            if (use_prior) {
-                const float rt = prior_score(tc, dc, depth_prior, pp, pl, texture, two_dss, two_ass);
-                if (db >= dmin && db <= dmax && rt > restricted_cost) {
-                    depth_now = db; plane_now = pl; cost_now = tc; restricted_cost = rt;
+            // a sum cut short by its limit, or of no view (weight_norm 0: NaN), is rejected here
+            const float tc = wcost / weight_norm;
+            if (depth >= dmin && depth <= dmax) {
+                const float4 terms = s.held(kHeldTerms);
+                if (terms.z == 0.0f) {
+                    if (tc < cost_now) {
+                        s.hold(kHeldNow, pl);
+                        cost_now = tc;
+                    }
+                } else if (limit >= 0.0f) {
+                    const float rt = prior_score(tc, s.held(t - 12).w, terms.x, s.held(kHeldPrior), pl, terms.y,
+                                                 two_dss, two_ass);
+                    if (rt > restricted_cost) {
+                        s.hold(kHeldNow, pl);
+                        cost_now = tc;
+                        restricted_cost = rt;
+                    }
                 }
-            } else if (db >= dmin && db <= dmax && tc < cost_now) {
-                depth_now = db; plane_now = pl; cost_now = tc;
             }
         }
     }
 
-    if (refine) {
-        if (!MAND && hier) {
-            if (cost_now < a.pre_costs[center] - 0.1f) {
-                a.costs[center] = cost_now;
-                a.planes[center] = plane_now;
-            }
-        } else {
-            a.costs[center] = cost_now;
-            a.planes[center] = plane_now;
-        }
+    if (refine && (MAND || !hier || cost_now < a.pre_costs[center] - 0.1f)) {
+        a.costs[center] = cost_now;
+        a.planes[center] = s.held(kHeldNow);
     }
-    a.rng[center] = rng.draw;
 }
 
 template <int NS, int BLK, bool MAND, bool CNT>
-__global__ void __launch_bounds__(BLK, HPM_SWEEP_MIN_BLOCKS) k_half_sweep(const __grid_constant__ RunArgs a, int color, int iter) {
+__global__ void __launch_bounds__(BLK, kSweepBlocks) k_half_sweep(const __grid_constant__ RunArgs a, int color, int iter) {
     extern __shared__ float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    const Scratch<NS, BLK, CNT> s{ smem + tid };
-    sweep_pixel<NS, BLK, MAND, CNT>(a, s, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y,
+    sweep_pixel<NS, BLK, MAND, CNT>(a, smem + tid, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y,
                                     color, iter);
 }
 
@@ -931,7 +1134,7 @@ __global__ void __launch_bounds__(BLK, HPM_SWEEP_MIN_BLOCKS) k_half_sweep(const 
 // whole warps idle instead of holding lanes of working ones.  Pixels of one colour read only the
 // other colour's state, so the mapping does not change any result.
 template <int NS, int BLK, bool CNT>
-__global__ void __launch_bounds__(BLK, HPM_SWEEP_MIN_BLOCKS) k_half_sweep_listed(const __grid_constant__ RunArgs a,
+__global__ void __launch_bounds__(BLK, kSweepBlocks) k_half_sweep_listed(const __grid_constant__ RunArgs a,
                                                                                  int color, int iter) {
     extern __shared__ float smem[];
     const int pair = blockIdx.y * blockDim.y + threadIdx.y;
@@ -940,10 +1143,10 @@ __global__ void __launch_bounds__(BLK, HPM_SWEEP_MIN_BLOCKS) k_half_sweep_listed
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= a.active_n[k]) return;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    const Scratch<NS, BLK, CNT> s{ smem + tid };
-    sweep_pixel<NS, BLK, false, CNT>(a, s, a.active_px[(size_t)k * a.W + x], pair, color, iter);
+    sweep_pixel<NS, BLK, false, CNT>(a, smem + tid, a.active_px[(size_t)k * a.W + x], pair, color, iter);
 }
 
+#ifndef HPM_NS
 // The pixels a prior-mode half-sweep updates (CheckerboardPropagation returns at once where
 // confidence > 0.3 or the prior mask is clear, HPM.cu:1352-1365): one warp per (row pair, colour)
 // writes their columns in increasing order and their count.
@@ -972,15 +1175,15 @@ cudaError_t launch_prior_active(const RunArgs& a, int* px, int* n, cudaStream_t 
     k_prior_active<<<dim3(a.cover_pairs, 2), 32, 0, st>>>(a, px, n);
     return cudaGetLastError();
 }
+#endif
 
 // The batched form of k_half_sweep_listed: tile t of run k maps to columns of that run's work lists.
 template <int NS, int BLK, bool CNT>
-__global__ void __launch_bounds__(BLK, HPM_SWEEP_MIN_BLOCKS)
+__global__ void __launch_bounds__(BLK, kSweepBlocks)
     k_half_sweep_batch_listed(const RunArgs* __restrict__ args, const int* __restrict__ tile_start, int n,
                               int color, int iter) {
     extern __shared__ float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    const Scratch<NS, BLK, CNT> s{ smem + tid };
     const int total = __ldg(tile_start + n);
     for (int b = blockIdx.x; b < total; b += gridDim.x) {
         const int k = batch_run_of(tile_start, n, b);
@@ -992,28 +1195,28 @@ __global__ void __launch_bounds__(BLK, HPM_SWEEP_MIN_BLOCKS)
         if (pair >= a.cover_pairs) continue;
         const int r = color * a.cover_pairs + pair;
         if (x >= a.active_n[r]) continue;
-        sweep_pixel<NS, BLK, false, CNT>(a, s, a.active_px[(size_t)r * a.W + x], pair, color, iter);
+        sweep_pixel<NS, BLK, false, CNT>(a, smem + tid, a.active_px[(size_t)r * a.W + x], pair, color, iter);
     }
 }
 
 template <int NS, int BLK, bool MAND, bool CNT>
-__global__ void __launch_bounds__(BLK, HPM_SWEEP_MIN_BLOCKS)
+__global__ void __launch_bounds__(BLK, kSweepBlocks)
     k_half_sweep_batch(const RunArgs* __restrict__ args, const int* __restrict__ tile_start, int n, int color,
                        int iter) {
     extern __shared__ float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    const Scratch<NS, BLK, CNT> s{ smem + tid };
     const int total = __ldg(tile_start + n);
     for (int b = blockIdx.x; b < total; b += gridDim.x) {
         const int k = batch_run_of(tile_start, n, b);
         const RunArgs& a = args[k];
         const int t = b - __ldg(tile_start + k);
         const int tx = (a.W + blockDim.x - 1) / blockDim.x;
-        sweep_pixel<NS, BLK, MAND, CNT>(a, s, (t % tx) * blockDim.x + threadIdx.x,
+        sweep_pixel<NS, BLK, MAND, CNT>(a, smem + tid, (t % tx) * blockDim.x + threadIdx.x,
                                         (t / tx) * blockDim.y + threadIdx.y, color, iter);
     }
 }
 
+#ifndef HPM_NS
 __global__ void k_export(const __grid_constant__ RunArgs a) {
     const int px = blockIdx.x * blockDim.x + threadIdx.x;
     const int py = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1030,151 +1233,143 @@ __global__ void k_eval_costs(const __grid_constant__ RunArgs a, int n, const int
     if (k >= n) return;
     const int x = px[2 * k], y = px[2 * k + 1];
     Patch P;
-    build_patch(a, x, y, P);
+    float tmp[kPatchWords];
+    build_patch(a, x, y, P, tmp);
     const float4 pl = planes[k];
     const PlaneM pm = plane_m(a, pl);
-    for (int j = 0; j < a.S; ++j) out[(size_t)k * a.S + j] = ncc_view(a, P, x, y, pm, j);
+    for (int j = 0; j < a.S; ++j) out[(size_t)k * a.S + j] = ncc_view<false>(a, P, x, y, pm, j);
 }
+#endif
 
 // ---------------------------------------------------------------- launchers
 
-template <int NS>
-static constexpr int block_threads() { return NS <= 10 ? 128 : (NS <= 16 ? 64 : 32); }
+#ifndef HPM_NS
+cudaError_t launch_weight_table(const hpm_params& prm, float* out, cudaStream_t st) {
+    const float two_ss = 2.0f * prm.sigma_spatial * prm.sigma_spatial;
+    const float two_sc = 2.0f * prm.sigma_color * prm.sigma_color;
+    k_weight_table<<<kWeightRows, 256, 0, st>>>(two_ss, two_sc, out);
+    return cudaGetLastError();
+}
+#endif
 
 template <int NS, bool CNT>
-static cudaError_t init_impl(const RunArgs& a, cudaStream_t st) {
+cudaError_t init_impl(const RunArgs& a, cudaStream_t st) {
     constexpr int BLK = 128;
-    const size_t shm = sizeof(float) * Scratch<NS, BLK>::kWords * BLK;
+    const size_t shm = sizeof(float) * InitScratch<NS, BLK>::kWords * BLK;
     auto k = k_random_init<NS, BLK, CNT>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-    if (e != cudaSuccess) return e;
     dim3 block(32, 4), grid((a.W + 31) / 32, (a.H + 3) / 4);
     k<<<grid, block, shm, st>>>(a);
     return cudaGetLastError();
 }
 
+template <int NS>
+static constexpr size_t sweep_smem() {
+    return sizeof(float) * Scratch<NS, kSweepThreads>::kWords * kSweepThreads;
+}
+
 template <int NS, bool MAND, bool CNT>
-static cudaError_t sweep_impl(const RunArgs& a, int color, int iter, cudaStream_t st) {
-    constexpr int BLK = block_threads<NS>();
-    const size_t shm = sizeof(float) * Scratch<NS, BLK>::kWords * BLK;
-    auto k = k_half_sweep<NS, BLK, MAND, CNT>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-    if (e != cudaSuccess) return e;
-#ifndef HPM_SWEEP_BX
-#define HPM_SWEEP_BX 32
-#endif
-    constexpr int BX = HPM_SWEEP_BX < BLK ? HPM_SWEEP_BX : BLK;
+cudaError_t sweep_impl(const RunArgs& a, int color, int iter, cudaStream_t st) {
+    constexpr int BLK = kSweepThreads, BX = 32;
     dim3 block(BX, BLK / BX), grid((a.W + BX - 1) / BX, (a.cover_pairs + BLK / BX - 1) / (BLK / BX));
-    if (!MAND && a.active_px) {
-        auto kl = k_half_sweep_listed<NS, BLK, CNT>;
-        if ((e = cudaFuncSetAttribute(kl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm)) != cudaSuccess)
-            return e;
-        kl<<<grid, block, shm, st>>>(a, color, iter);
-        return cudaGetLastError();
-    }
-    k<<<grid, block, shm, st>>>(a, color, iter);
+    if (!MAND && a.active_px)
+        k_half_sweep_listed<NS, BLK, CNT><<<grid, block, sweep_smem<NS>(), st>>>(a, color, iter);
+    else
+        k_half_sweep<NS, BLK, MAND, CNT><<<grid, block, sweep_smem<NS>(), st>>>(a, color, iter);
     return cudaGetLastError();
 }
 
 template <int NS, bool CNT>
-static cudaError_t init_batch_impl(const BatchLaunch& bl, cudaStream_t st) {
+cudaError_t init_batch_impl(const BatchLaunch& bl, cudaStream_t st) {
     constexpr int BLK = 128;
-    const size_t shm = sizeof(float) * Scratch<NS, BLK>::kWords * BLK;
+    const size_t shm = sizeof(float) * InitScratch<NS, BLK>::kWords * BLK;
     auto k = k_random_init_batch<NS, BLK, CNT>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-    if (e != cudaSuccess) return e;
     const int grid = bl.grid_blocks > 0 && bl.grid_blocks < bl.tiles ? bl.grid_blocks : bl.tiles;
     k<<<grid, dim3(16, 8), shm, st>>>(bl.args, bl.tile_start, bl.n);
     return cudaGetLastError();
 }
 
 template <int NS, bool MAND, bool CNT>
-static cudaError_t sweep_batch_impl(const BatchLaunch& bl, int color, int iter, cudaStream_t st) {
-    constexpr int BLK = block_threads<NS>();
-    const size_t shm = sizeof(float) * Scratch<NS, BLK>::kWords * BLK;
-    auto k = (!MAND && bl.listed) ? k_half_sweep_batch_listed<NS, BLK, CNT> : k_half_sweep_batch<NS, BLK, MAND, CNT>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-    if (e != cudaSuccess) return e;
+cudaError_t sweep_batch_impl(const BatchLaunch& bl, int color, int iter, cudaStream_t st) {
+    constexpr int BLK = kSweepThreads;
+    auto k = (!MAND && bl.listed) ? k_half_sweep_batch_listed<NS, BLK, CNT>
+                                  : k_half_sweep_batch<NS, BLK, MAND, CNT>;
     const int grid = bl.grid_blocks > 0 && bl.grid_blocks < bl.tiles ? bl.grid_blocks : bl.tiles;
     const int bx = (bl.bx > 0 && bl.bx <= BLK) ? bl.bx : 32;
-    k<<<grid, dim3(bx, BLK / bx), shm, st>>>(bl.args, bl.tile_start, bl.n, color, iter);
+    k<<<grid, dim3(bx, BLK / bx), sweep_smem<NS>(), st>>>(bl.args, bl.tile_start, bl.n, color, iter);
     return cudaGetLastError();
 }
 
-template <int NS, bool MAND, bool CNT>
-static int sweep_batch_occupancy() {
-    constexpr int BLK = block_threads<NS>();
-    const size_t shm = sizeof(float) * Scratch<NS, BLK>::kWords * BLK;
-    auto k = k_half_sweep_batch<NS, BLK, MAND, CNT>;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm) != cudaSuccess) return 0;
+template <int NS, bool MAND>
+int sweep_batch_occupancy() {
+    constexpr int BLK = kSweepThreads;
     int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, BLK, shm) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_half_sweep_batch<NS, BLK, MAND, false>, BLK,
+                                                      sweep_smem<NS>()) != cudaSuccess)
+        return 0;
     return blocks;
 }
 
-template <bool CNT>
-static cudaError_t init_dispatch(const RunArgs& a, cudaStream_t st) {
-    if (a.S <= 4) return init_impl<4, CNT>(a, st);
-    if (a.S <= 10) return init_impl<10, CNT>(a, st);
-    if (a.S <= 16) return init_impl<16, CNT>(a, st);
-    return init_impl<31, CNT>(a, st);
-}
+// The kernels are compiled once per source count they are specialised for, each in an object of its own
+// (-DHPM_NS=4, 10, 16, 31); the object without HPM_NS holds the dispatch.
+#define HPM_SWEEP_FORMS(linkage, NS)                                                        \
+    linkage template cudaError_t init_impl<NS, false>(const RunArgs&, cudaStream_t);        \
+    linkage template cudaError_t init_impl<NS, true>(const RunArgs&, cudaStream_t);         \
+    linkage template cudaError_t init_batch_impl<NS, false>(const BatchLaunch&, cudaStream_t); \
+    linkage template cudaError_t init_batch_impl<NS, true>(const BatchLaunch&, cudaStream_t);  \
+    HPM_SWEEP_FORMS_OF(linkage, NS, false, false)                                           \
+    HPM_SWEEP_FORMS_OF(linkage, NS, false, true)                                            \
+    HPM_SWEEP_FORMS_OF(linkage, NS, true, false)                                            \
+    HPM_SWEEP_FORMS_OF(linkage, NS, true, true)                                             \
+    linkage template int sweep_batch_occupancy<NS, false>();                                \
+    linkage template int sweep_batch_occupancy<NS, true>();
+#define HPM_SWEEP_FORMS_OF(linkage, NS, MAND, CNT)                                                     \
+    linkage template cudaError_t sweep_impl<NS, MAND, CNT>(const RunArgs&, int, int, cudaStream_t);    \
+    linkage template cudaError_t sweep_batch_impl<NS, MAND, CNT>(const BatchLaunch&, int, int, cudaStream_t);
+
+#ifdef HPM_NS
+HPM_SWEEP_FORMS(, HPM_NS)
+#else
+HPM_SWEEP_FORMS(extern, 4)
+HPM_SWEEP_FORMS(extern, 10)
+HPM_SWEEP_FORMS(extern, 16)
+HPM_SWEEP_FORMS(extern, 31)
+
+// The kernel specialisation of a run: the source count rounded up to 4, 10, 16 or 31.
+#define HPM_BY_SOURCES(s, fn, ...) \
+    ((s) <= 4 ? fn<4, __VA_ARGS__>  \
+              : (s) <= 10 ? fn<10, __VA_ARGS__> : (s) <= 16 ? fn<16, __VA_ARGS__> : fn<31, __VA_ARGS__>)
 
 cudaError_t launch_random_init(const RunArgs& a, cudaStream_t st) {
-    return a.hyp_count ? init_dispatch<true>(a, st) : init_dispatch<false>(a, st);
-}
-
-template <bool MAND, bool CNT>
-static cudaError_t sweep_dispatch(const RunArgs& a, int color, int iter, cudaStream_t st) {
-    if (a.S <= 4) return sweep_impl<4, MAND, CNT>(a, color, iter, st);
-    if (a.S <= 10) return sweep_impl<10, MAND, CNT>(a, color, iter, st);
-    if (a.S <= 16) return sweep_impl<16, MAND, CNT>(a, color, iter, st);
-    return sweep_impl<31, MAND, CNT>(a, color, iter, st);
+    return a.hyp_count ? HPM_BY_SOURCES(a.S, init_impl, true)(a, st) : HPM_BY_SOURCES(a.S, init_impl, false)(a, st);
 }
 
 cudaError_t launch_half_sweep(const RunArgs& a, int color, int iter, cudaStream_t st) {
     const bool mand = a.prm.mode & HPM_MODE_MAND;
     if (a.hyp_count)
-        return mand ? sweep_dispatch<true, true>(a, color, iter, st) : sweep_dispatch<false, true>(a, color, iter, st);
-    return mand ? sweep_dispatch<true, false>(a, color, iter, st) : sweep_dispatch<false, false>(a, color, iter, st);
-}
-
-template <bool CNT>
-static cudaError_t init_batch_dispatch(const BatchLaunch& bl, cudaStream_t st) {
-    if (bl.max_s <= 4) return init_batch_impl<4, CNT>(bl, st);
-    if (bl.max_s <= 10) return init_batch_impl<10, CNT>(bl, st);
-    if (bl.max_s <= 16) return init_batch_impl<16, CNT>(bl, st);
-    return init_batch_impl<31, CNT>(bl, st);
+        return mand ? HPM_BY_SOURCES(a.S, sweep_impl, true, true)(a, color, iter, st)
+                    : HPM_BY_SOURCES(a.S, sweep_impl, false, true)(a, color, iter, st);
+    return mand ? HPM_BY_SOURCES(a.S, sweep_impl, true, false)(a, color, iter, st)
+                : HPM_BY_SOURCES(a.S, sweep_impl, false, false)(a, color, iter, st);
 }
 
 cudaError_t launch_random_init_batch(const BatchLaunch& bl, cudaStream_t st) {
-    return bl.count ? init_batch_dispatch<true>(bl, st) : init_batch_dispatch<false>(bl, st);
-}
-
-template <bool MAND, bool CNT>
-static cudaError_t sweep_batch_dispatch(const BatchLaunch& bl, int color, int iter, cudaStream_t st) {
-    if (bl.max_s <= 4) return sweep_batch_impl<4, MAND, CNT>(bl, color, iter, st);
-    if (bl.max_s <= 10) return sweep_batch_impl<10, MAND, CNT>(bl, color, iter, st);
-    if (bl.max_s <= 16) return sweep_batch_impl<16, MAND, CNT>(bl, color, iter, st);
-    return sweep_batch_impl<31, MAND, CNT>(bl, color, iter, st);
+    return bl.count ? HPM_BY_SOURCES(bl.max_s, init_batch_impl, true)(bl, st)
+                    : HPM_BY_SOURCES(bl.max_s, init_batch_impl, false)(bl, st);
 }
 
 cudaError_t launch_half_sweep_batch(const BatchLaunch& bl, int color, int iter, cudaStream_t st) {
     if (bl.count)
-        return bl.mand ? sweep_batch_dispatch<true, true>(bl, color, iter, st)
-                       : sweep_batch_dispatch<false, true>(bl, color, iter, st);
-    return bl.mand ? sweep_batch_dispatch<true, false>(bl, color, iter, st)
-                   : sweep_batch_dispatch<false, false>(bl, color, iter, st);
+        return bl.mand ? HPM_BY_SOURCES(bl.max_s, sweep_batch_impl, true, true)(bl, color, iter, st)
+                       : HPM_BY_SOURCES(bl.max_s, sweep_batch_impl, false, true)(bl, color, iter, st);
+    return bl.mand ? HPM_BY_SOURCES(bl.max_s, sweep_batch_impl, true, false)(bl, color, iter, st)
+                   : HPM_BY_SOURCES(bl.max_s, sweep_batch_impl, false, false)(bl, color, iter, st);
 }
 
 int half_sweep_batch_occupancy(int max_s, bool mand) {
-    if (max_s <= 4) return mand ? sweep_batch_occupancy<4, true, false>() : sweep_batch_occupancy<4, false, false>();
-    if (max_s <= 10) return mand ? sweep_batch_occupancy<10, true, false>() : sweep_batch_occupancy<10, false, false>();
-    if (max_s <= 16) return mand ? sweep_batch_occupancy<16, true, false>() : sweep_batch_occupancy<16, false, false>();
-    return mand ? sweep_batch_occupancy<31, true, false>() : sweep_batch_occupancy<31, false, false>();
+    return mand ? HPM_BY_SOURCES(max_s, sweep_batch_occupancy, true)() : HPM_BY_SOURCES(max_s, sweep_batch_occupancy, false)();
 }
 
-int half_sweep_block_threads(int max_s) { return max_s <= 10 ? 128 : (max_s <= 16 ? 64 : 32); }
+int half_sweep_block_threads() { return kSweepThreads; }
 
 cudaError_t launch_export(const RunArgs& a, cudaStream_t st) {
     dim3 block(32, 8), grid((a.W + 31) / 32, (a.H + 7) / 8);
@@ -1188,5 +1383,7 @@ cudaError_t launch_eval_costs(const RunArgs& a, int n, const int32_t* px, const 
     k_eval_costs<<<(n + 127) / 128, 128, 0, st>>>(a, n, px, planes, out);
     return cudaGetLastError();
 }
+
+#endif  // HPM_NS
 
 }  // namespace hpm

@@ -45,6 +45,12 @@ struct RunArgs {
     const int* active_n;            // [colour * cover_pairs + pair]
     hpm_params prm;
     int S, W, H, cover_pairs;
+    int whole_levels;               // the reference's grey image holds whole levels 0..255 only
+    const uint8_t* ref_bytes;       // whole_levels: the same image as bytes
+    const float* weights;           // whole_levels: its bilateral weights, kWeightTable values (launch_weight_table)
+    // what a fetch is carried through, fma(fetch, tex_scale, tex_bias) - tex_bias: (1, 0) for textures of
+    // the format in use, (65280, 1.5 * 2^23) for the 8-bit copies of F32 images (Ctx::bind_bytes)
+    float tex_scale, tex_bias;
     uint64_t seed;
     uint32_t view_id;
     // profiling only (null otherwise): (hypothesis, source view) pairs costed
@@ -55,12 +61,15 @@ struct RunArgs {
     unsigned long long* hyp_count;
 };
 
+constexpr int kWeightTable = 6 * 256;  // six patch distances x level differences 0..255
+
 // Passed by value as a kernel parameter: sm_70 and later accept up to 32764 bytes.
 static_assert(sizeof(RunArgs) <= 32764, "RunArgs exceeds the kernel parameter limit");
 
 
 // Host launchers (pm_kernels.cu).  Return cudaError_t of the launch.
 cudaError_t launch_random_init(const RunArgs& a, cudaStream_t st);
+cudaError_t launch_weight_table(const hpm_params& prm, float* out, cudaStream_t st);
 cudaError_t launch_half_sweep(const RunArgs& a, int color, int iter, cudaStream_t st);
 // Prior mode: the compacted columns of the pixels the half-sweeps update (W * cover_pairs ints and
 // cover_pairs counts per colour in px / n), for RunArgs::active_px / active_n.
@@ -91,7 +100,7 @@ cudaError_t launch_random_init_batch(const BatchLaunch& bl, cudaStream_t st);
 cudaError_t launch_half_sweep_batch(const BatchLaunch& bl, int color, int iter, cudaStream_t st);
 // Resident blocks per SM of the batched half-sweep kernel, and its block size.
 int half_sweep_batch_occupancy(int max_s, bool mand);
-int half_sweep_block_threads(int max_s);
+int half_sweep_block_threads();
 
 // Rows covered by the checkerboard launch of RunPatchMatch (HPM.cu:3004-3011):
 // the grid spans ceil(floor(H/2)/16)*16 row pairs.

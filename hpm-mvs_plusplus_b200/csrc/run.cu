@@ -43,6 +43,100 @@ __global__ void k_to_u8(const float* __restrict__ src, int n, uint8_t* __restric
     if (i < n) dst[i] = (uint8_t)fminf(255.0f, fmaxf(0.0f, rintf(src[i])));
 }
 
+__global__ void k_whole_levels(const float* __restrict__ gray, int n, int* __restrict__ whole) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float v = gray[i];
+        if (!(v >= 0.0f && v <= 255.0f && v == rintf(v))) *whole = 0;
+    }
+}
+
+// Finds out which of a run's images hold whole levels 0..255 only, as every image made by
+// hpm_prepare_level does.  Images from hpm_set_view are looked at once, when a run first uses them;
+// under stream capture, where their contents can still change, they are taken as they are.
+int Ctx::look_at_levels(int ref, const int32_t* srcs, int n_src) {
+    bool unknown = views[ref].whole_levels < 0;
+    for (int j = 0; j < n_src; ++j) unknown = unknown || views[srcs[j]].whole_levels < 0;
+    if (!unknown) return HPM_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(stream, &cap);
+    if (e != cudaSuccess) return cuda_fail(e, "capture status");
+    if (cap != cudaStreamCaptureStatusNone) return HPM_OK;
+    if ((e = ensure_buf(level_flags, level_flags_cap, HPM_MAX_VIEWS)) != cudaSuccess) return cuda_fail(e, "alloc level flags");
+    int flags[HPM_MAX_VIEWS];
+    e = cudaMemsetAsync(level_flags, 0xff, sizeof(flags), stream);
+    if (e != cudaSuccess) return cuda_fail(e, "grey levels");
+    for (int j = -1; j < n_src; ++j) {
+        const int view = j < 0 ? ref : srcs[j];
+        const ViewState& v = views[view];
+        if (v.whole_levels >= 0) continue;
+        const int n = v.w * v.h;
+        k_whole_levels<<<std::min((n + 255) / 256, 1184), 256, 0, stream>>>(v.gray, n, level_flags + view);
+        ++launches;
+    }
+    e = cudaMemcpyAsync(flags, level_flags, sizeof(flags), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e != cudaSuccess) return cuda_fail(e, "grey levels");
+    for (int j = -1; j < n_src; ++j) {
+        const int view = j < 0 ? ref : srcs[j];
+        ViewState& v = views[view];
+        if (v.whole_levels >= 0) continue;
+        v.whole_levels = flags[view] ? 1 : 0;
+        if (v.whole_levels == 1) {
+            const int rc = bind_bytes(view);
+            if (rc) return rc;
+        }
+    }
+    return HPM_OK;
+}
+
+static cudaError_t make_texture(cudaArray_t arr, int addr_mode, cudaTextureReadMode read, cudaTextureObject_t* tex) {
+    cudaResourceDesc rd;
+    memset(&rd, 0, sizeof(rd));
+    rd.resType = cudaResourceTypeArray;
+    rd.res.array.array = arr;
+    cudaTextureDesc td;
+    memset(&td, 0, sizeof(td));
+    td.addressMode[0] = td.addressMode[1] = addr_mode == 1 ? cudaAddressModeWrap : cudaAddressModeClamp;
+    td.filterMode = cudaFilterModeLinear;
+    td.readMode = read;
+    td.normalizedCoords = 0;
+    return cudaCreateTextureObject(tex, &rd, &td, nullptr);
+}
+
+// 8-bit copy of a view's image of whole levels.  The unit filters with weights of 1/256, so an F32
+// fetch is a whole multiple N of 1/256 level, N <= 255 * 256, and an 8-bit fetch is N / 65280 rounded
+// to a multiple of 1/65535: fetch * 65280 lies within 0.4999 of N, and rounding it to the nearest
+// integer gives N, hence the F32 fetch times 256, for every N (tests/test_gpu_whole_levels.py).  A
+// quarter of the bytes puts neighbouring samples of a warp on fewer lines.
+int Ctx::bind_bytes(int view) {
+    ViewState& v = views[view];
+    const size_t n = (size_t)v.w * v.h;
+    cudaError_t e = ensure_buf(v.bytes, v.bytes_cap, n);
+    if (e != cudaSuccess) return cuda_fail(e, "alloc byte image");
+    k_to_u8<<<(int)((n + 255) / 256), 256, 0, stream>>>(v.gray, (int)n, v.bytes);
+    ++launches;
+    if (v.arr_fmt != HPM_TEX_F32) return HPM_OK;
+    if (!v.arr8 || v.arr8_w != v.w || v.arr8_h != v.h || v.arr8_mode != v.arr_mode) {
+        if (v.tex8) { cudaDestroyTextureObject(v.tex8); v.tex8 = 0; }
+        if (v.arr8 && (v.arr8_w != v.w || v.arr8_h != v.h)) {
+            cudaFreeArray(v.arr8);
+            v.arr8 = nullptr;
+        }
+        if (!v.arr8) {
+            const cudaChannelFormatDesc fd = cudaCreateChannelDesc(8, 0, 0, 0, cudaChannelFormatKindUnsigned);
+            if ((e = cudaMallocArray(&v.arr8, &fd, v.w, v.h)) != cudaSuccess) return cuda_fail(e, "alloc byte image array");
+            v.arr8_w = v.w; v.arr8_h = v.h;
+        }
+        if ((e = make_texture(v.arr8, v.arr_mode, cudaReadModeNormalizedFloat, &v.tex8)) != cudaSuccess)
+            return cuda_fail(e, "create byte texture");
+        v.arr8_mode = v.arr_mode;
+    }
+    e = cudaMemcpy2DToArrayAsync(v.arr8, 0, 0, v.bytes, (size_t)v.w, (size_t)v.w, v.h, cudaMemcpyDeviceToDevice, stream);
+    if (e != cudaSuccess) return cuda_fail(e, "copy byte image to array");
+    v.bytes_bound = true;
+    return HPM_OK;
+}
+
 int Ctx::bind_texture(int view) {
     ViewState& v = views[view];
     cudaError_t e;
@@ -65,19 +159,8 @@ int Ctx::bind_texture(int view) {
             v.arr_w = v.w; v.arr_h = v.h;
             v.arr_fmt = tex_format;
         }
-        cudaResourceDesc rd;
-        memset(&rd, 0, sizeof(rd));
-        rd.resType = cudaResourceTypeArray;
-        rd.res.array.array = v.arr;
-        cudaTextureDesc td;
-        memset(&td, 0, sizeof(td));
-        const cudaTextureAddressMode am = addr_mode == 1 ? cudaAddressModeWrap : cudaAddressModeClamp;
-        td.addressMode[0] = am;
-        td.addressMode[1] = am;
-        td.filterMode = cudaFilterModeLinear;
-        td.readMode = tex_format == HPM_TEX_U8 ? cudaReadModeNormalizedFloat : cudaReadModeElementType;
-        td.normalizedCoords = 0;
-        e = cudaCreateTextureObject(&v.tex, &rd, &td, nullptr);
+        e = make_texture(v.arr, addr_mode,
+                         tex_format == HPM_TEX_U8 ? cudaReadModeNormalizedFloat : cudaReadModeElementType, &v.tex);
         if (e != cudaSuccess) return cuda_fail(e, "create texture");
         v.arr_mode = addr_mode;
     }
@@ -103,7 +186,8 @@ int Ctx::bind_texture(int view) {
                                      cudaMemcpyDeviceToDevice, stream);
     }
     if (e != cudaSuccess) return cuda_fail(e, "copy image to array");
-    return HPM_OK;
+    v.bytes_bound = false;
+    return v.whole_levels == 1 ? bind_bytes(view) : HPM_OK;
 }
 
 int Ctx::fill_run_args(int ref, const int32_t* srcs, int n_src, const hpm_params* params, RunArgs& a) {
@@ -131,6 +215,7 @@ int Ctx::fill_run_args(int ref, const int32_t* srcs, int n_src, const hpm_params
     // 8-bit textures return grey / 255; the NCC is scale-free, only the flat-source test scales
     a.var_s_min = tex_format == HPM_TEX_U8 ? 1e-5f / (255.0f * 255.0f) : 1e-5f;
     a.ncc_shift = ncc_mode == HPM_NCC_SHIFTED ? 1 : 0;
+    a.tex_scale = 1.0f;
     a.ref_img = rv.gray;
     a.prm = *params;
     a.S = n_src;
@@ -150,7 +235,9 @@ int Ctx::prepare_run(int ref, const int32_t* srcs, int n_src, const hpm_params* 
     if (e != cudaSuccess) return cuda_fail(e, "alloc run buffers");
     RunBufs b;
     b.planes = planes; b.costs = costs; b.pre_costs = pre_costs; b.sel = sel; b.rng = rng; b.conf = conf;
-    return prepare_run_into(ref, srcs, n_src, params, texture_level, seed, b, a);
+    const int rc = prepare_run_into(ref, srcs, n_src, params, texture_level, seed, b, a);
+    if (rc) return rc;
+    return take_whole_levels(ref, srcs, weights, a);
 }
 
 // The hypothesis reload and run setup of one run (HPM.cpp:741-906, 942-984)
@@ -244,6 +331,7 @@ int Ctx::prepare_run_into(int ref, const int32_t* srcs, int n_src, const hpm_par
     } else {
         a.prm.mode &= ~HPM_MODE_UPSAMPLE;
     }
+    if ((rc = look_at_levels(ref, srcs, n_src))) return rc;
     const bool want_texture = !prior && !mand;
     if (want_texture) {
         e = ensure_map(ref, HPM_MAP_TEXTURE0 + texture_level, W, H);
@@ -251,6 +339,27 @@ int Ctx::prepare_run_into(int ref, const int32_t* srcs, int n_src, const hpm_par
         a.texture = rv.maps[HPM_MAP_TEXTURE0 + texture_level].ptr;
     }
 
+    return HPM_OK;
+}
+
+// What a run gains from images of whole levels: the reference's bytes and weight table (pm_kernels.cu,
+// build_patch), and the sources' 8-bit textures when every source has one.
+int Ctx::take_whole_levels(int ref, const int32_t* srcs, float* weights, RunArgs& a) {
+    if (views[ref].whole_levels == 1) {
+        cudaError_t e = launch_weight_table(a.prm, weights, stream);
+        if (e != cudaSuccess) return cuda_fail(e, "weight table");
+        ++launches;
+        a.whole_levels = 1;
+        a.ref_bytes = views[ref].bytes;
+        a.weights = weights;
+    }
+    for (int j = 0; j < a.S; ++j)
+        if (!views[srcs[j]].bytes_bound) return HPM_OK;
+    // fetches become multiples of 1/256 level, the moments of the source grow by powers of two
+    for (int j = 0; j < a.S; ++j) a.tex[j + 1] = views[srcs[j]].tex8;
+    a.tex_scale = 65280.0f;
+    a.tex_bias = 12582912.0f;
+    a.var_s_min *= 65536.0f;
     return HPM_OK;
 }
 
