@@ -10,16 +10,32 @@
 //
 // Parallel form used here, per view i (views stay sequential):
 //   1. candidates (parallel over pixels q and sources j): the source pixel
-//      P[q][j] and whether the geometric test passes, T[q][j], ignoring masks;
+//      P[q][j] and whether the geometric test passes, T[q][j], ignoring the
+//      marks that view i itself sets;
 //   2. a causal fixed point: eff[q][j] = T[q][j] and P[q][j] not marked before q.
-//      Each Jacobi iteration computes acceptance from eff, the last counted
-//      pixel of every source up to q (a max-scan over q), the first pixel that
+//      Each Jacobi round computes acceptance from eff, the first pixel that
 //      marks each source pixel (atomicMin), and eff again.  eff[q] depends only
-//      on pixels before q, so the system has one solution and an iteration that
-//      changes nothing has reached it; iterations are capped and a sequential
+//      on pixels before q, so the system has one solution and a round that
+//      changes nothing has reached it; rounds are capped and a sequential
 //      pass takes over beyond the cap;
 //   3. marks become permanent, confidences take the value of the last pixel
 //      that marked them (atomicMax), points are compacted in raster order.
+//
+// Entry (q, j), an eff bit, is source j's used position from q until the next
+// pixel with bit j.  It is marked by the accepted pixels of that interval, the
+// first of them counts for the rounds and the last for the confidence.  A
+// counted pixel is nearly always accepted itself, so the first is q; the other
+// ends are looked up in bitmaps (one per source, one of accepted pixels), 32
+// pixels at a time, and 1024 at a time where a summary word shows nothing set.  (Prefix maxima of the last counted pixel for every
+// pixel and source, ten words a pixel written and read again in every round,
+// took two thirds of a scan: 11 views of 1600x1200 with 10 sources took 33.9 ms
+// and take 13.4.  A further summary level of 32 chunks changed nothing.)
+// Marks carry the round that set them, so no round clears them.
+//
+// Rounds are launched as many as the previous view needed; each kernel returns
+// at once when the round before it changed nothing, so the host reads the change
+// flags once a view instead of once a round.
+//
 // Arithmetic mirrors the host code of the reference (g++ without -ffast-math):
 // float geometry, double where pow(float, int) promotes; exp(float) is the
 // float function there (the double exp rounded to float here).  No implicit
@@ -33,14 +49,44 @@
 
 namespace hpm {
 
-constexpr int kScanBlock = 1024;
+constexpr int kScanBlock = 1024;  // pixels of a chunk: one word of summary bits
 constexpr int kMaxScanIterations = 256;
-// fixed-point rounds launched between host reads of their change flags: at 4 the extra rounds after
-// the fixed point cost more device time than the host round trips they save (confidence scans
-// 19.9 -> 21.5 ms per view on the 49-view 1600x1200 workload), so one
-constexpr int kRoundsPerCheck = 1;
-// "not marked" value of marktime: the byte pattern 0x7f written by cudaMemset
-constexpr int32_t kUnmarked = 0x7F7F7F7F;
+constexpr uint32_t kAccepted = 1u << 31;  // in a pixel's word beside the eff bits of at most 31 sources
+
+// One source of the view being scanned.  slot: the mark buffers it uses (a source listed twice shares them).
+struct ScanSource {
+    hpm_camera cam;  // scaled to W x H
+    int W, H, slot;
+    const float* depth;
+    const float* normal;
+    uint8_t* mask;   // used pixels, persistent across the views of one scan
+    float* cons;     // working confidence (confidence mode)
+};
+
+// One view of a scan against its sources; a kernel parameter.
+struct ScanRun {
+    hpm_camera cam;
+    int W, H, npix, n;
+    int stride;             // pixels rounded up to whole chunks: stride of the per-source arrays
+    const float* depth;
+    const float* normal;
+    const uint8_t* color;   // BGR (fusion)
+    const uint8_t* sky;     // BGR sky mask or null
+    uint8_t* mask;
+    float* cons;
+    int32_t* pos;           // [j * stride + q] source pixel of a passing pair
+    float* wexp;            // [j * stride + q] its weight
+    uint32_t* test;         // T bits
+    uint32_t* word;         // eff bits, kAccepted
+    uint32_t* chunk;        // OR of a chunk's words
+    uint32_t* map;          // [j * stride / 32 + q / 32] bit q % 32: eff bit j; j = n: accepted
+    float* dyn;             // sum of the counted weights
+    unsigned long long* first_mark;  // [slot * mark_stride + p]  (~round << 32) | first marking pixel
+    unsigned long long* last_mark;   // [slot * mark_stride + p]  (view << 32) | last marking pixel
+    size_t mark_stride;
+    ScanSource src[31];
+};
+static_assert(sizeof(ScanRun) <= 32764, "ScanRun exceeds the kernel parameter limit");
 
 __device__ __forceinline__ float3 sc_world_point(int x, int y, float depth, const hpm_camera& c) {
     const float X0 = depth * (x - c.K[2]) / c.K[0];
@@ -77,257 +123,277 @@ __device__ __forceinline__ float host_angle(const float* a, const float* b) {  /
 }
 
 template <int MODE>
-__global__ void k_candidates(const ScanView* __restrict__ views, int i, const int32_t* __restrict__ srcs, int n_ngb,
-                             int32_t* __restrict__ pos, double* __restrict__ wexp, uint32_t* __restrict__ test,
-                             int npix) {
+__global__ void __launch_bounds__(256) k_candidates(const __grid_constant__ ScanRun a) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= npix) return;
-    const ScanView& vi = views[i];
-    const int W = vi.W;
-    const int r = q / W, c = q - r * W;
+    if (q >= a.npix) return;
+    const int r = q / a.W, c = q - r * a.W;
     uint32_t T = 0;
-    const float ref_depth = vi.depth[q];
-    bool valid = vi.mask[q] != 1 && ref_depth > 0.0f;
-    if (MODE == 0 && valid && (ref_depth < vi.cam.depth_min || ref_depth > vi.cam.depth_max)) valid = false;
-    float3 X = make_float3(0.f, 0.f, 0.f);
-    if (valid) X = sc_world_point(c, r, ref_depth, vi.cam);
-    const float* rn = vi.normal + 3 * (size_t)q;
-    for (int j = 0; j < n_ngb; ++j) {
-        int p = -1;
-        if (valid) {
-            const ScanView& vs = views[srcs[j]];
+    const float ref_depth = a.depth[q];
+    bool valid = a.mask[q] != 1 && ref_depth > 0.0f;
+    if (MODE == 0 && valid && (ref_depth < a.cam.depth_min || ref_depth > a.cam.depth_max)) valid = false;
+    if (valid) {
+        const float3 X = sc_world_point(c, r, ref_depth, a.cam);
+        const float rn[3] = { a.normal[3 * (size_t)q], a.normal[3 * (size_t)q + 1], a.normal[3 * (size_t)q + 2] };
+#pragma unroll 1
+        for (int j = 0; j < a.n; ++j) {
+            const ScanSource& vs = a.src[j];
             float pd;
             const float2 pt = sc_project(X, vs.cam, pd);
             const int sr = host_trunc(pt.y + 0.5f);
             const int scc = host_trunc(pt.x + 0.5f);
-            if (scc >= 0 && scc < vs.W && sr >= 0 && sr < vs.H) {
-                p = sr * vs.W + scc;
-                const float sd = vs.depth[p];
-                bool ok = sd > 0.0f;
-                if (MODE == 0 && ok && (sd < vi.cam.depth_min || sd > vi.cam.depth_max)) ok = false;
-                if (ok) {
-                    const float3 tX = sc_world_point(scc, sr, sd, vs.cam);
-                    float proj;
-                    const float2 tp = sc_project(tX, vi.cam, proj);
-                    const double dx = (double)(c - tp.x), dy = (double)(r - tp.y);
-                    const float reproj = (float)sqrt(dx * dx + dy * dy);
-                    const float rel = (float)(fabs((double)(proj - ref_depth)) / (double)ref_depth);
-                    const float ang = host_angle(rn, vs.normal + 3 * (size_t)p);
-                    if (reproj < 2.0f && rel < 0.01f && ang < 0.174533f) {
-                        const float idx = reproj + 200 * rel + ang * 10;
-                        T |= 1u << j;
-                        // exp(float) of the reference's host code: the float function
-                        wexp[(size_t)q * n_ngb + j] = (double)(float)exp((double)(-idx));
-                    }
-                }
+            if (!(scc >= 0 && scc < vs.W && sr >= 0 && sr < vs.H)) continue;
+            const int p = sr * vs.W + scc;
+            const float sd = vs.depth[p];
+            if (!(sd > 0.0f)) continue;
+            if (MODE == 0 && (sd < a.cam.depth_min || sd > a.cam.depth_max)) continue;
+            const float3 tX = sc_world_point(scc, sr, sd, vs.cam);
+            float proj;
+            const float2 tp = sc_project(tX, a.cam, proj);
+            const double dx = (double)(c - tp.x), dy = (double)(r - tp.y);
+            const float reproj = (float)sqrt(dx * dx + dy * dy);
+            const float rel = (float)(fabs((double)(proj - ref_depth)) / (double)ref_depth);
+            if (!(reproj < 2.0f && rel < 0.01f)) continue;  // most misses end before the normals and the arc cosine
+            const float ang = host_angle(rn, vs.normal + 3 * (size_t)p);
+            if (!(ang < 0.174533f) || vs.mask[p] == 1) continue;
+            const float idx = reproj + 200 * rel + ang * 10;
+            T |= 1u << j;
+            // exp(float) of the reference's host code: the float function
+            a.wexp[(size_t)j * a.stride + q] = (float)exp((double)(-idx));
+            a.pos[(size_t)j * a.stride + q] = p;
+        }
+    }
+    a.test[q] = T;
+    a.word[q] = T;
+}
+
+// A round's kernels run when the round before changed something.
+__device__ __forceinline__ bool settled(const int* before) { return before && *before == 0; }
+
+// Acceptance from the eff bits, the chunks' summaries, and the marks of accepted pixels on the
+// positions they counted.  One block per chunk; pixels past the last have empty words.
+__global__ void __launch_bounds__(kScanBlock) k_accept(const __grid_constant__ ScanRun a, const int* before,
+                                                       uint32_t round) {
+    __shared__ uint32_t ws[32];
+    if (settled(before)) return;
+    const int q = blockIdx.x * kScanBlock + threadIdx.x;
+    uint32_t w = 0;
+    if (q < a.npix) {
+        const uint32_t e = a.word[q] & ~kAccepted;
+        w = e;
+        float d = 0.0f;
+        for (uint32_t m = e; m; m &= m - 1) {
+            const int j = __ffs(m) - 1;
+            d = (float)((double)d + (double)a.wexp[(size_t)j * a.stride + q]);
+        }
+        const int n = __popc(e);
+        a.dyn[q] = d;
+        if (n >= 1 && (double)d > 0.3 * n) {
+            w |= kAccepted;
+            const unsigned long long mark = (unsigned long long)~round << 32 | (uint32_t)q;
+            for (uint32_t m = e; m; m &= m - 1) {
+                const int j = __ffs(m) - 1;
+                atomicMin(a.first_mark + a.src[j].slot * a.mark_stride + a.pos[(size_t)j * a.stride + q], mark);
             }
         }
-        pos[(size_t)q * n_ngb + j] = p;
     }
-    test[q] = T;
-}
-
-// eff = T minus pairs whose source pixel is masked or marked before q.
-__global__ void k_update_eff(const ScanView* __restrict__ views, const int32_t* __restrict__ srcs, int n_ngb,
-                             const int32_t* __restrict__ pos, const uint32_t* __restrict__ test,
-                             uint32_t* __restrict__ eff, int* __restrict__ changed, int npix, int use_marks) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= npix) return;
-    const uint32_t T = test[q];
-    uint32_t e = T;
-    for (int j = 0; j < n_ngb; ++j) {
-        if (!((T >> j) & 1u)) continue;
-        const ScanView& vs = views[srcs[j]];
-        const int p = pos[(size_t)q * n_ngb + j];
-        bool blocked = vs.mask[p] == 1;
-        if (use_marks && vs.marktime[p] < q) blocked = true;
-        if (blocked) e &= ~(1u << j);
+    a.word[q] = w;
+    const int lane = threadIdx.x & 31, words = a.stride / 32;
+    const uint32_t any = __reduce_or_sync(0xffffffffu, w);
+    for (int j = 0; j <= a.n; ++j) {
+        const uint32_t b = __ballot_sync(0xffffffffu, w & (j < a.n ? 1u << j : kAccepted));
+        if (lane == 0) a.map[(size_t)j * words + (q >> 5)] = b;
     }
-    if (e != eff[q]) {
-        eff[q] = e;
-        if (changed) *changed = 1;
-    }
-}
-
-__global__ void k_accept(const uint32_t* __restrict__ eff, const double* __restrict__ wexp, int n_ngb,
-                         float* __restrict__ dyn, uint8_t* __restrict__ acc, int npix) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= npix) return;
-    const uint32_t e = eff[q];
-    float d = 0.0f;
-    int n = 0;
-    for (int j = 0; j < n_ngb; ++j)
-        if ((e >> j) & 1u) {
-            d = (float)((double)d + wexp[(size_t)q * n_ngb + j]);
-            ++n;
-        }
-    dyn[q] = d;
-    acc[q] = (n >= 1 && (double)d > 0.3 * n) ? 1 : 0;
-}
-
-// last[q][j] = max{q' <= q : eff[q'] has bit j}, per block of kScanBlock pixels.
-__global__ void k_last_local(const uint32_t* __restrict__ eff, int n_ngb, int32_t* __restrict__ last,
-                             int32_t* __restrict__ block_max, int npix) {
-    __shared__ int32_t s[kScanBlock];
-    const int j = blockIdx.y;
-    const int q = blockIdx.x * kScanBlock + threadIdx.x;
-    int v = -1;
-    if (q < npix && ((eff[q] >> j) & 1u)) v = q;
-    s[threadIdx.x] = v;
+    if (lane == 0) ws[threadIdx.x >> 5] = any;
     __syncthreads();
-    for (int off = 1; off < kScanBlock; off <<= 1) {
-        const int t = (int)threadIdx.x >= off ? s[threadIdx.x - off] : -1;
-        __syncthreads();
-        s[threadIdx.x] = max(s[threadIdx.x], t);
-        __syncthreads();
-    }
-    if (q < npix) last[(size_t)q * n_ngb + j] = s[threadIdx.x];
-    if (threadIdx.x == kScanBlock - 1) block_max[(size_t)j * gridDim.x + blockIdx.x] = s[threadIdx.x];
-}
-
-__global__ void k_last_blocks(int32_t* __restrict__ block_max, int nblocks, int n_ngb) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n_ngb) return;
-    int run = -1;
-    for (int b = 0; b < nblocks; ++b) {  // exclusive prefix max over blocks
-        const int v = block_max[(size_t)j * nblocks + b];
-        block_max[(size_t)j * nblocks + b] = run;
-        run = max(run, v);
+    if (threadIdx.x < 32) {
+        const uint32_t all = __reduce_or_sync(0xffffffffu, ws[threadIdx.x]);
+        if (threadIdx.x == 0) a.chunk[blockIdx.x] = all;
     }
 }
 
-__global__ void k_last_combine(int32_t* __restrict__ last, const int32_t* __restrict__ block_max, int n_ngb,
-                               int npix, int nblocks) {
+// The first chunk from `c` on whose summary has a bit of `m`, or one past the last.
+__device__ __forceinline__ int next_chunk(const ScanRun& a, int c, uint32_t m) {
+    const int chunks = a.stride / kScanBlock;
+    for (; c < chunks; c += 4) {  // four loads in flight
+        uint32_t v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = c + k < chunks ? a.chunk[c + k] & m : 0u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (v[k]) return c + k;
+    }
+    return chunks;
+}
+
+// The first pixel from `q` on with eff bit j (or accepted, when ALSO_ACCEPTED), or stride.
+template <bool ALSO_ACCEPTED>
+__device__ __forceinline__ int next_pixel(const ScanRun& a, int q, int j) {
+    if (q >= a.stride) return a.stride;
+    const int words = a.stride / 32;
+    const uint32_t* eff = a.map + (size_t)j * words;
+    const uint32_t* acc = a.map + (size_t)a.n * words;
+    auto bits = [&](int w) { return ALSO_ACCEPTED ? eff[w] | acc[w] : eff[w]; };
+    int w = q >> 5;
+    uint32_t b = bits(w) & (0xffffffffu << (q & 31));
+    while (!b && (++w & 31)) b = bits(w);  // to the end of the chunk: 32 words
+    if (!b) {
+        const int c = next_chunk(a, w >> 5, ALSO_ACCEPTED ? 1u << j | kAccepted : 1u << j);
+        if (c * kScanBlock >= a.stride) return a.stride;
+        w = c * 32;
+        const int end = w + 32;
+        for (b = bits(w); !b && w + 1 < end;) b = bits(++w);
+        if (!b) return a.stride;
+    }
+    return w * 32 + __ffs(b) - 1;
+}
+
+// The last accepted pixel in [lo, hi], or -1.
+__device__ __forceinline__ int last_accepted(const ScanRun& a, int lo, int hi) {
+    const uint32_t* acc = a.map + (size_t)a.n * (a.stride / 32);
+    int w = hi >> 5;
+    const int w_lo = lo >> 5;
+    uint32_t b = acc[w] & (0xffffffffu >> (31 - (hi & 31)));
+    while (!b && w > w_lo) {
+        if (!(w & 31)) {  // the chunk below: skip those without an accepted pixel
+            int c = (w >> 5) - 1;
+            while (c > (w_lo >> 5) && !(a.chunk[c] & kAccepted)) --c;
+            w = c * 32 + 32;
+        }
+        b = acc[--w];
+    }
+    if (!b) return -1;
+    const int q = w * 32 + 31 - __clz(b);
+    return q >= lo ? q : -1;
+}
+
+// Marks of counted but not accepted pixels: by the next accepted pixel, unless a pixel up to it counts
+// the source again.
+__global__ void __launch_bounds__(256) k_mark_stale(const __grid_constant__ ScanRun a, const int* before,
+                                                    uint32_t round) {
+    if (settled(before)) return;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= npix) return;
-    const int b = q / kScanBlock;
-    for (int j = 0; j < n_ngb; ++j) {
-        const int pre = block_max[(size_t)j * nblocks + b];
-        int32_t& v = last[(size_t)q * n_ngb + j];
-        v = max(v, pre);
+    if (q >= a.npix) return;
+    const uint32_t w = a.word[q];
+    if (w & kAccepted) return;
+    for (uint32_t m = w; m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        const int n = next_pixel<true>(a, q + 1, j);
+        if (n < a.npix && !((a.word[n] >> j) & 1u))
+            atomicMin(a.first_mark + a.src[j].slot * a.mark_stride + a.pos[(size_t)j * a.stride + q],
+                      (unsigned long long)~round << 32 | (uint32_t)n);
     }
 }
 
-// The marks of every source of the current view back to "not marked" (marktime) and -1
-// (marklast, confidence mode): one launch for all sources of a round, row j of the grid for
-// source j.
-__global__ void k_reset_marks(const ScanView* __restrict__ views, const int32_t* __restrict__ srcs, int with_last) {
-    const ScanView& vs = views[srcs[blockIdx.y]];
+// eff = T minus the pairs whose source pixel is marked before q.
+__global__ void __launch_bounds__(256) k_update_eff(const __grid_constant__ ScanRun a, const int* before,
+                                                    uint32_t round, int* __restrict__ changed) {
+    if (settled(before)) return;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= a.npix) return;
+    const uint32_t T = a.test[q];
+    uint32_t e = T;
+    for (uint32_t m = T; m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        const unsigned long long v = a.first_mark[a.src[j].slot * a.mark_stride + a.pos[(size_t)j * a.stride + q]];
+        if ((uint32_t)(v >> 32) == ~round && (uint32_t)v < (uint32_t)q) e &= ~(1u << j);
+    }
+    const uint32_t w = a.word[q];
+    if (e != (w & ~kAccepted)) {
+        a.word[q] = e;  // the next round sets kAccepted
+        *changed = 1;
+    }
+}
+
+// The settled marks: the source pixels of all marked entries become used; with MODE 0 each also
+// learns the last accepted pixel of its interval.
+template <int MODE>
+__global__ void __launch_bounds__(256) k_settle(const __grid_constant__ ScanRun a, uint32_t view) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= a.npix) return;
+    const uint32_t w = a.word[q];
+    for (uint32_t m = w & ~kAccepted; m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        int last = w & kAccepted ? q : -1;
+        if (MODE == 0) {
+            last = last_accepted(a, q, min(next_pixel<false>(a, q + 1, j), a.npix) - 1);
+        } else if (last < 0) {
+            const int n = next_pixel<true>(a, q + 1, j);
+            if (n < a.npix && !((a.word[n] >> j) & 1u)) last = n;
+        }
+        if (last < 0) continue;
+        const int p = a.pos[(size_t)j * a.stride + q];
+        a.src[j].mask[p] = 1;
+        if (MODE == 0)
+            atomicMax(a.last_mark + a.src[j].slot * a.mark_stride + p, (unsigned long long)view << 32 | (uint32_t)last);
+    }
+}
+
+// Confidences of the sources' pixels marked in this view: grid row j for source j.
+__global__ void __launch_bounds__(256) k_marked_conf(const __grid_constant__ ScanRun a, uint32_t view) {
+    const ScanSource& vs = a.src[blockIdx.y];
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= vs.W * vs.H) return;
-    vs.marktime[p] = kUnmarked;
-    if (with_last) vs.marklast[p] = -1;
+    const unsigned long long v = a.last_mark[vs.slot * a.mark_stride + p];
+    if ((uint32_t)(v >> 32) == view) vs.cons[p] = a.dyn[(uint32_t)v];
 }
 
-template <int MODE>
-__global__ void k_marks(const ScanView* __restrict__ views, const int32_t* __restrict__ srcs, int n_ngb,
-                        const int32_t* __restrict__ pos, const int32_t* __restrict__ last,
-                        const uint8_t* __restrict__ acc, int npix) {
+__global__ void __launch_bounds__(256) k_conf_own(const __grid_constant__ ScanRun a, float* __restrict__ out) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= npix || !acc[q]) return;
-    for (int j = 0; j < n_ngb; ++j) {
-        const int L = last[(size_t)q * n_ngb + j];
-        if (L < 0) continue;
-        const ScanView& vs = views[srcs[j]];
-        const int p = pos[(size_t)L * n_ngb + j];
-        atomicMin(&vs.marktime[p], q);
-        if (MODE == 0) atomicMax(&vs.marklast[p], q);
+    if (q >= a.npix) return;
+    float v = a.cons[q];
+    if (a.word[q] & kAccepted) {
+        v = a.dyn[q];
+        a.cons[q] = v;
     }
+    out[q] = v;  // confidence.dmb of view i is written after its own scan (main.cpp:1091-1095)
 }
 
 // Exact sequential pass (the reference loop) over the precomputed candidates;
 // used when the fixed point has not settled within kMaxScanIterations.
-template <int MODE>
-__global__ void k_sequential(const ScanView* __restrict__ views, const int32_t* __restrict__ srcs, int n_ngb,
-                             const int32_t* __restrict__ pos, const double* __restrict__ wexp,
-                             const uint32_t* __restrict__ test, float* __restrict__ dyn, uint8_t* __restrict__ acc,
-                             int npix) {
+__global__ void k_sequential(const __grid_constant__ ScanRun a, uint32_t round) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    int used[32];
-    for (int j = 0; j < n_ngb; ++j) used[j] = -1;
-    for (int q = 0; q < npix; ++q) {
-        const uint32_t T = test[q];
+    int used[31];
+    for (int j = 0; j < a.n; ++j) used[j] = -1;
+    for (int c = 0; c < a.stride / kScanBlock; ++c) a.chunk[c] = 0;
+    for (int w = 0; w < (a.n + 1) * (a.stride / 32); ++w) a.map[w] = 0;
+    for (int q = 0; q < a.npix; ++q) {
+        const uint32_t T = a.test[q];
+        uint32_t e = 0;
         float d = 0.0f;
-        int n = 0;
-        for (int j = 0; j < n_ngb; ++j) {
+        for (int j = 0; j < a.n; ++j) {
             if (!((T >> j) & 1u)) continue;
-            const ScanView& vs = views[srcs[j]];
-            const int p = pos[(size_t)q * n_ngb + j];
-            if (vs.mask[p] == 1 || vs.marktime[p] != kUnmarked) continue;
+            const int p = a.pos[(size_t)j * a.stride + q];
+            if ((uint32_t)(a.first_mark[a.src[j].slot * a.mark_stride + p] >> 32) == ~round) continue;
             used[j] = p;
-            d = (float)((double)d + wexp[(size_t)q * n_ngb + j]);
-            ++n;
+            d = (float)((double)d + (double)a.wexp[(size_t)j * a.stride + q]);
+            e |= 1u << j;
         }
-        const bool a = n >= 1 && (double)d > 0.3 * n;
-        dyn[q] = d;
-        acc[q] = a ? 1 : 0;
-        if (a)
-            for (int j = 0; j < n_ngb; ++j)
-                if (used[j] >= 0) {
-                    const ScanView& vs = views[srcs[j]];
-                    if (vs.marktime[used[j]] == kUnmarked) vs.marktime[used[j]] = q;
-                    if (MODE == 0) vs.marklast[used[j]] = q;
-                }
+        const int n = __popc(e);
+        const bool ok = n >= 1 && (double)d > 0.3 * n;
+        a.dyn[q] = d;
+        a.word[q] = ok ? e | kAccepted : e;
+        a.chunk[q / kScanBlock] |= a.word[q];
+        for (int j = 0; j <= a.n; ++j)
+            if (j < a.n ? (e >> j) & 1u : (uint32_t)ok) a.map[(size_t)j * (a.stride / 32) + (q >> 5)] |= 1u << (q & 31);
+        if (ok)
+            for (int j = 0; j < a.n; ++j)
+                if (used[j] >= 0)
+                    a.first_mark[a.src[j].slot * a.mark_stride + used[j]] = (unsigned long long)~round << 32 | (uint32_t)q;
     }
 }
 
-template <int MODE>
-__global__ void k_apply_marks(ScanView* __restrict__ views, int sid, const float* __restrict__ dyn) {
-    ScanView& vs = views[sid];
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= vs.W * vs.H) return;
-    if (vs.marktime[p] != kUnmarked) {
-        vs.mask[p] = 1;
-        if (MODE == 0) vs.cons[p] = dyn[vs.marklast[p]];
-    }
+// Fusion output: accepted pixels outside the sky (RunFusion_Sky_Strict, main.cpp:805).
+__device__ __forceinline__ bool fused(const ScanRun& a, int q) {
+    if (q >= a.npix || !(a.word[q] & kAccepted)) return false;
+    if (!a.sky) return true;
+    const uint8_t* s = a.sky + 3 * (size_t)q;
+    return (int)s[0] != 234 && (int)s[1] != 235 && (int)s[2] != 55;
 }
 
-__global__ void k_conf_own(ScanView* __restrict__ views, int i, const float* __restrict__ dyn,
-                           const uint8_t* __restrict__ acc, float* __restrict__ out, int npix) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= npix) return;
-    float* cons = views[i].cons;
-    if (acc[q]) cons[q] = dyn[q];
-    out[q] = cons[q];  // confidence.dmb of view i is written after its own scan (main.cpp:1091-1095)
-}
-
-// Fusion output: keep flag (sky test of RunFusion_Sky_Strict, main.cpp:805) and points.
-__global__ void k_fuse_flags(const ScanView* __restrict__ views, int i, const uint8_t* __restrict__ acc,
-                             int32_t* __restrict__ keep, int npix) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= npix) return;
-    const ScanView& v = views[i];
-    int k = acc[q];
-    if (k && v.sky) {
-        const uint8_t* s = v.sky + 3 * (size_t)q;
-        k = ((int)s[0] != 234 && (int)s[1] != 235 && (int)s[2] != 55) ? 1 : 0;
-    }
-    keep[q] = k;
-}
-
-__global__ void k_fuse_emit(const ScanView* __restrict__ views, int i, const int32_t* __restrict__ keep,
-                            const int32_t* __restrict__ offset, hpm_point* __restrict__ out, int64_t base,
-                            int64_t capacity, int npix) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= npix || !keep[q]) return;
-    const int64_t k = base + offset[q];
-    if (k >= capacity) return;
-    const ScanView& v = views[i];
-    const int r = q / v.W, c = q - r * v.W;
-    const float3 X = sc_world_point(c, r, v.depth[q], v.cam);
-    hpm_point p;
-    p.coord[0] = X.x; p.coord[1] = X.y; p.coord[2] = X.z;
-    p.normal[0] = v.normal[3 * (size_t)q]; p.normal[1] = v.normal[3 * (size_t)q + 1];
-    p.normal[2] = v.normal[3 * (size_t)q + 2];
-    p.color[0] = (float)v.color[3 * (size_t)q]; p.color[1] = (float)v.color[3 * (size_t)q + 1];
-    p.color[2] = (float)v.color[3 * (size_t)q + 2];
-    out[k] = p;
-}
-
-// Compaction offsets of the fused points: an exclusive prefix sum of the keep
-// flags in three launches over tiles of kScanBlock pixels -- tile totals, an
-// exclusive scan of the totals (one block), and each tile's scan plus its
-// offset.  Warp scans by shuffle, then a scan of the 32 warp totals.
+// Compaction of the fused points in three launches over tiles of kScanBlock
+// pixels: tile totals, an exclusive scan of the totals onto the points already
+// emitted (one block), and each tile's own scan, which writes the points.
+// Warp scans by shuffle, then a scan of the 32 warp totals.
 __device__ __forceinline__ int32_t warp_inclusive_sum(int32_t v) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -350,17 +416,22 @@ __device__ __forceinline__ int32_t block_inclusive_sum(int32_t v, int32_t* ws) {
     return v + (w > 0 ? ws[w - 1] : 0);
 }
 
-__global__ void __launch_bounds__(kScanBlock) k_tile_sums(const int32_t* __restrict__ in, int n,
-                                                          int32_t* __restrict__ tile_sum) {
+__global__ void __launch_bounds__(kScanBlock) k_fuse_count(const __grid_constant__ ScanRun a,
+                                                           int32_t* __restrict__ tile_sum) {
     __shared__ int32_t ws[32];
-    const int q = blockIdx.x * kScanBlock + threadIdx.x;
-    block_inclusive_sum(q < n ? in[q] : 0, ws);
-    if (threadIdx.x == 0) tile_sum[blockIdx.x] = ws[31];
+    const int n = __popc(__ballot_sync(0xffffffffu, fused(a, blockIdx.x * kScanBlock + threadIdx.x)));
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = n;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int32_t v = warp_inclusive_sum(ws[threadIdx.x]);
+        if (threadIdx.x == 31) tile_sum[blockIdx.x] = v;
+    }
 }
 
-// exclusive scan of the tile totals in place (one block, chunks with a carry); total = sum of all
+// exclusive scan of the tile totals in place (one block, chunks with a carry); emitted[0] = points before
+// this view, emitted[1] = after it
 __global__ void __launch_bounds__(kScanBlock) k_scan_tile_sums(int32_t* __restrict__ tile_sum, int ntiles,
-                                                               int32_t* __restrict__ total) {
+                                                               long long* __restrict__ emitted) {
     __shared__ int32_t ws[32];
     int32_t carry = 0;
     for (int base = 0; base < ntiles; base += kScanBlock) {
@@ -371,17 +442,32 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_tile_sums(int32_t* __restri
         carry += ws[31];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *total = carry;
+    if (threadIdx.x == 0) {
+        emitted[0] = emitted[1];
+        emitted[1] += carry;
+    }
 }
 
-__global__ void __launch_bounds__(kScanBlock) k_scan_tiles(const int32_t* __restrict__ in, int n,
-                                                           const int32_t* __restrict__ tile_off,
-                                                           int32_t* __restrict__ out) {
+__global__ void __launch_bounds__(kScanBlock) k_fuse_emit(const __grid_constant__ ScanRun a,
+                                                          const int32_t* __restrict__ tile_off,
+                                                          const long long* __restrict__ emitted,
+                                                          hpm_point* __restrict__ out, int64_t capacity) {
     __shared__ int32_t ws[32];
     const int q = blockIdx.x * kScanBlock + threadIdx.x;
-    const int32_t v = q < n ? in[q] : 0;
-    const int32_t inc = block_inclusive_sum(v, ws);
-    if (q < n) out[q] = tile_off[blockIdx.x] + inc - v;
+    const bool keep = fused(a, q);
+    const int32_t inc = block_inclusive_sum(keep ? 1 : 0, ws);
+    if (!keep) return;
+    const int64_t k = emitted[0] + tile_off[blockIdx.x] + inc - 1;
+    if (k >= capacity) return;
+    const int r = q / a.W, c = q - r * a.W;
+    const float3 X = sc_world_point(c, r, a.depth[q], a.cam);
+    hpm_point p;
+    p.coord[0] = X.x; p.coord[1] = X.y; p.coord[2] = X.z;
+    for (int d = 0; d < 3; ++d) {
+        p.normal[d] = a.normal[3 * (size_t)q + d];
+        p.color[d] = (float)a.color[3 * (size_t)q + d];
+    }
+    out[k] = p;
 }
 
 // ---------------------------------------------------------------- host driver
@@ -405,8 +491,7 @@ int Ctx::consistency_scan(int mode, int n_views, const int32_t* src_off, const i
         return fail(HPM_E_INVALID, "consistency scan: bad arguments");
     if (depth_kind != HPM_MAP_DEPTH && depth_kind != HPM_MAP_DEPTH_GEOM)
         return fail(HPM_E_INVALID, "consistency scan: depth kind must be DEPTH or DEPTH_GEOM");
-    std::vector<ScanView> hv(n_views);
-    size_t max_pix = 0, total_pix = 0;
+    size_t max_pix = 0;
     int max_ngb = 0;
     for (int v = 0; v < n_views; ++v) {
         ViewState& vs = views[v];
@@ -424,169 +509,163 @@ int Ctx::consistency_scan(int mode, int n_views, const int32_t* src_off, const i
         max_ngb = std::max(max_ngb, ng);
         if (mode == 1 && (!vs.color || vs.color_w != dm.w || vs.color_h != dm.h))
             return fail(HPM_E_STATE, "view %d lacks a colour image of its map size", v);
-        ScanView s{};
-        s.depth = dm.ptr;
-        s.normal = nm.ptr;
-        s.color = vs.color;
-        s.W = dm.w;
-        s.H = dm.h;
-        s.cam = vs.cam;
-        hv[v] = s;
         max_pix = std::max(max_pix, (size_t)dm.w * dm.h);
-        total_pix += (size_t)dm.w * dm.h;
     }
     // per-view scan state, carved out of one allocation in 256-byte aligned pieces
     auto al = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
-    size_t state_bytes = al(sizeof(ScanView) * n_views) + al(4 * (size_t)src_off[n_views] + 4);
-    for (int v = 0; v < n_views; ++v) {
-        const size_t n = (size_t)hv[v].W * hv[v].H;
-        state_bytes += al(n) + 3 * al(4 * n) + (mode == 1 ? al(3 * n) : 0);
-    }
+    struct State { uint8_t* mask; float* cons; const uint8_t* sky; };
+    std::vector<State> hv(n_views);
+    size_t state_bytes = 0;
+    auto pixels = [&](int v) { return (size_t)views[v].w * views[v].h; };
+    for (int v = 0; v < n_views; ++v)
+        state_bytes += al(pixels(v)) + (mode == 0 ? al(4 * pixels(v)) : (sky_host && sky_host[v] ? al(3 * pixels(v)) : 0));
     cudaError_t e = ensure_dev(scan_state, scan_state_cap, state_bytes);
     if (e != cudaSuccess) return cuda_fail(e, "alloc scan state");
     uint8_t* cur = scan_state;
     auto carve = [&](size_t bytes) { uint8_t* p = cur; cur += al(bytes); return p; };
     for (int v = 0; v < n_views; ++v) {
-        const size_t n = (size_t)hv[v].W * hv[v].H;
-        hv[v].mask = carve(n);
-        hv[v].cons = reinterpret_cast<float*>(carve(4 * n));
-        hv[v].marktime = reinterpret_cast<int32_t*>(carve(4 * n));
-        hv[v].marklast = reinterpret_cast<int32_t*>(carve(4 * n));
+        hv[v].mask = carve(pixels(v));
+        hv[v].cons = mode == 0 ? reinterpret_cast<float*>(carve(4 * pixels(v))) : nullptr;
+    }
+    e = cudaMemsetAsync(scan_state, 0, cur - scan_state, stream);
+    if (e != cudaSuccess) return cuda_fail(e, "clear scan state");
+    for (int v = 0; v < n_views; ++v) {
+        hv[v].sky = nullptr;
         if (mode == 1 && sky_host && sky_host[v]) {
-            uint8_t* sky = carve(3 * n);
-            e = cudaMemcpyAsync(sky, sky_host[v], 3 * n, cudaMemcpyHostToDevice, stream);
+            uint8_t* sky = carve(3 * pixels(v));
+            e = cudaMemcpyAsync(sky, sky_host[v], 3 * pixels(v), cudaMemcpyHostToDevice, stream);
             if (e != cudaSuccess) return cuda_fail(e, "upload sky mask");
             hv[v].sky = sky;
         }
-        cudaMemsetAsync(hv[v].mask, 0, n, stream);
-        cudaMemsetAsync(hv[v].cons, 0, 4 * n, stream);
-        cudaMemsetAsync(hv[v].marktime, 0x7f, 4 * n, stream);
     }
-    ScanView* d_views = reinterpret_cast<ScanView*>(carve(sizeof(ScanView) * n_views));
-    int32_t* d_srcs = reinterpret_cast<int32_t*>(carve(4 * (size_t)src_off[n_views] + 4));
-    e = cudaMemcpyAsync(d_views, hv.data(), sizeof(ScanView) * n_views, cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_srcs, src_ids, 4 * (size_t)src_off[n_views], cudaMemcpyHostToDevice, stream);
-    if (e != cudaSuccess) return cuda_fail(e, "upload scan views");
 
-    // per-pixel work buffers (sized for the largest view)
-    const size_t nblocks_max = (max_pix + kScanBlock - 1) / kScanBlock;
+    // work buffers, sized for the largest view and the most sources; the marks start as marked by no round
     const size_t ng = std::max(1, max_ngb);
-    const size_t wbytes = al(4 * max_pix * ng) + al(8 * max_pix * ng) + al(4 * max_pix * ng) + 5 * al(4 * max_pix) +
-                          al(max_pix) + al(4 * nblocks_max * ng) + al(64) + al(4 * kMaxScanIterations);
+    const size_t stride_max = (max_pix + kScanBlock - 1) / kScanBlock * kScanBlock;
+    const size_t mark_bytes = al(8 * max_pix * ng);
+    const size_t wbytes = 2 * al(4 * stride_max * ng) + 3 * al(4 * stride_max) + al(4 * stride_max / kScanBlock) +
+                          al(4 * stride_max / kScanBlock) + al(4 * (ng + 1) * (stride_max / 32)) + (mode == 0 ? 2 : 1) * mark_bytes + al(64) +
+                          al(4 * kMaxScanIterations);
     e = ensure_dev(scan_work, scan_work_cap, wbytes);
     if (e != cudaSuccess) return cuda_fail(e, "alloc scan work");
     cur = scan_work;
-    int32_t* pos = reinterpret_cast<int32_t*>(carve(4 * max_pix * ng));
-    double* wexp = reinterpret_cast<double*>(carve(8 * max_pix * ng));
-    int32_t* last = reinterpret_cast<int32_t*>(carve(4 * max_pix * ng));
-    uint32_t* test = reinterpret_cast<uint32_t*>(carve(4 * max_pix));
-    uint32_t* eff = reinterpret_cast<uint32_t*>(carve(4 * max_pix));
-    float* dyn = reinterpret_cast<float*>(carve(4 * max_pix));
-    uint8_t* acc = carve(max_pix);
-    int32_t* keep = reinterpret_cast<int32_t*>(carve(4 * max_pix));
-    int32_t* offs = reinterpret_cast<int32_t*>(carve(4 * max_pix));
-    int32_t* block_max = reinterpret_cast<int32_t*>(carve(4 * nblocks_max * ng));
-    int32_t* d_total = reinterpret_cast<int32_t*>(carve(64));
+    ScanRun a{};
+    a.pos = reinterpret_cast<int32_t*>(carve(4 * stride_max * ng));
+    a.wexp = reinterpret_cast<float*>(carve(4 * stride_max * ng));
+    a.test = reinterpret_cast<uint32_t*>(carve(4 * stride_max));
+    a.word = reinterpret_cast<uint32_t*>(carve(4 * stride_max));
+    a.dyn = reinterpret_cast<float*>(carve(4 * stride_max));
+    a.chunk = reinterpret_cast<uint32_t*>(carve(4 * stride_max / kScanBlock));
+    int32_t* tile_sum = reinterpret_cast<int32_t*>(carve(4 * stride_max / kScanBlock));
+    a.map = reinterpret_cast<uint32_t*>(carve(4 * (ng + 1) * (stride_max / 32)));
+    a.first_mark = reinterpret_cast<unsigned long long*>(carve(mark_bytes));
+    a.last_mark = mode == 0 ? reinterpret_cast<unsigned long long*>(carve(mark_bytes)) : nullptr;
+    a.mark_stride = max_pix;
+    long long* d_emitted = reinterpret_cast<long long*>(carve(64));
     int* d_changed = reinterpret_cast<int*>(carve(4 * kMaxScanIterations));  // one flag per round
+    e = cudaMemsetAsync(a.first_mark, 0xff, mark_bytes, stream);
+    if (e == cudaSuccess && mode == 0) e = cudaMemsetAsync(a.last_mark, 0, mark_bytes, stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_emitted, 0, 16, stream);
+    if (e != cudaSuccess) return cuda_fail(e, "clear scan work");
 
-    int64_t emitted = 0;
+    uint32_t round = 0;  // rounds of the whole scan, counted from 1: later ones win the atomicMin of the marks
+    int expected = 4;    // rounds to launch before the first look at their change flags
     int max_iter = 0;
     for (int i = 0; i < n_views; ++i) {
-        const int npix = hv[i].W * hv[i].H;
-        const int n_ngb = src_off[i + 1] - src_off[i];
-        const int32_t* srcs = d_srcs + src_off[i];
-        const int blocks = (npix + 255) / 256;
-        const int nblocks = (npix + kScanBlock - 1) / kScanBlock;
-        if (mode == 0) k_candidates<0><<<blocks, 256, 0, stream>>>(d_views, i, srcs, n_ngb, pos, wexp, test, npix);
-        else k_candidates<1><<<blocks, 256, 0, stream>>>(d_views, i, srcs, n_ngb, pos, wexp, test, npix);
-        cudaMemsetAsync(eff, 0xff, 4 * (size_t)npix, stream);
-        k_update_eff<<<blocks, 256, 0, stream>>>(d_views, srcs, n_ngb, pos, test, eff, nullptr, npix, 0);
-        launches += 2;
-        bool converged = n_ngb == 0;
-        int it = 0;
-        int max_sp = 0;
-        for (int j = 0; j < n_ngb; ++j) {
-            const ScanView& vs = hv[src_ids[src_off[i] + j]];
-            max_sp = std::max(max_sp, vs.W * vs.H);
+        a.W = views[i].w;
+        a.H = views[i].h;
+        a.npix = a.W * a.H;
+        a.stride = (a.npix + kScanBlock - 1) / kScanBlock * kScanBlock;
+        a.n = src_off[i + 1] - src_off[i];
+        a.cam = views[i].cam;
+        a.depth = views[i].maps[depth_kind].ptr;
+        a.normal = views[i].maps[HPM_MAP_NORMAL].ptr;
+        a.color = views[i].color;
+        a.sky = hv[i].sky;
+        a.mask = hv[i].mask;
+        a.cons = hv[i].cons;
+        int max_sp = 1;
+        for (int j = 0; j < a.n; ++j) {
+            const int sid = src_ids[src_off[i] + j];
+            ScanSource& s = a.src[j];
+            s.cam = views[sid].cam;
+            s.W = views[sid].w;
+            s.H = views[sid].h;
+            s.depth = views[sid].maps[depth_kind].ptr;
+            s.normal = views[sid].maps[HPM_MAP_NORMAL].ptr;
+            s.mask = hv[sid].mask;
+            s.cons = hv[sid].cons;
+            s.slot = (int)(std::find(src_ids + src_off[i], src_ids + src_off[i] + j, sid) - (src_ids + src_off[i]));
+            max_sp = std::max(max_sp, s.W * s.H);
         }
-        const dim3 reset_grid((max_sp + 255) / 256, std::max(1, n_ngb));
-        // rounds of the fixed point run kRoundsPerCheck at a time between reads of their change
-        // flags; a round after the one that changed nothing recomputes the same state from the same
-        // eff, so extra rounds would leave every result as it was at the fixed point
-        while (!converged && it < kMaxScanIterations) {
-            const int batch = std::min(kRoundsPerCheck, kMaxScanIterations - it);
-            cudaMemsetAsync(d_changed + it, 0, 4 * (size_t)batch, stream);
-            for (int r = 0; r < batch; ++r) {
-                k_accept<<<blocks, 256, 0, stream>>>(eff, wexp, n_ngb, dyn, acc, npix);
-                k_last_local<<<dim3(nblocks, n_ngb), kScanBlock, 0, stream>>>(eff, n_ngb, last, block_max, npix);
-                k_last_blocks<<<1, 32, 0, stream>>>(block_max, nblocks, n_ngb);
-                k_last_combine<<<blocks, 256, 0, stream>>>(last, block_max, n_ngb, npix, nblocks);
-                k_reset_marks<<<reset_grid, 256, 0, stream>>>(d_views, srcs, mode == 0 ? 1 : 0);
-                if (mode == 0) k_marks<0><<<blocks, 256, 0, stream>>>(d_views, srcs, n_ngb, pos, last, acc, npix);
-                else k_marks<1><<<blocks, 256, 0, stream>>>(d_views, srcs, n_ngb, pos, last, acc, npix);
-                k_update_eff<<<blocks, 256, 0, stream>>>(d_views, srcs, n_ngb, pos, test, eff, d_changed + it + r,
-                                                         npix, 1);
-                launches += 7;
+        const int blocks = (a.npix + 255) / 256;
+        const int chunks = a.stride / kScanBlock;
+        if (mode == 0) k_candidates<0><<<blocks, 256, 0, stream>>>(a);
+        else k_candidates<1><<<blocks, 256, 0, stream>>>(a);
+        ++launches;
+        e = cudaMemsetAsync(d_changed, 0, 4 * kMaxScanIterations, stream);
+        if (e != cudaSuccess) return cuda_fail(e, "clear change flags");
+        int launched = 0, it = 0;
+        bool converged = a.n == 0;
+        while (!converged && launched < kMaxScanIterations) {
+            const int until = std::min(kMaxScanIterations, launched + expected);
+            const int from = launched;
+            for (; launched < until; ++launched) {
+                const int* before = launched ? d_changed + launched - 1 : nullptr;
+                ++round;
+                k_accept<<<chunks, kScanBlock, 0, stream>>>(a, before, round);
+                k_mark_stale<<<blocks, 256, 0, stream>>>(a, before, round);
+                k_update_eff<<<blocks, 256, 0, stream>>>(a, before, round, d_changed + launched);
+                launches += 3;
             }
-            int changed[kRoundsPerCheck];
-            e = cudaMemcpyAsync(changed, d_changed + it, 4 * (size_t)batch, cudaMemcpyDeviceToHost, stream);
+            int changed[kMaxScanIterations];
+            e = cudaMemcpyAsync(changed + from, d_changed + from, 4 * (size_t)(launched - from), cudaMemcpyDeviceToHost,
+                                stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
             if (e != cudaSuccess) return cuda_fail(e, "consistency iteration");
-            int r = 0;
-            while (r < batch && changed[r] != 0) ++r;
-            if (r < batch) {
-                converged = true;
-                it += r + 1;
-            } else {
-                it += batch;
+            for (int r = from; r < launched && !converged; ++r) {
+                it = r + 1;
+                converged = changed[r] == 0;
             }
+            expected = converged ? expected : 2;
         }
-        if (!converged) {
-            for (int j = 0; j < n_ngb; ++j) {
-                const ScanView& vs = hv[src_ids[src_off[i] + j]];
-                cudaMemsetAsync(vs.marktime, 0x7f, 4 * (size_t)vs.W * vs.H, stream);
-                if (mode == 0) cudaMemsetAsync(vs.marklast, 0xff, 4 * (size_t)vs.W * vs.H, stream);
-            }
-            if (mode == 0) k_sequential<0><<<1, 32, 0, stream>>>(d_views, srcs, n_ngb, pos, wexp, test, dyn, acc, npix);
-            else k_sequential<1><<<1, 32, 0, stream>>>(d_views, srcs, n_ngb, pos, wexp, test, dyn, acc, npix);
-            ++launches;
-        } else if (n_ngb == 0) {
-            cudaMemsetAsync(acc, 0, npix, stream);
-        }
-        max_iter = std::max(max_iter, converged ? it : kMaxScanIterations + 1);
-        for (int j = 0; j < n_ngb; ++j) {
-            const int sid = src_ids[src_off[i] + j];
-            const int sp = hv[sid].W * hv[sid].H;
-            if (mode == 0) k_apply_marks<0><<<(sp + 255) / 256, 256, 0, stream>>>(d_views, sid, dyn);
-            else k_apply_marks<1><<<(sp + 255) / 256, 256, 0, stream>>>(d_views, sid, dyn);
-            ++launches;
-        }
-        if (mode == 0) {
-            e = ensure_map(i, HPM_MAP_CONF, hv[i].W, hv[i].H);
-            if (e != cudaSuccess) return cuda_fail(e, "alloc confidence map");
-            k_conf_own<<<blocks, 256, 0, stream>>>(d_views, i, dyn, acc, views[i].maps[HPM_MAP_CONF].ptr, npix);
+        if (a.n == 0) {
+            // no sources: nothing counted, nothing accepted (the words are the empty tests)
+        } else if (!converged) {
+            k_sequential<<<1, 1, 0, stream>>>(a, ++round);
             ++launches;
         } else {
-            k_fuse_flags<<<blocks, 256, 0, stream>>>(d_views, i, acc, keep, npix);
-            // block_max is free here (the mark iterations of view i are done): tile totals
-            k_tile_sums<<<nblocks, kScanBlock, 0, stream>>>(keep, npix, block_max);
-            k_scan_tile_sums<<<1, kScanBlock, 0, stream>>>(block_max, nblocks, d_total);
-            if (out) {
-                k_scan_tiles<<<nblocks, kScanBlock, 0, stream>>>(keep, npix, block_max, offs);
-                k_fuse_emit<<<blocks, 256, 0, stream>>>(d_views, i, keep, offs, out, emitted, capacity, npix);
-            }
-            launches += out ? 5 : 3;
-            int32_t total = 0;
-            e = cudaMemcpyAsync(&total, d_total, 4, cudaMemcpyDeviceToHost, stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-            if (e != cudaSuccess) return cuda_fail(e, "fusion count");
-            emitted += total;
+            expected = std::min(16, std::max(2, it));
         }
+        max_iter = std::max(max_iter, converged ? it : kMaxScanIterations + 1);
+        if (a.n > 0) {
+            if (mode == 0) {
+                k_settle<0><<<blocks, 256, 0, stream>>>(a, (uint32_t)i + 1);
+                k_marked_conf<<<dim3((max_sp + 255) / 256, a.n), 256, 0, stream>>>(a, (uint32_t)i + 1);
+                launches += 2;
+            } else {
+                k_settle<1><<<blocks, 256, 0, stream>>>(a, (uint32_t)i + 1);
+                ++launches;
+            }
+        }
+        if (mode == 0) {
+            e = ensure_map(i, HPM_MAP_CONF, a.W, a.H);
+            if (e != cudaSuccess) return cuda_fail(e, "alloc confidence map");
+            k_conf_own<<<blocks, 256, 0, stream>>>(a, views[i].maps[HPM_MAP_CONF].ptr);
+            ++launches;
+        } else {
+            k_fuse_count<<<chunks, kScanBlock, 0, stream>>>(a, tile_sum);
+            k_scan_tile_sums<<<1, kScanBlock, 0, stream>>>(tile_sum, chunks, d_emitted);
+            if (out) k_fuse_emit<<<chunks, kScanBlock, 0, stream>>>(a, tile_sum, d_emitted, out, capacity);
+            launches += out ? 3 : 2;
+        }
+        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "consistency scan launch");
     }
-    e = cudaStreamSynchronize(stream);
+    long long emitted[2] = { 0, 0 };
+    e = cudaMemcpyAsync(emitted, d_emitted, sizeof(emitted), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return cuda_fail(e, "consistency scan");
-    if (n_points) *n_points = emitted;
+    if (n_points) *n_points = emitted[1];
     if (max_iterations_used) *max_iterations_used = max_iter;
     return HPM_OK;
 }
