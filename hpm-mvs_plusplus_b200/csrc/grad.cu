@@ -22,7 +22,7 @@
 // through the views (its patch and samples in local memory, every sample taken
 // two or three times) was bound by latency: 10,000 pairs x 10 views, 313 warps
 // on the whole GPU, took 1.19 ms, and three steps on 640x480 pixels x 10 views
-// 244 ms; they take 0.20 and 19.8, with the same bits.
+// 244 ms; they take 0.18 and 10.9, with the same bits.
 #include "ctx.hpp"
 #include "hpm_device.cuh"
 #include "hpm_geometry.h"
@@ -91,7 +91,34 @@ struct Lane {
 constexpr int kPatchStride = 73;  // 36 weights, 36 texels; odd, so the pixels of a warp stay off each other's banks
 constexpr int kGradThreads = 128;
 
-static size_t patch_smem(int S) { return sizeof(float) * kPatchStride * (32 / S) * (kGradThreads / 32); }
+// What a lane needs of its view, in shared memory: the lanes of a warp each index another view, which
+// constant memory would serve one after the other.  18 words apart, two lanes to a bank at most.
+struct View {
+    float A[9], b[3];
+    const float* img;
+    int w, h;
+    int pad[2];
+};
+static_assert(sizeof(View) == 72, "View stride");
+
+static size_t grad_smem(int S) {
+    return sizeof(View) * S + sizeof(float) * kPatchStride * (32 / S) * (kGradThreads / 32);
+}
+
+// The block's views into shared memory; the patches follow them.
+__device__ __forceinline__ float* load_views(const RunArgs& a, const SrcImages& si, View* views) {
+    for (int j = threadIdx.x; j < a.S; j += blockDim.x) {
+        View v{};
+        for (int k = 0; k < 9; ++k) v.A[k] = a.basis[j + 1].A[k];
+        for (int k = 0; k < 3; ++k) v.b[k] = a.basis[j + 1].b[k];
+        v.img = si.img[j + 1];
+        v.w = si.w[j + 1];
+        v.h = si.h[j + 1];
+        views[j] = v;
+    }
+    __syncthreads();
+    return reinterpret_cast<float*>(views + a.S);
+}
 
 struct RefPatch {
     const float* w;  // shared memory
@@ -138,11 +165,14 @@ __device__ __forceinline__ RefPatch ref_patch(const RunArgs& a, int px, int py, 
     return P;
 }
 
-// Cost of one view and, with GRAD, d cost / d theta.
-template <bool GRAD>
-__device__ __forceinline__ float cost_grad_view(const RunArgs& a, const SrcImages& si, const RefPatch& P, int px,
-                                                int py, const float theta[3], int j, float* grad) {
-    if (GRAD) grad[0] = grad[1] = grad[2] = 0.f;
+// Cost of one view and, where `want`, d cost / d theta.  The kernels call it at one place, and the sample
+// loops are unrolled by kSampleUnroll only: three inlined copies with six samples each waited for
+// instructions two thirds of the time (refinement of 640x480 pixels: 19.2 ms, 10.2 here).
+constexpr int kSampleUnroll = 3;
+
+__device__ __forceinline__ float cost_grad_view(const RunArgs& a, const View& view, const RefPatch& P, int px, int py,
+                                                const float theta[3], bool want, float* grad) {
+    grad[0] = grad[1] = grad[2] = 0.f;
     if (P.var < 1e-5f) return 2.0f;
     const float nx = theta[1], ny = theta[2];
     const float nn = 1.0f - nx * nx - ny * ny;
@@ -155,19 +185,15 @@ __device__ __forceinline__ float cost_grad_view(const RunArgs& a, const SrcImage
     const float w = -theta[0] * nr;
     const float t[3] = { nx / fx, ny / fy, nz - nx * cx / fx - ny * cy / fy };
     const float m[3] = { t[0] / w, t[1] / w, t[2] / w };
-    if (j < 0 || j > 30) {
-        atomicAdd(&g_grad_oob, 1u);
-        return 2.0f;
-    }
-    const float* A = a.basis[j + 1].A;
-    const float* b = a.basis[j + 1].b;
+    const float* A = view.A;
+    const float b[3] = { view.b[0], view.b[1], view.b[2] };
     float H[9];
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
         for (int k = 0; k < 3; ++k) H[3 * r + k] = A[3 * r + k] - b[r] * m[k];
-    const float* img = si.img[j + 1];
-    const int sw = si.w[j + 1], sh = si.h[j + 1];
+    const float* img = view.img;
+    const int sw = view.w, sh = view.h;
     if (!img || sw <= 0 || sh <= 0) {
         atomicAdd(&g_grad_oob, 1u);
         return 2.0f;
@@ -179,20 +205,15 @@ __device__ __forceinline__ float cost_grad_view(const RunArgs& a, const SrcImage
     }
     float v[36];
     float Ss = 0.f;
-#pragma unroll 1
-    for (int i = 0; i < 6; ++i) {
-        const float ux = (float)(px - 5 + 2 * i);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            const float uy = (float)(py - 5 + 2 * k);
-            const float qz = H[6] * ux + H[7] * uy + H[8];
-            const float X = (H[0] * ux + H[1] * uy + H[2]) / qz;
-            const float Y = (H[3] * ux + H[4] * uy + H[5]) / qz;
-            float gx, gy;
-            const float vk = bilinear<false>(img, sw, sh, X, Y, gx, gy);
-            v[i * 6 + k] = vk;
-            Ss += P.w[i * 6 + k] * vk;
-        }
+#pragma unroll kSampleUnroll
+    for (int k = 0; k < 36; ++k) {
+        const float ux = (float)(px - 5 + 2 * (k / 6)), uy = (float)(py - 5 + 2 * (k % 6));
+        const float qz = H[6] * ux + H[7] * uy + H[8];
+        const float X = (H[0] * ux + H[1] * uy + H[2]) / qz;
+        const float Y = (H[3] * ux + H[4] * uy + H[5]) / qz;
+        float gx, gy;
+        v[k] = bilinear<false>(img, sw, sh, X, Y, gx, gy);
+        Ss += P.w[k] * v[k];
     }
     Ss /= P.W;
     float vs = 0.f, cv = 0.f;
@@ -208,27 +229,22 @@ __device__ __forceinline__ float cost_grad_view(const RunArgs& a, const SrcImage
     const float c = 1.0f - cov / sig;
     if (c < 0.0f) return 0.0f;
     if (c > 2.0f) return 2.0f;
-    if (!GRAD) return c;
+    if (!want) return c;
     float dm0 = 0.f, dm1 = 0.f, dm2 = 0.f;
-#pragma unroll 1
-    for (int i = 0; i < 6; ++i) {
-        const float ux = (float)(px - 5 + 2 * i);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            const float uy = (float)(py - 5 + 2 * k);
-            const float qz = H[6] * ux + H[7] * uy + H[8];
-            const float X = (H[0] * ux + H[1] * uy + H[2]) / qz;
-            const float Y = (H[3] * ux + H[4] * uy + H[5]) / qz;
-            float gx, gy;
-            const float vk = bilinear<true>(img, sw, sh, X, Y, gx, gy);
-            const float wk = P.w[i * 6 + k], rk = P.r[i * 6 + k];
-            const float dcdv = wk / P.W * (-(rk - P.mean) / sig + cov * (vk - Ss) / (sig * var_s));
-            const float gb = (gx * b[0] + gy * b[1] - (gx * X + gy * Y) * b[2]) / qz;
-            const float f = -dcdv * gb;
-            dm0 += f * ux;
-            dm1 += f * uy;
-            dm2 += f;
-        }
+#pragma unroll kSampleUnroll
+    for (int k = 0; k < 36; ++k) {
+        const float ux = (float)(px - 5 + 2 * (k / 6)), uy = (float)(py - 5 + 2 * (k % 6));
+        const float qz = H[6] * ux + H[7] * uy + H[8];
+        const float X = (H[0] * ux + H[1] * uy + H[2]) / qz;
+        const float Y = (H[3] * ux + H[4] * uy + H[5]) / qz;
+        float gx, gy;
+        bilinear<true>(img, sw, sh, X, Y, gx, gy);
+        const float dcdv = P.w[k] / P.W * (-(P.r[k] - P.mean) / sig + cov * (v[k] - Ss) / (sig * var_s));
+        const float gb = (gx * b[0] + gy * b[1] - (gx * X + gy * Y) * b[2]) / qz;
+        const float f = -dcdv * gb;
+        dm0 += f * ux;
+        dm1 += f * uy;
+        dm2 += f;
     }
     const float dw = -(dm0 * m[0] + dm1 * m[1] + dm2 * m[2]) / w;
     float dn0 = (dm0 / fx - dm2 * cx / fx) / w, dn1 = (dm1 / fy - dm2 * cy / fy) / w, dn2 = dm2 / w;
@@ -246,7 +262,8 @@ __global__ void __launch_bounds__(kGradThreads) k_cost_grad(const __grid_constan
                                                             const int32_t* __restrict__ px,
                                                             const float* __restrict__ theta, float* __restrict__ cost,
                                                             float* __restrict__ grad) {
-    extern __shared__ float smem[];
+    extern __shared__ View views[];
+    float* smem = load_views(a, si, views);
     const Lane L(a.S);
     const int k = (blockIdx.x * (kGradThreads / 32) + (threadIdx.x >> 5)) * L.per_warp + L.pixel;
     bool on = L.pixel < L.per_warp && k < n;
@@ -263,13 +280,10 @@ __global__ void __launch_bounds__(kGradThreads) k_cost_grad(const __grid_constan
     if (!on) return;
     const float th[3] = { theta[3 * k], theta[3 * k + 1], theta[3 * k + 2] };
     const size_t at = (size_t)k * a.S + L.view;
-    if (grad) {
-        float g[3];
-        cost[at] = cost_grad_view<true>(a, si, P, x, y, th, L.view, g);
+    float g[3];
+    cost[at] = cost_grad_view(a, views[L.view], P, x, y, th, grad != nullptr, g);
+    if (grad)
         for (int q = 0; q < 3; ++q) grad[at * 3 + q] = g[q];
-    } else {
-        cost[at] = cost_grad_view<false>(a, si, P, x, y, th, L.view, nullptr);
-    }
 }
 
 // d = M^-1 rhs for a 3x3 M through its adjugate; false when M is singular.
@@ -289,12 +303,15 @@ __device__ bool solve3(const float M[9], const float rhs[3], float d[3]) {
 // Gauss-Newton on the sum of squared per-view costs, a Levenberg damping that
 // grows tenfold on every rejected step; the valid views are those with a cost
 // in (0, 2) at the start.  Depth stays in [dmin, dmax].  The lanes of a pixel
-// carry the same state; a warp goes on while one of its pixels does.
+// carry the same state.  Every turn costs each pixel's views once, for whatever
+// it needs next (the start, the gradients of a step, a trial); a warp goes on
+// while one of its pixels does.
 __global__ void __launch_bounds__(kGradThreads) k_gn_refine(const __grid_constant__ RunArgs a,
                                                             const __grid_constant__ SrcImages si, int steps,
                                                             float* __restrict__ depth, float* __restrict__ normal,
                                                             float* __restrict__ cost_out, size_t n_px) {
-    extern __shared__ float smem[];
+    extern __shared__ View views[];
+    float* smem = load_views(a, si, views);
     const Lane L(a.S);
     const size_t i = ((size_t)blockIdx.x * (kGradThreads / 32) + (threadIdx.x >> 5)) * L.per_warp + L.pixel;
     bool on = L.pixel < L.per_warp && i < n_px;
@@ -318,64 +335,76 @@ __global__ void __launch_bounds__(kGradThreads) k_gn_refine(const __grid_constan
     }
     if (!__any_sync(0xffffffffu, on)) return;
     const RefPatch P = ref_patch(a, x, y, on, L, smem);
-    float c = on ? cost_grad_view<false>(a, si, P, x, y, th, L.view, nullptr) : 0.f;
-    const bool mine = on && c > 0.0f && c < 2.0f;
-    const uint32_t valid = (__ballot_sync(0xffffffffu, mine) >> L.base) & ((1u << a.S) - 1u);
-    auto sum_squares = [&](float v) {
-        float e = 0.f;
-        for (int j = 0; j < a.S; ++j) {
-            const float cj = L.of(v, j);
-            if ((valid >> j) & 1u) e += cj * cj;
-        }
-        return e;
-    };
-    float e0 = sum_squares(c);
-    const bool refined = on && __popc(valid) >= 2;
-    bool active = refined;
-    float lambda = 1e-3f;
-    for (int it = 0; it < steps; ++it) {
-        if (!__any_sync(0xffffffffu, active)) break;
+    enum { kStart, kGradient, kTrial };
+    int turn = kStart, it = 0, attempt = 0;
+    bool active = on, mine = on, refined = false;
+    uint32_t valid = 0;
+    float e0 = 0.f, lambda = 1e-3f;
+    float tn[3] = { th[0], th[1], th[2] };  // what the next turn costs
+    float JtJ[9] = { 0.f }, Jtr[3] = { 0.f, 0.f, 0.f };
+    for (int left = 1 + steps * 5; left > 0 && __any_sync(0xffffffffu, active); --left) {
         float g[3] = { 0.f, 0.f, 0.f };
-        if (active && mine) c = cost_grad_view<true>(a, si, P, x, y, th, L.view, g);
-        float JtJ[9] = { 0.f }, Jtr[3] = { 0.f, 0.f, 0.f };
+        float c = 0.f;
+        if (active && mine) c = cost_grad_view(a, views[L.view], P, x, y, tn, turn == kGradient, g);
+        if (turn == kStart) mine = on && c > 0.0f && c < 2.0f;
+        const uint32_t votes = __ballot_sync(0xffffffffu, mine);
+        valid = (votes >> L.base) & ((1u << a.S) - 1u);
+        // sums over the views in their order: squared costs, and for the gradients J^T J and J^T r
+        const bool sums = __any_sync(0xffffffffu, active && turn == kGradient);
+        float e = 0.f, A[9] = { 0.f }, r[3] = { 0.f, 0.f, 0.f };
         for (int j = 0; j < a.S; ++j) {
             const float cj = L.of(c, j);
+            const bool use = (valid >> j) & 1u;
+            if (use) e += cj * cj;
+            if (!sums) continue;
             const float gj[3] = { L.of(g[0], j), L.of(g[1], j), L.of(g[2], j) };
-            if (!((valid >> j) & 1u)) continue;
+            if (!use) continue;
 #pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                Jtr[r] += gj[r] * cj;
+            for (int p = 0; p < 3; ++p) {
+                r[p] += gj[p] * cj;
 #pragma unroll
-                for (int q = 0; q < 3; ++q) JtJ[3 * r + q] += gj[r] * gj[q];
+                for (int q = 0; q < 3; ++q) A[3 * p + q] += gj[p] * gj[q];
             }
         }
-        bool accepted = false;
-        for (int attempt = 0; attempt < 4; ++attempt) {
-            const bool need = active && !accepted;
-            if (!__any_sync(0xffffffffu, need)) break;
-            float M[9], rhs[3] = { -Jtr[0], -Jtr[1], -Jtr[2] }, dlt[3], tn[3];
-            for (int q = 0; q < 9; ++q) M[q] = JtJ[q];
-            for (int q = 0; q < 3; ++q) M[4 * q] += lambda * (JtJ[4 * q] + 1e-12f);
-            bool trial = solve3(M, rhs, dlt);
-            if (trial) {
+        if (!active) continue;
+        bool search = false;  // look for the next trial of this step
+        if (turn == kStart) {
+            e0 = e;
+            refined = active = __popc(valid) >= 2;
+            active = active && steps > 0;
+            turn = kGradient;
+        } else if (turn == kGradient) {
+#pragma unroll
+            for (int q = 0; q < 9; ++q) JtJ[q] = A[q];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) Jtr[q] = r[q];
+            attempt = 0;
+            search = true;
+        } else if (e < e0) {
+            th[0] = tn[0]; th[1] = tn[1]; th[2] = tn[2];
+            e0 = e;
+            lambda = fmaxf(lambda * 0.1f, 1e-6f);
+            turn = kGradient;  // of the next step, at the accepted point
+            active = ++it < steps;
+        } else {
+            lambda *= 10.f;
+            ++attempt;
+            search = true;
+        }
+        if (search) {
+            turn = kTrial;
+            for (; attempt < 4; ++attempt) {
+                float M[9], rhs[3] = { -Jtr[0], -Jtr[1], -Jtr[2] }, dlt[3];
+                for (int q = 0; q < 9; ++q) M[q] = JtJ[q];
+                for (int q = 0; q < 3; ++q) M[4 * q] += lambda * (JtJ[4 * q] + 1e-12f);
+                if (!solve3(M, rhs, dlt)) { lambda *= 10.f; continue; }
                 tn[0] = th[0] + dlt[0]; tn[1] = th[1] + dlt[1]; tn[2] = th[2] + dlt[2];
-                trial = tn[0] >= a.prm.depth_min && tn[0] <= a.prm.depth_max &&
-                        tn[1] * tn[1] + tn[2] * tn[2] < 0.999f;
+                if (!(tn[0] >= a.prm.depth_min && tn[0] <= a.prm.depth_max) ||
+                    !(tn[1] * tn[1] + tn[2] * tn[2] < 0.999f)) { lambda *= 10.f; continue; }
+                break;
             }
-            float ct = 0.f;
-            if (need && trial && mine) ct = cost_grad_view<false>(a, si, P, x, y, tn, L.view, nullptr);
-            const float e1 = sum_squares(ct);
-            if (!need) continue;
-            if (trial && e1 < e0) {
-                th[0] = tn[0]; th[1] = tn[1]; th[2] = tn[2];
-                e0 = e1;
-                lambda = fmaxf(lambda * 0.1f, 1e-6f);
-                accepted = true;
-            } else {
-                lambda *= 10.f;
-            }
+            active = attempt < 4;
         }
-        active = active && accepted;
     }
     if (!refined || L.view != 0) return;
     // camera-frame normal -> world frame (R^T n)
@@ -442,7 +471,7 @@ int Ctx::eval_cost_grad(int ref, const int32_t* srcs, int n_src, const hpm_param
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_th, theta, (size_t)n * 12, cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return cuda_fail(e, "upload hypotheses");
     if ((e = grad_oob_reset(stream)) != cudaSuccess) return cuda_fail(e, "self-check reset");
-    k_cost_grad<<<grad_blocks(n, a.S), kGradThreads, patch_smem(a.S), stream>>>(a, si, n, d_px, d_th, d_c,
+    k_cost_grad<<<grad_blocks(n, a.S), kGradThreads, grad_smem(a.S), stream>>>(a, si, n, d_px, d_th, d_c,
                                                                               grad ? d_g : nullptr);
     ++launches;
     unsigned int oob = 0;
@@ -469,7 +498,7 @@ int Ctx::eval_cost_grad_device(int ref, const int32_t* srcs, int n_src, const hp
     cudaError_t e;
     if ((e = grad_oob_reset(stream)) != cudaSuccess) return cuda_fail(e, "self-check reset");
     // pixels outside the reference image are skipped and counted by the kernel (no host copy to check them)
-    k_cost_grad<<<grad_blocks(n, a.S), kGradThreads, patch_smem(a.S), stream>>>(a, si, n, d_px, d_theta, d_cost,
+    k_cost_grad<<<grad_blocks(n, a.S), kGradThreads, grad_smem(a.S), stream>>>(a, si, n, d_px, d_theta, d_cost,
                                                                               d_grad);
     ++launches;
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "cost gradient launch");
@@ -497,7 +526,7 @@ int Ctx::gn_refine(int ref, const int32_t* srcs, int n_src, const hpm_params* pa
     cudaError_t e = ensure_map(ref, HPM_MAP_COST, v.w, v.h);
     if (e != cudaSuccess) return cuda_fail(e, "alloc cost map");
     if ((e = grad_oob_reset(stream)) != cudaSuccess) return cuda_fail(e, "self-check reset");
-    k_gn_refine<<<grad_blocks((size_t)v.w * v.h, a.S), kGradThreads, patch_smem(a.S), stream>>>(
+    k_gn_refine<<<grad_blocks((size_t)v.w * v.h, a.S), kGradThreads, grad_smem(a.S), stream>>>(
         a, si, steps, dm.ptr, nm.ptr, v.maps[HPM_MAP_COST].ptr, (size_t)v.w * v.h);
     ++launches;
     e = cudaGetLastError();
