@@ -29,7 +29,7 @@
 // pixels at a time, and 1024 at a time where a summary word shows nothing set.  (Prefix maxima of the last counted pixel for every
 // pixel and source, ten words a pixel written and read again in every round,
 // took two thirds of a scan: 11 views of 1600x1200 with 10 sources took 33.9 ms
-// and take 13.4.  A further summary level of 32 chunks changed nothing.)
+// and take 11.4.  A further summary level of 32 chunks changed nothing.)
 // Marks carry the round that set them, so no round clears them.
 //
 // Rounds are launched as many as the previous view needed; each kernel returns
@@ -56,6 +56,7 @@ constexpr uint32_t kAccepted = 1u << 31;  // in a pixel's word beside the eff bi
 // One source of the view being scanned.  slot: the mark buffers it uses (a source listed twice shares them).
 struct ScanSource {
     hpm_camera cam;  // scaled to W x H
+    float centre[3];
     int W, H, slot;
     const float* depth;
     const float* normal;
@@ -66,7 +67,9 @@ struct ScanSource {
 // One view of a scan against its sources; a kernel parameter.
 struct ScanRun {
     hpm_camera cam;
+    float centre[3];
     int W, H, npix, n;
+    bool distinct;          // no source is listed twice: slot j for source j
     int stride;             // pixels rounded up to whole chunks: stride of the per-source arrays
     const float* depth;
     const float* normal;
@@ -88,17 +91,19 @@ struct ScanRun {
 };
 static_assert(sizeof(ScanRun) <= 32764, "ScanRun exceeds the kernel parameter limit");
 
-__device__ __forceinline__ float3 sc_world_point(int x, int y, float depth, const hpm_camera& c) {
+// Camera centre, in the reference's float arithmetic (Get3DPointonWorld's C; the same on the host).
+static void camera_centre(const hpm_camera& c, float C[3]) {
+    for (int k = 0; k < 3; ++k) C[k] = -(c.R[k] * c.t[0] + c.R[3 + k] * c.t[1] + c.R[6 + k] * c.t[2]);
+}
+
+__device__ __forceinline__ float3 sc_world_point(int x, int y, float depth, const hpm_camera& c, const float* C) {
     const float X0 = depth * (x - c.K[2]) / c.K[0];
     const float X1 = depth * (y - c.K[5]) / c.K[4];
     const float X2 = depth;
     const float T0 = c.R[0] * X0 + c.R[3] * X1 + c.R[6] * X2;
     const float T1 = c.R[1] * X0 + c.R[4] * X1 + c.R[7] * X2;
     const float T2 = c.R[2] * X0 + c.R[5] * X1 + c.R[8] * X2;
-    const float C0 = -(c.R[0] * c.t[0] + c.R[3] * c.t[1] + c.R[6] * c.t[2]);
-    const float C1 = -(c.R[1] * c.t[0] + c.R[4] * c.t[1] + c.R[7] * c.t[2]);
-    const float C2 = -(c.R[2] * c.t[0] + c.R[5] * c.t[1] + c.R[8] * c.t[2]);
-    return make_float3(T0 + C0, T1 + C1, T2 + C2);
+    return make_float3(T0 + C[0], T1 + C[1], T2 + C[2]);
 }
 
 __device__ __forceinline__ float2 sc_project(float3 X, const hpm_camera& c, float& depth) {
@@ -132,7 +137,7 @@ __global__ void __launch_bounds__(256) k_candidates(const __grid_constant__ Scan
     bool valid = a.mask[q] != 1 && ref_depth > 0.0f;
     if (MODE == 0 && valid && (ref_depth < a.cam.depth_min || ref_depth > a.cam.depth_max)) valid = false;
     if (valid) {
-        const float3 X = sc_world_point(c, r, ref_depth, a.cam);
+        const float3 X = sc_world_point(c, r, ref_depth, a.cam, a.centre);
         const float rn[3] = { a.normal[3 * (size_t)q], a.normal[3 * (size_t)q + 1], a.normal[3 * (size_t)q + 2] };
 #pragma unroll 1
         for (int j = 0; j < a.n; ++j) {
@@ -146,7 +151,7 @@ __global__ void __launch_bounds__(256) k_candidates(const __grid_constant__ Scan
             const float sd = vs.depth[p];
             if (!(sd > 0.0f)) continue;
             if (MODE == 0 && (sd < a.cam.depth_min || sd > a.cam.depth_max)) continue;
-            const float3 tX = sc_world_point(scc, sr, sd, vs.cam);
+            const float3 tX = sc_world_point(scc, sr, sd, vs.cam, vs.centre);
             float proj;
             const float2 tp = sc_project(tX, a.cam, proj);
             const double dx = (double)(c - tp.x), dy = (double)(r - tp.y);
@@ -166,6 +171,26 @@ __global__ void __launch_bounds__(256) k_candidates(const __grid_constant__ Scan
     a.word[q] = T;
 }
 
+// The set bits of a word, kBatch at a time: a batch's gathers are in flight together (one bit after the
+// other, k_update_eff spent its time waiting for two dependent gathers a bit).
+constexpr int kBatch = 4;
+struct Batch {
+    int j[kBatch];  // -1 past the last
+    __device__ __forceinline__ explicit Batch(uint32_t& bits) {
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            j[k] = __ffs(bits) - 1;
+            bits &= bits - 1;
+        }
+    }
+};
+
+// Where source j's marks start.  (The lanes of a warp ask for different sources, which the constant
+// memory of the parameters would serve one after the other.)
+__device__ __forceinline__ size_t marks_of(const ScanRun& a, int j) {
+    return (a.distinct ? j : a.src[j].slot) * a.mark_stride;
+}
+
 // A round's kernels run when the round before changed something.
 __device__ __forceinline__ bool settled(const int* before) { return before && *before == 0; }
 
@@ -181,18 +206,28 @@ __global__ void __launch_bounds__(kScanBlock) k_accept(const __grid_constant__ S
         const uint32_t e = a.word[q] & ~kAccepted;
         w = e;
         float d = 0.0f;
-        for (uint32_t m = e; m; m &= m - 1) {
-            const int j = __ffs(m) - 1;
-            d = (float)((double)d + (double)a.wexp[(size_t)j * a.stride + q]);
+        for (uint32_t m = e; m;) {
+            const Batch b(m);
+            float x[kBatch];
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) x[k] = b.j[k] >= 0 ? a.wexp[(size_t)b.j[k] * a.stride + q] : 0.0f;
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k)
+                if (b.j[k] >= 0) d = (float)((double)d + (double)x[k]);
         }
         const int n = __popc(e);
         a.dyn[q] = d;
         if (n >= 1 && (double)d > 0.3 * n) {
             w |= kAccepted;
             const unsigned long long mark = (unsigned long long)~round << 32 | (uint32_t)q;
-            for (uint32_t m = e; m; m &= m - 1) {
-                const int j = __ffs(m) - 1;
-                atomicMin(a.first_mark + a.src[j].slot * a.mark_stride + a.pos[(size_t)j * a.stride + q], mark);
+            for (uint32_t m = e; m;) {
+                const Batch b(m);
+                int p[kBatch];
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k) p[k] = b.j[k] >= 0 ? a.pos[(size_t)b.j[k] * a.stride + q] : 0;
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k)
+                    if (b.j[k] >= 0) atomicMin(a.first_mark + marks_of(a, b.j[k]) + p[k], mark);
             }
         }
     }
@@ -266,6 +301,10 @@ __device__ __forceinline__ int last_accepted(const ScanRun& a, int lo, int hi) {
     return q >= lo ? q : -1;
 }
 
+// Pixels walked one by one, all sources of a pixel together, before the bitmaps are searched source by
+// source: most intervals end within a few pixels.
+constexpr int kWalk = 16;
+
 // Marks of counted but not accepted pixels: by the next accepted pixel, unless a pixel up to it counts
 // the source again.
 __global__ void __launch_bounds__(256) k_mark_stale(const __grid_constant__ ScanRun a, const int* before,
@@ -273,14 +312,24 @@ __global__ void __launch_bounds__(256) k_mark_stale(const __grid_constant__ Scan
     if (settled(before)) return;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= a.npix) return;
-    const uint32_t w = a.word[q];
-    if (w & kAccepted) return;
-    for (uint32_t m = w; m; m &= m - 1) {
+    uint32_t m = a.word[q];
+    if (m & kAccepted) return;
+    const int walk = min(q + kWalk, a.npix - 1);
+    int n = q;
+    uint32_t w = 0;
+    while (m && n < walk && !(w & kAccepted)) {
+        w = a.word[++n];
+        m &= ~w;  // counted again
+    }
+    for (; m; m &= m - 1) {
         const int j = __ffs(m) - 1;
-        const int n = next_pixel<true>(a, q + 1, j);
-        if (n < a.npix && !((a.word[n] >> j) & 1u))
-            atomicMin(a.first_mark + a.src[j].slot * a.mark_stride + a.pos[(size_t)j * a.stride + q],
-                      (unsigned long long)~round << 32 | (uint32_t)n);
+        int by = n;
+        if (!(w & kAccepted)) {
+            by = next_pixel<true>(a, n + 1, j);
+            if (by >= a.npix || ((a.word[by] >> j) & 1u)) continue;
+        }
+        atomicMin(a.first_mark + marks_of(a, j) + a.pos[(size_t)j * a.stride + q],
+                  (unsigned long long)~round << 32 | (uint32_t)by);
     }
 }
 
@@ -292,10 +341,18 @@ __global__ void __launch_bounds__(256) k_update_eff(const __grid_constant__ Scan
     if (q >= a.npix) return;
     const uint32_t T = a.test[q];
     uint32_t e = T;
-    for (uint32_t m = T; m; m &= m - 1) {
-        const int j = __ffs(m) - 1;
-        const unsigned long long v = a.first_mark[a.src[j].slot * a.mark_stride + a.pos[(size_t)j * a.stride + q]];
-        if ((uint32_t)(v >> 32) == ~round && (uint32_t)v < (uint32_t)q) e &= ~(1u << j);
+    for (uint32_t m = T; m;) {
+        const Batch b(m);
+        int p[kBatch];
+        unsigned long long v[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) p[k] = b.j[k] >= 0 ? a.pos[(size_t)b.j[k] * a.stride + q] : 0;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k)
+            v[k] = b.j[k] >= 0 ? a.first_mark[marks_of(a, b.j[k]) + p[k]] : 0ull;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k)
+            if (b.j[k] >= 0 && (uint32_t)(v[k] >> 32) == ~round && (uint32_t)v[k] < (uint32_t)q) e &= ~(1u << b.j[k]);
     }
     const uint32_t w = a.word[q];
     if (e != (w & ~kAccepted)) {
@@ -310,31 +367,52 @@ template <int MODE>
 __global__ void __launch_bounds__(256) k_settle(const __grid_constant__ ScanRun a, uint32_t view) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= a.npix) return;
-    const uint32_t w = a.word[q];
-    for (uint32_t m = w & ~kAccepted; m; m &= m - 1) {
-        const int j = __ffs(m) - 1;
-        int last = w & kAccepted ? q : -1;
-        if (MODE == 0) {
-            last = last_accepted(a, q, min(next_pixel<false>(a, q + 1, j), a.npix) - 1);
-        } else if (last < 0) {
-            const int n = next_pixel<true>(a, q + 1, j);
-            if (n < a.npix && !((a.word[n] >> j) & 1u)) last = n;
+    const uint32_t own = a.word[q];
+    uint32_t m = own & ~kAccepted;
+    int last = own & kAccepted ? q : -1, n = q;  // last accepted pixel up to n
+    auto settle = [&](uint32_t bits, int by) {  // the sources whose interval's marking pixel is known
+        if (by < 0) return;
+        for (; bits; bits &= bits - 1) {
+            const int j = __ffs(bits) - 1;
+            const int p = a.pos[(size_t)j * a.stride + q];
+            a.src[j].mask[p] = 1;
+            if (MODE == 0)
+                atomicMax(a.last_mark + marks_of(a, j) + p, (unsigned long long)view << 32 | (uint32_t)by);
         }
-        if (last < 0) continue;
-        const int p = a.pos[(size_t)j * a.stride + q];
-        a.src[j].mask[p] = 1;
-        if (MODE == 0)
-            atomicMax(a.last_mark + a.src[j].slot * a.mark_stride + p, (unsigned long long)view << 32 | (uint32_t)last);
+    };
+    const int walk = min(q + kWalk, a.npix - 1);
+    while (m && n < walk && !(MODE == 1 && last >= 0)) {
+        const uint32_t w = a.word[++n];
+        settle(m & w, last);  // counted again: the interval ends before n
+        m &= ~w;
+        if (w & kAccepted) last = n;
+    }
+    for (; m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        int by = last;
+        if (MODE == 0) {
+            const int next = min(next_pixel<false>(a, n + 1, j), a.npix);
+            if (next > n + 1) by = max(by, last_accepted(a, n + 1, next - 1));
+        } else if (by < 0) {
+            const int next = next_pixel<true>(a, n + 1, j);
+            if (next < a.npix && !((a.word[next] >> j) & 1u)) by = next;
+        }
+        settle(1u << j, by);
     }
 }
 
 // Confidences of the sources' pixels marked in this view: grid row j for source j.
 __global__ void __launch_bounds__(256) k_marked_conf(const __grid_constant__ ScanRun a, uint32_t view) {
     const ScanSource& vs = a.src[blockIdx.y];
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= vs.W * vs.H) return;
-    const unsigned long long v = a.last_mark[vs.slot * a.mark_stride + p];
-    if ((uint32_t)(v >> 32) == view) vs.cons[p] = a.dyn[(uint32_t)v];
+    const int p = 4 * (blockIdx.x * blockDim.x + threadIdx.x), n = vs.W * vs.H;
+    if (p >= n) return;
+    // the marks of four pixels in two loads; mark_stride is a multiple of four
+    const ulonglong2* marks = reinterpret_cast<const ulonglong2*>(a.last_mark + vs.slot * a.mark_stride + p);
+    const ulonglong2 lo = marks[0], hi = marks[1];
+    const unsigned long long v[4] = { lo.x, lo.y, hi.x, hi.y };
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (p + k < n && (uint32_t)(v[k] >> 32) == view) vs.cons[p + k] = a.dyn[(uint32_t)v[k]];
 }
 
 __global__ void __launch_bounds__(256) k_conf_own(const __grid_constant__ ScanRun a, float* __restrict__ out) {
@@ -460,7 +538,7 @@ __global__ void __launch_bounds__(kScanBlock) k_fuse_emit(const __grid_constant_
     const int64_t k = emitted[0] + tile_off[blockIdx.x] + inc - 1;
     if (k >= capacity) return;
     const int r = q / a.W, c = q - r * a.W;
-    const float3 X = sc_world_point(c, r, a.depth[q], a.cam);
+    const float3 X = sc_world_point(c, r, a.depth[q], a.cam, a.centre);
     hpm_point p;
     p.coord[0] = X.x; p.coord[1] = X.y; p.coord[2] = X.z;
     for (int d = 0; d < 3; ++d) {
@@ -542,7 +620,8 @@ int Ctx::consistency_scan(int mode, int n_views, const int32_t* src_off, const i
     // work buffers, sized for the largest view and the most sources; the marks start as marked by no round
     const size_t ng = std::max(1, max_ngb);
     const size_t stride_max = (max_pix + kScanBlock - 1) / kScanBlock * kScanBlock;
-    const size_t mark_bytes = al(8 * max_pix * ng);
+    const size_t mark_stride = (max_pix + 3) & ~size_t(3);
+    const size_t mark_bytes = al(8 * mark_stride * ng);
     const size_t wbytes = 2 * al(4 * stride_max * ng) + 3 * al(4 * stride_max) + al(4 * stride_max / kScanBlock) +
                           al(4 * stride_max / kScanBlock) + al(4 * (ng + 1) * (stride_max / 32)) + (mode == 0 ? 2 : 1) * mark_bytes + al(64) +
                           al(4 * kMaxScanIterations);
@@ -560,7 +639,7 @@ int Ctx::consistency_scan(int mode, int n_views, const int32_t* src_off, const i
     a.map = reinterpret_cast<uint32_t*>(carve(4 * (ng + 1) * (stride_max / 32)));
     a.first_mark = reinterpret_cast<unsigned long long*>(carve(mark_bytes));
     a.last_mark = mode == 0 ? reinterpret_cast<unsigned long long*>(carve(mark_bytes)) : nullptr;
-    a.mark_stride = max_pix;
+    a.mark_stride = mark_stride;
     long long* d_emitted = reinterpret_cast<long long*>(carve(64));
     int* d_changed = reinterpret_cast<int*>(carve(4 * kMaxScanIterations));  // one flag per round
     e = cudaMemsetAsync(a.first_mark, 0xff, mark_bytes, stream);
@@ -578,6 +657,7 @@ int Ctx::consistency_scan(int mode, int n_views, const int32_t* src_off, const i
         a.stride = (a.npix + kScanBlock - 1) / kScanBlock * kScanBlock;
         a.n = src_off[i + 1] - src_off[i];
         a.cam = views[i].cam;
+        camera_centre(a.cam, a.centre);
         a.depth = views[i].maps[depth_kind].ptr;
         a.normal = views[i].maps[HPM_MAP_NORMAL].ptr;
         a.color = views[i].color;
@@ -585,10 +665,12 @@ int Ctx::consistency_scan(int mode, int n_views, const int32_t* src_off, const i
         a.mask = hv[i].mask;
         a.cons = hv[i].cons;
         int max_sp = 1;
+        a.distinct = true;
         for (int j = 0; j < a.n; ++j) {
             const int sid = src_ids[src_off[i] + j];
             ScanSource& s = a.src[j];
             s.cam = views[sid].cam;
+            camera_centre(s.cam, s.centre);
             s.W = views[sid].w;
             s.H = views[sid].h;
             s.depth = views[sid].maps[depth_kind].ptr;
@@ -596,6 +678,7 @@ int Ctx::consistency_scan(int mode, int n_views, const int32_t* src_off, const i
             s.mask = hv[sid].mask;
             s.cons = hv[sid].cons;
             s.slot = (int)(std::find(src_ids + src_off[i], src_ids + src_off[i] + j, sid) - (src_ids + src_off[i]));
+            a.distinct = a.distinct && s.slot == j;
             max_sp = std::max(max_sp, s.W * s.H);
         }
         const int blocks = (a.npix + 255) / 256;
@@ -641,7 +724,7 @@ int Ctx::consistency_scan(int mode, int n_views, const int32_t* src_off, const i
         if (a.n > 0) {
             if (mode == 0) {
                 k_settle<0><<<blocks, 256, 0, stream>>>(a, (uint32_t)i + 1);
-                k_marked_conf<<<dim3((max_sp + 255) / 256, a.n), 256, 0, stream>>>(a, (uint32_t)i + 1);
+                k_marked_conf<<<dim3((max_sp + 1023) / 1024, a.n), 256, 0, stream>>>(a, (uint32_t)i + 1);
                 launches += 2;
             } else {
                 k_settle<1><<<blocks, 256, 0, stream>>>(a, (uint32_t)i + 1);
