@@ -54,6 +54,15 @@ struct InitScratch {
     __device__ __forceinline__ float& ca(int d, int j) const { return base[(d * NS + j) * BLK]; }
 };
 
+// A source view's part of the geometric cost, in shared memory: in view selection every lane goes
+// through its own selected views.
+struct alignas(16) GeomView {
+    float fwd_A[9], fwd_b[3], bwd_A[9], bwd_b[3];
+    const float* depth;
+    int w, h;
+};
+static_assert(sizeof(GeomView) == 112, "seven 16-byte loads");
+
 // Per-thread scratch of a half-sweep.  The cost rows of the eight directions are written once, an NCC
 // apart, and read once, by view selection: they stream through the thread's local memory, so that
 // shared memory (view weights, final costs, candidate positions) leaves the L1 to the textures and
@@ -65,6 +74,7 @@ struct Scratch {
     float* base;   // smem + threadIdx linear
     float* rows;   // local memory, kRowWords
     float4* cand;  // local memory: plane_m of the eight directions' planes and their depth at the pixel
+    const GeomView* views;  // shared memory, geometric modes only
     static constexpr int kWords = NS + 16;
     static constexpr int kRowWords = 8 * NS < 72 ? 72 : 8 * NS;  // at least a patch's texels and weights
     __device__ __forceinline__ float& ca(int d, int j) const { return rows[d * NS + j]; }
@@ -688,27 +698,32 @@ __device__ __forceinline__ Selection view_selection(const RunArgs& a, int px, in
     float fc[8];
 #pragma unroll
     for (int d = 0; d < 8; ++d) fc[d] = s.fc(d) = 0.0f;
+    if (!geom) {
 #pragma unroll 1
-    for (int j = 0; j < S; ++j) {
-        const float w = s.vw(j);
-        if (!(w > 0)) continue;
-        if (!geom) {
+        for (int j = 0; j < S; ++j) {
+            const float w = s.vw(j);
+            if (!(w > 0)) continue;
 #pragma unroll
             for (int d = 0; d < 8; ++d) fc[d] += w * s.ca(d, j);
-        } else {
+        }
+    } else {
+#pragma unroll 1
+        for (uint32_t m = o.temp_selected; m; m &= m - 1) {
+            const int j = __ffs(m) - 1;
+            const float w = s.vw(j);
+            const GeomView v = s.views[j];
 #pragma unroll 1
             for (int h = 0; h < 8; h += 4) {
                 float sx[4], sy[4], sd[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const float depth = (flags >> (h + k)) & 1u ? s.cand[h + k].w : 0.0f;
-                    sd[k] = geom_source_depth(a.depth_src[j + 1], a.dsw[j + 1], a.dsh[j + 1], a.fwd[j + 1].A,
-                                              a.fwd[j + 1].b, depth, px, py, sx[k], sy[k]);
+                    sd[k] = geom_source_depth(v.depth, v.w, v.h, v.fwd_A, v.fwd_b, depth, px, py, sx[k], sy[k]);
                 }
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const float g = (flags >> (h + k)) & 1u
-                                        ? 0.2f * geom_back_cost(a.bwd[j + 1].A, a.bwd[j + 1].b, sx[k], sy[k], sd[k], px, py)
+                                        ? 0.2f * geom_back_cost(v.bwd_A, v.bwd_b, sx[k], sy[k], sd[k], px, py)
                                         : 0.1f * 3.0f;
                     s.fc(h + k) += w * (s.ca(h + k, j) + g);
                 }
@@ -764,8 +779,8 @@ constexpr float kLogMargin = 1e-5f;
 // The decisions between slots are the reference's, in its order, and the
 // random draws happen in the same sequence.
 template <int NS, int BLK, bool MAND, bool CNT>
-__device__ __forceinline__ void sweep_pixel(const RunArgs& a, float* smem_column, int px, int pair, int color,
-                                            int iter) {
+__device__ __forceinline__ void sweep_pixel(const RunArgs& a, float* smem_column, const GeomView* views, int px,
+                                            int pair, int color, int iter) {
     const int py = 2 * pair + ((px & 1) ^ color);
     const int W = a.W, H = a.H, S = a.S;
     if (px >= W || py >= H || pair >= a.cover_pairs) return;
@@ -781,7 +796,7 @@ __device__ __forceinline__ void sweep_pixel(const RunArgs& a, float* smem_column
     }
     float rows[Scratch<NS, BLK>::kRowWords];
     float4 cand[8];
-    const Scratch<NS, BLK> s{ smem_column, rows, cand };
+    const Scratch<NS, BLK> s{ smem_column, rows, cand, views };
     Patch P;
     build_patch(a, px, py, P, rows);
     const uint32_t all_views = (S >= 32) ? 0xffffffffu : ((1u << S) - 1u);
@@ -1121,12 +1136,34 @@ __device__ __forceinline__ void sweep_pixel(const RunArgs& a, float* smem_column
     }
 }
 
+// The views' geometry into shared memory, behind the threads' columns; every thread of the block calls it.
+template <int NS, int BLK>
+__device__ __forceinline__ GeomView* load_geom_views(const RunArgs& a, float* smem, int tid) {
+    GeomView* views = reinterpret_cast<GeomView*>(smem + Scratch<NS, BLK>::kWords * BLK);
+    if (a.prm.mode & HPM_MODE_GEOM) {
+        for (int j = tid; j < a.S; j += BLK) {
+            GeomView v;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) { v.fwd_A[k] = a.fwd[j + 1].A[k]; v.bwd_A[k] = a.bwd[j + 1].A[k]; }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) { v.fwd_b[k] = a.fwd[j + 1].b[k]; v.bwd_b[k] = a.bwd[j + 1].b[k]; }
+            v.depth = a.depth_src[j + 1];
+            v.w = a.dsw[j + 1];
+            v.h = a.dsh[j + 1];
+            views[j] = v;
+        }
+        __syncthreads();
+    }
+    return views;
+}
+
 template <int NS, int BLK, bool MAND, bool CNT>
 __global__ void __launch_bounds__(BLK, kSweepBlocks) k_half_sweep(const __grid_constant__ RunArgs a, int color, int iter) {
     extern __shared__ float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    sweep_pixel<NS, BLK, MAND, CNT>(a, smem + tid, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y,
-                                    color, iter);
+    const GeomView* views = load_geom_views<NS, BLK>(a, smem, tid);
+    sweep_pixel<NS, BLK, MAND, CNT>(a, smem + tid, views, blockIdx.x * blockDim.x + threadIdx.x,
+                                    blockIdx.y * blockDim.y + threadIdx.y, color, iter);
 }
 
 // Prior mode with work lists (RunArgs::active_px): thread x of a row pair takes the x-th pixel the
@@ -1143,7 +1180,7 @@ __global__ void __launch_bounds__(BLK, kSweepBlocks) k_half_sweep_listed(const _
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= a.active_n[k]) return;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    sweep_pixel<NS, BLK, false, CNT>(a, smem + tid, a.active_px[(size_t)k * a.W + x], pair, color, iter);
+    sweep_pixel<NS, BLK, false, CNT>(a, smem + tid, nullptr, a.active_px[(size_t)k * a.W + x], pair, color, iter);
 }
 
 #ifndef HPM_NS
@@ -1195,7 +1232,7 @@ __global__ void __launch_bounds__(BLK, kSweepBlocks)
         if (pair >= a.cover_pairs) continue;
         const int r = color * a.cover_pairs + pair;
         if (x >= a.active_n[r]) continue;
-        sweep_pixel<NS, BLK, false, CNT>(a, smem + tid, a.active_px[(size_t)r * a.W + x], pair, color, iter);
+        sweep_pixel<NS, BLK, false, CNT>(a, smem + tid, nullptr, a.active_px[(size_t)r * a.W + x], pair, color, iter);
     }
 }
 
@@ -1211,7 +1248,9 @@ __global__ void __launch_bounds__(BLK, kSweepBlocks)
         const RunArgs& a = args[k];
         const int t = b - __ldg(tile_start + k);
         const int tx = (a.W + blockDim.x - 1) / blockDim.x;
-        sweep_pixel<NS, BLK, MAND, CNT>(a, smem + tid, (t % tx) * blockDim.x + threadIdx.x,
+        if (a.prm.mode & HPM_MODE_GEOM) __syncthreads();  // the tile before may still read its views
+        const GeomView* views = load_geom_views<NS, BLK>(a, smem, tid);
+        sweep_pixel<NS, BLK, MAND, CNT>(a, smem + tid, views, (t % tx) * blockDim.x + threadIdx.x,
                                         (t / tx) * blockDim.y + threadIdx.y, color, iter);
     }
 }
@@ -1264,7 +1303,7 @@ cudaError_t init_impl(const RunArgs& a, cudaStream_t st) {
 
 template <int NS>
 static constexpr size_t sweep_smem() {
-    return sizeof(float) * Scratch<NS, kSweepThreads>::kWords * kSweepThreads;
+    return sizeof(float) * Scratch<NS, kSweepThreads>::kWords * kSweepThreads + sizeof(GeomView) * NS;
 }
 
 template <int NS, bool MAND, bool CNT>
