@@ -63,7 +63,7 @@ struct alignas(16) GeomView {
 };
 static_assert(sizeof(GeomView) == 112, "seven 16-byte loads");
 
-// Per-thread scratch of a half-sweep.  The cost rows of the eight directions are written once, an NCC
+// Per-thread scratch of a half-sweep, in blocks of at most BLK threads.  The cost rows of the eight directions are written once, an NCC
 // apart, and read once, by view selection: they stream through the thread's local memory, so that
 // shared memory (view weights, final costs, candidate positions) leaves the L1 to the textures and
 // the registers alone bound the resident warps.  After view selection the rows' words hold the
@@ -1141,7 +1141,7 @@ template <int NS, int BLK>
 __device__ __forceinline__ GeomView* load_geom_views(const RunArgs& a, float* smem, int tid) {
     GeomView* views = reinterpret_cast<GeomView*>(smem + Scratch<NS, BLK>::kWords * BLK);
     if (a.prm.mode & HPM_MODE_GEOM) {
-        for (int j = tid; j < a.S; j += BLK) {
+        for (int j = tid; j < a.S; j += blockDim.x * blockDim.y) {
             GeomView v;
 #pragma unroll
             for (int k = 0; k < 9; ++k) { v.fwd_A[k] = a.fwd[j + 1].A[k]; v.bwd_A[k] = a.bwd[j + 1].A[k]; }
@@ -1306,10 +1306,25 @@ static constexpr size_t sweep_smem() {
     return sizeof(float) * Scratch<NS, kSweepThreads>::kWords * kSweepThreads + sizeof(GeomView) * NS;
 }
 
+// Row pairs of a block, one warp each.  An image of less than one wave of four-warp blocks runs in
+// two-warp blocks, which spread over the SMs more evenly: 320x240 has 300 blocks of four warps for
+// 3 x 148 places, and its half-sweeps take 142 instead of 155 us (photometric, 4 sources), 297 instead
+// of 313 (prior, 10 sources).  From 400x300 on (494 blocks) four warps are as fast or faster, since the
+// warps of a block share what they fetch.
+static int block_pairs(int blocks_of_four) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 4;
+    return blocks_of_four < kSweepBlocks * sms ? 2 : 4;
+}
+
 template <int NS, bool MAND, bool CNT>
 cudaError_t sweep_impl(const RunArgs& a, int color, int iter, cudaStream_t st) {
     constexpr int BLK = kSweepThreads, BX = 32;
-    dim3 block(BX, BLK / BX), grid((a.W + BX - 1) / BX, (a.cover_pairs + BLK / BX - 1) / (BLK / BX));
+    const int across = (a.W + BX - 1) / BX;
+    const int pairs = block_pairs(across * ((a.cover_pairs + 3) / 4));
+    const dim3 block(BX, pairs), grid(across, (a.cover_pairs + pairs - 1) / pairs);
     if (!MAND && a.active_px)
         k_half_sweep_listed<NS, BLK, CNT><<<grid, block, sweep_smem<NS>(), st>>>(a, color, iter);
     else
