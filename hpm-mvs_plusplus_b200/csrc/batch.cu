@@ -130,7 +130,7 @@ int Ctx::tune_batch(const BatchLaunch& base, int n, size_t total_px, uint64_t ke
     if (!rc) {
         cudaEventRecord(t0, stream);
         for (int k = 0; k < n && !rc; ++k) {
-            if ((e = launch_half_sweep(h_bargs[k], 0, 0, stream)) != cudaSuccess) rc = cuda_fail(e, "autotuner launch");
+            if ((e = launch_half_sweep(h_bargs[k], 0, 0, 0, h_bargs[k].cover_pairs, stream)) != cudaSuccess) rc = cuda_fail(e, "autotuner launch");
             ++launches;
         }
         cudaEventRecord(t1, stream);
@@ -300,7 +300,7 @@ int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int
         }
         for (int k = 0; k < n; ++k) {
             if ((r = record_start(1, t))) return r;
-            if ((e = launch_half_sweep(h_bargs[k], color, iter, stream)) != cudaSuccess)
+            if ((e = launch_half_sweep(h_bargs[k], color, iter, 0, h_bargs[k].cover_pairs, stream)) != cudaSuccess)
                 return cuda_fail(e, "half sweep");
             if (t) cudaEventRecord(t->stop, stream);
             ++launches;

@@ -108,6 +108,12 @@ Ctx::~Ctx() {
     if (prof_hyp) cudaFree(prof_hyp);
     if (half_stage) cudaFree(half_stage);
     if (level_flags) cudaFree(level_flags);
+    for (int b = 0; b < kBands; ++b) {
+        if (band_stream[b]) cudaStreamDestroy(band_stream[b]);
+        for (auto& parity : band_done)
+            if (parity[b]) cudaEventDestroy(parity[b]);
+    }
+    if (band_start) cudaEventDestroy(band_start);
     if (stream) cudaStreamDestroy(stream);
 }
 

@@ -145,10 +145,17 @@ struct Ctx {
     };
     std::vector<BatchGraph> batch_graphs;
 
+    // Half-sweeps in bands of rows (Ctx::launch_sweeps): band 0 runs on the context's stream, the others on
+    // these, which wait for the context's stream before a run and are waited for by it after the run.
+    static constexpr int kBands = 4;
+    cudaStream_t band_stream[kBands] = {};       // [0] unused
+    cudaEvent_t band_done[2][kBands] = {};       // by parity of the half-sweep
+    cudaEvent_t band_start = nullptr;
+
     // profiling (hpm_profile_enable): CUDA events around every PatchMatch
     // kernel launch, read back and summed by hpm_profile_read
     int prof_flags = 0;
-    struct TimedLaunch { cudaEvent_t start, stop; int kind; };
+    struct TimedLaunch { cudaEvent_t start, stop; int kind; int launches; };
     std::vector<TimedLaunch> prof_events;  // pool; the first prof_used are pending
     size_t prof_used = 0;
     unsigned long long* prof_hyp = nullptr;  // device counters [init, sweep credited, sweep sampled]
@@ -174,6 +181,8 @@ struct Ctx {
                   const hpm_params* params, int texture_level, const uint64_t* seeds);
     int tune_batch(const BatchLaunch& bl, int n, size_t total_px, uint64_t key, BatchShape& out);
     int launch_schedule(const RunArgs& a, int n_half_sweeps);
+    int launch_sweeps(const RunArgs& a, int n_half_sweeps);
+    bool ensure_bands();
     int debug_run_partial(int ref, const int32_t* srcs, int n_src, const hpm_params* params, int texture_level,
                           uint64_t seed, int n_half_sweeps, float* planes_out, float* costs_out, uint32_t* sel_out,
                           uint32_t* draws_out);

@@ -1158,12 +1158,14 @@ __device__ __forceinline__ GeomView* load_geom_views(const RunArgs& a, float* sm
 }
 
 template <int NS, int BLK, bool MAND, bool CNT>
-__global__ void __launch_bounds__(BLK, kSweepBlocks) k_half_sweep(const __grid_constant__ RunArgs a, int color, int iter) {
+__global__ void __launch_bounds__(BLK, kSweepBlocks) k_half_sweep(const __grid_constant__ RunArgs a, int color, int iter,
+                                                                    int first_pair, int last_pair) {
     extern __shared__ float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const GeomView* views = load_geom_views<NS, BLK>(a, smem, tid);
-    sweep_pixel<NS, BLK, MAND, CNT>(a, smem + tid, views, blockIdx.x * blockDim.x + threadIdx.x,
-                                    blockIdx.y * blockDim.y + threadIdx.y, color, iter);
+    const int pair = first_pair + blockIdx.y * blockDim.y + threadIdx.y;
+    if (pair >= last_pair) return;
+    sweep_pixel<NS, BLK, MAND, CNT>(a, smem + tid, views, blockIdx.x * blockDim.x + threadIdx.x, pair, color, iter);
 }
 
 // Prior mode with work lists (RunArgs::active_px): thread x of a row pair takes the x-th pixel the
@@ -1172,10 +1174,11 @@ __global__ void __launch_bounds__(BLK, kSweepBlocks) k_half_sweep(const __grid_c
 // other colour's state, so the mapping does not change any result.
 template <int NS, int BLK, bool CNT>
 __global__ void __launch_bounds__(BLK, kSweepBlocks) k_half_sweep_listed(const __grid_constant__ RunArgs a,
-                                                                                 int color, int iter) {
+                                                                         int color, int iter, int first_pair,
+                                                                         int last_pair) {
     extern __shared__ float smem[];
-    const int pair = blockIdx.y * blockDim.y + threadIdx.y;
-    if (pair >= a.cover_pairs) return;
+    const int pair = first_pair + blockIdx.y * blockDim.y + threadIdx.y;
+    if (pair >= last_pair) return;
     const int k = color * a.cover_pairs + pair;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= a.active_n[k]) return;
@@ -1306,29 +1309,33 @@ static constexpr size_t sweep_smem() {
     return sizeof(float) * Scratch<NS, kSweepThreads>::kWords * kSweepThreads + sizeof(GeomView) * NS;
 }
 
+static int blocks_of_four(const RunArgs& a) { return (a.W + 31) / 32 * ((a.cover_pairs + 3) / 4); }
+
+static bool one_wave(int blocks) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return false;
+    return blocks < kSweepBlocks * sms;
+}
+
 // Row pairs of a block, one warp each.  An image of less than one wave of four-warp blocks runs in
 // two-warp blocks, which spread over the SMs more evenly: 320x240 has 300 blocks of four warps for
 // 3 x 148 places, and its half-sweeps take 142 instead of 155 us (photometric, 4 sources), 297 instead
 // of 313 (prior, 10 sources).  From 400x300 on (494 blocks) four warps are as fast or faster, since the
 // warps of a block share what they fetch.
-static int block_pairs(int blocks_of_four) {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return 4;
-    return blocks_of_four < kSweepBlocks * sms ? 2 : 4;
-}
+static int block_pairs(const RunArgs& a) { return one_wave(blocks_of_four(a)) ? 2 : 4; }
 
 template <int NS, bool MAND, bool CNT>
-cudaError_t sweep_impl(const RunArgs& a, int color, int iter, cudaStream_t st) {
+cudaError_t sweep_impl(const RunArgs& a, int color, int iter, int first_pair, int last_pair, cudaStream_t st) {
     constexpr int BLK = kSweepThreads, BX = 32;
     const int across = (a.W + BX - 1) / BX;
-    const int pairs = block_pairs(across * ((a.cover_pairs + 3) / 4));
-    const dim3 block(BX, pairs), grid(across, (a.cover_pairs + pairs - 1) / pairs);
+    const int pairs = block_pairs(a);
+    const dim3 block(BX, pairs), grid(across, (last_pair - first_pair + pairs - 1) / pairs);
     if (!MAND && a.active_px)
-        k_half_sweep_listed<NS, BLK, CNT><<<grid, block, sweep_smem<NS>(), st>>>(a, color, iter);
+        k_half_sweep_listed<NS, BLK, CNT><<<grid, block, sweep_smem<NS>(), st>>>(a, color, iter, first_pair, last_pair);
     else
-        k_half_sweep<NS, BLK, MAND, CNT><<<grid, block, sweep_smem<NS>(), st>>>(a, color, iter);
+        k_half_sweep<NS, BLK, MAND, CNT><<<grid, block, sweep_smem<NS>(), st>>>(a, color, iter, first_pair, last_pair);
     return cudaGetLastError();
 }
 
@@ -1377,7 +1384,7 @@ int sweep_batch_occupancy() {
     linkage template int sweep_batch_occupancy<NS, false>();                                \
     linkage template int sweep_batch_occupancy<NS, true>();
 #define HPM_SWEEP_FORMS_OF(linkage, NS, MAND, CNT)                                                     \
-    linkage template cudaError_t sweep_impl<NS, MAND, CNT>(const RunArgs&, int, int, cudaStream_t);    \
+    linkage template cudaError_t sweep_impl<NS, MAND, CNT>(const RunArgs&, int, int, int, int, cudaStream_t);    \
     linkage template cudaError_t sweep_batch_impl<NS, MAND, CNT>(const BatchLaunch&, int, int, cudaStream_t);
 
 #ifdef HPM_NS
@@ -1397,13 +1404,14 @@ cudaError_t launch_random_init(const RunArgs& a, cudaStream_t st) {
     return a.hyp_count ? HPM_BY_SOURCES(a.S, init_impl, true)(a, st) : HPM_BY_SOURCES(a.S, init_impl, false)(a, st);
 }
 
-cudaError_t launch_half_sweep(const RunArgs& a, int color, int iter, cudaStream_t st) {
+cudaError_t launch_half_sweep(const RunArgs& a, int color, int iter, int first_pair, int last_pair, cudaStream_t st) {
     const bool mand = a.prm.mode & HPM_MODE_MAND;
+    if (last_pair <= first_pair) return cudaSuccess;
     if (a.hyp_count)
-        return mand ? HPM_BY_SOURCES(a.S, sweep_impl, true, true)(a, color, iter, st)
-                    : HPM_BY_SOURCES(a.S, sweep_impl, false, true)(a, color, iter, st);
-    return mand ? HPM_BY_SOURCES(a.S, sweep_impl, true, false)(a, color, iter, st)
-                : HPM_BY_SOURCES(a.S, sweep_impl, false, false)(a, color, iter, st);
+        return mand ? HPM_BY_SOURCES(a.S, sweep_impl, true, true)(a, color, iter, first_pair, last_pair, st)
+                    : HPM_BY_SOURCES(a.S, sweep_impl, false, true)(a, color, iter, first_pair, last_pair, st);
+    return mand ? HPM_BY_SOURCES(a.S, sweep_impl, true, false)(a, color, iter, first_pair, last_pair, st)
+                : HPM_BY_SOURCES(a.S, sweep_impl, false, false)(a, color, iter, first_pair, last_pair, st);
 }
 
 cudaError_t launch_random_init_batch(const BatchLaunch& bl, cudaStream_t st) {
@@ -1423,6 +1431,7 @@ int half_sweep_batch_occupancy(int max_s, bool mand) {
     return mand ? HPM_BY_SOURCES(max_s, sweep_batch_occupancy, true)() : HPM_BY_SOURCES(max_s, sweep_batch_occupancy, false)();
 }
 
+bool half_sweep_one_wave(const RunArgs& a) { return one_wave(blocks_of_four(a)); }
 int half_sweep_block_threads() { return kSweepThreads; }
 
 cudaError_t launch_export(const RunArgs& a, cudaStream_t st) {

@@ -70,7 +70,10 @@ static_assert(sizeof(RunArgs) <= 32764, "RunArgs exceeds the kernel parameter li
 // Host launchers (pm_kernels.cu).  Return cudaError_t of the launch.
 cudaError_t launch_random_init(const RunArgs& a, cudaStream_t st);
 cudaError_t launch_weight_table(const hpm_params& prm, float* out, cudaStream_t st);
-cudaError_t launch_half_sweep(const RunArgs& a, int color, int iter, cudaStream_t st);
+// Whether a half-sweep's four-warp blocks all fit on the GPU at once.
+bool half_sweep_one_wave(const RunArgs& a);
+// One half-sweep over the row pairs [first_pair, last_pair) (all of them: 0, cover_pairs).
+cudaError_t launch_half_sweep(const RunArgs& a, int color, int iter, int first_pair, int last_pair, cudaStream_t st);
 // Prior mode: the compacted columns of the pixels the half-sweeps update (W * cover_pairs ints and
 // cover_pairs counts per colour in px / n), for RunArgs::active_px / active_n.
 cudaError_t launch_prior_active(const RunArgs& a, int* px, int* n, cudaStream_t st);

@@ -1,0 +1,43 @@
+"""Half-sweeps in bands of rows on several streams, as a single run above one wave of blocks takes them,
+against the whole-image launches of the batching form on the same views: the maps are equal bit for bit.
+The heights give bands of 16 row pairs and more with each remainder of the four-row-pair blocks.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import hpm_b200
+from test_gpu_batch import _load, _maps, _same
+
+pytestmark = pytest.mark.gpu
+
+
+# 32-pixel columns x four-pair rows of blocks: 444 places on 148 SMs; one band, two, three, four bands
+@pytest.mark.parametrize("width,height", [(2250, 47), (1700, 70), (1200, 103), (640, 166), (417, 301)])
+@pytest.mark.parametrize("mode", [0, hpm_b200.MODE_GEOM, hpm_b200.MODE_GEOM | hpm_b200.MODE_MAND,
+                                  hpm_b200.MODE_PRIOR])
+def test_bands_equal_whole_launches(width, height, mode):
+    from hpm_b200 import synth
+    scene = synth.make_scene(n_views=3, width=width, height=height, n_src=2, seed=21, supersample=1)
+    srcs = [[j for j, _ in p] for p in scene.pairs]
+    refs = [0, 1]
+    kind = hpm_b200.MAP_DEPTH_GEOM if mode & hpm_b200.MODE_GEOM else hpm_b200.MAP_DEPTH
+    out = []
+    for batched in (False, True):
+        with hpm_b200.Context(0) as ctx:
+            cams = _load(ctx, scene)
+            if mode == hpm_b200.MODE_PRIOR:
+                for r in refs:
+                    ctx.build_prior(r, 0)
+            params = [hpm_b200.Params.make(len(srcs[r]) + 1, *hpm_b200.widened_range(cams[r]), mode=mode)
+                      for r in refs]
+            if batched:
+                ctx.run_batch(refs, [srcs[r] for r in refs], params, [31, 32])
+            else:
+                for k, r in enumerate(refs):
+                    ctx.run_patchmatch(r, srcs[r], params[k], seed=31 + k)
+            out.append(_maps(ctx, refs, kind))
+    for a, b in zip(*out):
+        for x, y in zip(a, b):
+            assert np.isfinite(x).any() and _same(x, y)
