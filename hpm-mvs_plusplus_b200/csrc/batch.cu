@@ -155,6 +155,49 @@ int Ctx::tune_batch(const BatchLaunch& base, int n, size_t total_px, uint64_t ke
     return HPM_OK;
 }
 
+// The half-sweeps of a batch, its runs in two groups of about the same number of tiles, each on a stream
+// of its own: runs read nothing of one another, so the last, partly filled wave of one group's launch runs
+// beside the other group's blocks.  One group and two on B200, a whole batch: 5 views of 320x240
+// photometric 3.99 and 3.48 ms, prior 2.14 and 1.82, 48 of 64x48 2.37 and 1.99, 12 of 200x150 with 10
+// sources mandatory 8.19 and 7.25, 6 of 640x480 19.0 and 18.8, 5 of 1280x960 no change.  Three and four
+// groups give what two do.  A persistent grid fills the GPU by itself and stays one group.
+int Ctx::launch_batch_sweeps(const BatchLaunch& all, const int* tile_start, int n_half_sweeps) {
+    cudaError_t e = cudaSuccess;
+    TimedLaunch* t = nullptr;
+    int rc = HPM_OK;
+    const int groups = all.n > 1 && !all.grid_blocks && n_half_sweeps > 1 && ensure_bands() ? 2 : 1;
+    BatchLaunch group[2] = { all, all };
+    if (groups == 2) {
+        int k = 1;  // runs of the first group: up to the run with the middle tile in its second half
+        while (k + 1 < all.n && tile_start[k] + tile_start[k + 1] < all.tiles) ++k;
+        group[0].n = k;
+        group[0].tiles = tile_start[k];
+        group[1].args += k;
+        group[1].tile_start += k;
+        group[1].n = all.n - k;
+        group[1].tiles = all.tiles - tile_start[k];
+    }
+    cudaStream_t const streams[2] = { stream, band_stream[1] };
+    if ((rc = record_start(1, t))) return rc;
+    if (t) t->launches = n_half_sweeps;  // timed together
+    if (groups == 2 && ((e = cudaEventRecord(band_start, stream)) != cudaSuccess ||
+                        (e = cudaStreamWaitEvent(streams[1], band_start, 0)) != cudaSuccess))
+        return cuda_fail(e, "batch streams");
+    for (int s = 0; s < n_half_sweeps; ++s)
+        for (int g = 0; g < groups && e == cudaSuccess; ++g) {
+            e = launch_half_sweep_batch(group[g], s & 1, s >> 1, streams[g]);
+            ++launches;
+        }
+    if (groups == 2 && e == cudaSuccess && (e = cudaEventRecord(band_done[0][1], streams[1])) == cudaSuccess)
+        e = cudaStreamWaitEvent(stream, band_done[0][1], 0);
+    if (e != cudaSuccess) {  // the other stream's work ends before the context goes on
+        if (groups == 2) cudaStreamSynchronize(streams[1]);
+        return cuda_fail(e, "batched half sweeps");
+    }
+    if (t) cudaEventRecord(t->stop, stream);
+    return HPM_OK;
+}
+
 int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int32_t* src_ids,
                    const hpm_params* params, int texture_level, const uint64_t* seeds) {
     cudaSetDevice(device);
@@ -287,24 +330,18 @@ int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int
     bs.tiles = h_btiles[(n + 1) + n];
     bs.bx = shape.bx;
 
-    // one half-sweep stage of every run: one batched launch, or the single-view kernel per run
-    auto sweep_stage = [&](int color, int iter, TimedLaunch*& t) -> int {
+    // the half-sweeps of every run: batched launches stage by stage, or the single-view kernel per run
+    auto sweeps = [&](TimedLaunch*& t) -> int {
+        if (!shape.perview) return launch_batch_sweeps(bs, h_btiles + (n + 1), 2 * iters);
         int r = HPM_OK;
-        if (!shape.perview) {
-            if ((r = record_start(1, t))) return r;
-            if ((e = launch_half_sweep_batch(bs, color, iter, stream)) != cudaSuccess)
-                return cuda_fail(e, "batched half sweep");
-            if (t) cudaEventRecord(t->stop, stream);
-            ++launches;
-            return HPM_OK;
-        }
-        for (int k = 0; k < n; ++k) {
-            if ((r = record_start(1, t))) return r;
-            if ((e = launch_half_sweep(h_bargs[k], color, iter, 0, h_bargs[k].cover_pairs, stream)) != cudaSuccess)
-                return cuda_fail(e, "half sweep");
-            if (t) cudaEventRecord(t->stop, stream);
-            ++launches;
-        }
+        for (int s = 0; s < 2 * iters; ++s)
+            for (int k = 0; k < n; ++k) {
+                if ((r = record_start(1, t))) return r;
+                if ((e = launch_half_sweep(h_bargs[k], s & 1, s >> 1, 0, h_bargs[k].cover_pairs, stream)) != cudaSuccess)
+                    return cuda_fail(e, "half sweep");
+                if (t) cudaEventRecord(t->stop, stream);
+                ++launches;
+            }
         return HPM_OK;
     };
     const bool timing = prof_flags & HPM_PROFILE_TIMING;
@@ -317,9 +354,7 @@ int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int
         if ((e = launch_random_init_batch(bi, stream)) != cudaSuccess) return cuda_fail(e, "batched init launch");
         if (t) cudaEventRecord(t->stop, stream);
         ++launches;
-        for (int k = 0; k < 2 * iters; ++k)
-            if ((rc = sweep_stage(k & 1, k >> 1, t))) return rc;
-        return HPM_OK;
+        return sweeps(t);
     };
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -328,7 +363,8 @@ int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int
     };
     set_grid();
     // a graph of per-view launches would hold this batch's RunArgs as parameters; the batched kernels read
-    // theirs from device memory, refreshed before every replay
+    // theirs from device memory, refreshed before every replay (their blocks walk whatever tiles the table
+    // gives their group of runs)
     BatchGraph* graph = nullptr;
     if (use_graph && have_shape && !shape.perview)
         for (auto& g : batch_graphs)
@@ -338,7 +374,7 @@ int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int
                 graph = &g;
     if (graph) {
         if ((e = cudaGraphLaunch(graph->exec, stream)) != cudaSuccess) return cuda_fail(e, "batch graph launch");
-        launches += 1 + 2 * iters * (shape.perview ? n : 1);
+        launches += graph->launches;
     } else if (!have_shape && (batch_flags & HPM_BATCH_AUTOTUNE) && iters > 0) {
         // initialise, tune the half-sweep on a snapshot of the initialised state, then sweep
         if ((rc = record_start(0, t))) return rc;
@@ -353,8 +389,7 @@ int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int
         bs.tiles = h_btiles[(n + 1) + n];
         bs.bx = shape.bx;
         set_grid();
-        for (int k = 0; k < 2 * iters; ++k)
-            if ((rc = sweep_stage(k & 1, k >> 1, t))) return rc;
+        if ((rc = sweeps(t))) return rc;
     } else {
         if ((rc = schedule())) return rc;
         if (use_graph && !shape.perview) {
@@ -364,6 +399,7 @@ int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int
                 return cuda_fail(e, "batch graph capture");
             const int64_t l0 = launches;
             const int crc = schedule();
+            const int64_t recorded = launches - l0;
             const cudaError_t ce = cudaStreamEndCapture(stream, &g);
             launches = l0;
             if (crc) { if (g) cudaGraphDestroy(g); return crc; }
@@ -376,6 +412,7 @@ int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int
             bg.n = n; bg.init_tiles = bi.tiles; bg.sweep_tiles = bs.tiles; bg.max_s = max_s; bg.mand = mand;
             bg.listed = listed;
             bg.iters = iters; bg.bx = bs.bx; bg.grid = bs.grid_blocks; bg.perview = shape.perview; bg.exec = ex;
+            bg.launches = recorded;
             batch_graphs.push_back(bg);
         }
     }

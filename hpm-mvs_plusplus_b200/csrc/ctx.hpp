@@ -141,14 +141,16 @@ struct Ctx {
     struct BatchGraph {
         int n = 0, init_tiles = 0, sweep_tiles = 0, max_s = 0, iters = 0, bx = 0, grid = 0;
         bool mand = false, perview = false, listed = false;
+        int64_t launches = 0;
         cudaGraphExec_t exec = nullptr;
     };
     std::vector<BatchGraph> batch_graphs;
 
     unsigned int* grad_oob = nullptr;  // pinned: skipped accesses of the gradient kernels (grad.cu)
 
-    // Half-sweeps in bands of rows (Ctx::launch_sweeps): band 0 runs on the context's stream, the others on
-    // these, which wait for the context's stream before a run and are waited for by it after the run.
+    // Half-sweeps in bands of rows (Ctx::launch_sweeps) and batches in two groups (Ctx::launch_batch_sweeps):
+    // the first part runs on the context's stream, the others on these, which wait for the context's stream
+    // before the half-sweeps and are waited for by it after them.
     static constexpr int kBands = 4;
     cudaStream_t band_stream[kBands] = {};       // [0] unused
     cudaEvent_t band_done[2][kBands] = {};       // by parity of the half-sweep
@@ -184,6 +186,7 @@ struct Ctx {
     int tune_batch(const BatchLaunch& bl, int n, size_t total_px, uint64_t key, BatchShape& out);
     int launch_schedule(const RunArgs& a, int n_half_sweeps);
     int launch_sweeps(const RunArgs& a, int n_half_sweeps);
+    int launch_batch_sweeps(const BatchLaunch& all, const int* tile_start, int n_half_sweeps);
     bool ensure_bands();
     int debug_run_partial(int ref, const int32_t* srcs, int n_src, const hpm_params* params, int texture_level,
                           uint64_t seed, int n_half_sweeps, float* planes_out, float* costs_out, uint32_t* sel_out,

@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(BLK, kSweepBlocks) k_random_init_batch(const R
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const InitScratch<NS, BLK> s{ smem + tid };
     const int total = __ldg(tile_start + n);
-    for (int b = blockIdx.x; b < total; b += gridDim.x) {
+    for (int b = __ldg(tile_start) + blockIdx.x; b < total; b += gridDim.x) {
         const int k = batch_run_of(tile_start, n, b);
         const RunArgs& a = args[k];
         const int t = b - __ldg(tile_start + k);
@@ -1225,7 +1225,7 @@ __global__ void __launch_bounds__(BLK, kSweepBlocks)
     extern __shared__ float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const int total = __ldg(tile_start + n);
-    for (int b = blockIdx.x; b < total; b += gridDim.x) {
+    for (int b = __ldg(tile_start) + blockIdx.x; b < total; b += gridDim.x) {
         const int k = batch_run_of(tile_start, n, b);
         const RunArgs& a = args[k];
         const int t = b - __ldg(tile_start + k);
@@ -1246,7 +1246,7 @@ __global__ void __launch_bounds__(BLK, kSweepBlocks)
     extern __shared__ float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const int total = __ldg(tile_start + n);
-    for (int b = blockIdx.x; b < total; b += gridDim.x) {
+    for (int b = __ldg(tile_start) + blockIdx.x; b < total; b += gridDim.x) {
         const int k = batch_run_of(tile_start, n, b);
         const RunArgs& a = args[k];
         const int t = b - __ldg(tile_start + k);

@@ -1,6 +1,10 @@
-"""Half-sweeps in bands of rows on several streams, as a single run above one wave of blocks takes them,
+"""Half-sweeps on several streams.
+
+In bands of rows, as a single run above one wave of blocks takes them,
 against the whole-image launches of the batching form on the same views: the maps are equal bit for bit.
 The heights give bands of 16 row pairs and more with each remainder of the four-row-pair blocks.
+
+In two groups of a batch's runs, with the large views first, last and alone: the maps of single runs.
 """
 from __future__ import annotations
 
@@ -41,3 +45,28 @@ def test_bands_equal_whole_launches(width, height, mode):
     for a, b in zip(*out):
         for x, y in zip(a, b):
             assert np.isfinite(x).any() and _same(x, y)
+
+
+@pytest.mark.parametrize("heights", [(40, 40), (200, 8, 8), (8, 8, 200), (24, 40, 24, 56, 8, 16)])
+def test_groups_equal_single_runs(heights):
+    from hpm_b200 import synth
+    n = len(heights)
+    scene = synth.make_scene(n_views=n, width=96, height=72, n_src=1, seed=22, supersample=1,
+                             sizes=[(96, h) for h in heights])
+    srcs = [[j for j, _ in p] for p in scene.pairs]
+    out = []
+    for batched in (False, True):
+        with hpm_b200.Context(0) as ctx:
+            ctx.set_batch_options(0)
+            cams = _load(ctx, scene)
+            params = [hpm_b200.Params.make(len(srcs[r]) + 1, *hpm_b200.widened_range(cams[r]), mode=0)
+                      for r in range(n)]
+            if batched:
+                ctx.run_batch(list(range(n)), srcs, params, list(range(40, 40 + n)))
+            else:
+                for r in range(n):
+                    ctx.run_patchmatch(r, srcs[r], params[r], seed=40 + r)
+            out.append(_maps(ctx, range(n), hpm_b200.MAP_DEPTH))
+    for a, b in zip(*out):
+        for x, y in zip(a, b):
+            assert _same(x, y)
