@@ -108,7 +108,6 @@ Ctx::~Ctx() {
     if (prof_hyp) cudaFree(prof_hyp);
     if (half_stage) cudaFree(half_stage);
     if (level_flags) cudaFree(level_flags);
-    if (grad_oob) cudaFreeHost(grad_oob);
     for (int b = 0; b < kBands; ++b) {
         if (band_stream[b]) cudaStreamDestroy(band_stream[b]);
         for (auto& parity : band_done)

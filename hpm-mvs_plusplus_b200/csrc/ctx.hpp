@@ -146,8 +146,6 @@ struct Ctx {
     };
     std::vector<BatchGraph> batch_graphs;
 
-    unsigned int* grad_oob = nullptr;  // pinned: skipped accesses of the gradient kernels (grad.cu)
-
     // Half-sweeps in bands of rows (Ctx::launch_sweeps) and batches in two groups (Ctx::launch_batch_sweeps):
     // the first part runs on the context's stream, the others on these, which wait for the context's stream
     // before the half-sweeps and are waited for by it after them.
@@ -207,7 +205,6 @@ struct Ctx {
     int reconstruct(int n_views, const hpm_camera* cams, const int32_t* src_off, const int32_t* src_ids,
                     const hpm_recon_options* opt, int64_t* n_points_out);
     cudaError_t ensure_scratch(size_t bytes);
-    cudaError_t grad_oob_reset(RunArgs& a);
     int fill_src_images(const int32_t* srcs, int n_src, SrcImages& si);
     int eval_cost_grad(int ref, const int32_t* srcs, int n_src, const hpm_params* params, int n, const int32_t* px,
                        const float* theta, float* cost, float* grad);

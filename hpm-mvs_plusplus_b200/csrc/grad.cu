@@ -37,12 +37,9 @@ struct SrcImages {
 namespace {
 
 // Self-check of the gradient kernels: an index outside its buffer (which the
-// clamping below rules out) is counted in *oob and the access skipped, so a
-// wrong index surfaces as an error status instead of a memory fault.  The
-// counter is a word of pinned host memory of the context: a launch without such
-// an index neither writes nor copies it.  Setting and reading a device symbol
-// instead took two copies a call (10000 pixels x 10 views: 181 and 165 us a call).
-__device__ __forceinline__ void count_oob(unsigned int* oob) { atomicAdd_system(oob, 1u); }
+// clamping below rules out) is counted here and the access skipped, so a
+// wrong index surfaces as an error status instead of a memory fault.
+__device__ unsigned int g_grad_oob;
 
 // Exact bilinear sample with clamp-to-edge addressing and, with GRAD, its
 // derivatives.  The position is first clamped to [-2, size + 1] (a NaN to -2):
@@ -50,8 +47,7 @@ __device__ __forceinline__ void count_oob(unsigned int* oob) { atomicAdd_system(
 // gradient are unchanged, and the integer tap index x0 + 1 cannot overflow for a
 // sample position near a plane's horizon, where X grows without bound.
 template <bool GRAD>
-__device__ __forceinline__ float bilinear(const float* img, int w, int h, float X, float Y, float& gx, float& gy,
-                                          unsigned int* oob) {
+__device__ __forceinline__ float bilinear(const float* img, int w, int h, float X, float Y, float& gx, float& gy) {
     X = fminf(fmaxf(X, -2.0f), (float)w + 1.0f);
     Y = fminf(fmaxf(Y, -2.0f), (float)h + 1.0f);
     const float fx = floorf(X), fy = floorf(Y);
@@ -61,7 +57,7 @@ __device__ __forceinline__ float bilinear(const float* img, int w, int h, float 
     const int ya = min(max(y0, 0), h - 1), yb = min(max(y0 + 1, 0), h - 1);
     if ((unsigned)xa >= (unsigned)w || (unsigned)xb >= (unsigned)w || (unsigned)ya >= (unsigned)h ||
         (unsigned)yb >= (unsigned)h) {
-        count_oob(oob);
+        atomicAdd(&g_grad_oob, 1u);
         gx = gy = 0.0f;
         return 0.0f;
     }
@@ -199,7 +195,7 @@ __device__ __forceinline__ float cost_grad_view(const RunArgs& a, const View& vi
     const float* img = view.img;
     const int sw = view.w, sh = view.h;
     if (!img || sw <= 0 || sh <= 0) {
-        count_oob(a.grad_oob);
+        atomicAdd(&g_grad_oob, 1u);
         return 2.0f;
     }
     {
@@ -216,7 +212,7 @@ __device__ __forceinline__ float cost_grad_view(const RunArgs& a, const View& vi
         const float X = (H[0] * ux + H[1] * uy + H[2]) / qz;
         const float Y = (H[3] * ux + H[4] * uy + H[5]) / qz;
         float gx, gy;
-        v[k] = bilinear<false>(img, sw, sh, X, Y, gx, gy, a.grad_oob);
+        v[k] = bilinear<false>(img, sw, sh, X, Y, gx, gy);
         Ss += P.w[k] * v[k];
     }
     Ss /= P.W;
@@ -242,7 +238,7 @@ __device__ __forceinline__ float cost_grad_view(const RunArgs& a, const View& vi
         const float X = (H[0] * ux + H[1] * uy + H[2]) / qz;
         const float Y = (H[3] * ux + H[4] * uy + H[5]) / qz;
         float gx, gy;
-        bilinear<true>(img, sw, sh, X, Y, gx, gy, a.grad_oob);
+        bilinear<true>(img, sw, sh, X, Y, gx, gy);
         const float dcdv = P.w[k] / P.W * (-(P.r[k] - P.mean) / sig + cov * (v[k] - Ss) / (sig * var_s));
         const float gb = (gx * b[0] + gy * b[1] - (gx * X + gy * Y) * b[2]) / qz;
         const float f = -dcdv * gb;
@@ -276,7 +272,7 @@ __global__ void __launch_bounds__(kGradThreads) k_cost_grad(const __grid_constan
         x = px[2 * k];
         y = px[2 * k + 1];
         if (x < 0 || x >= a.W || y < 0 || y >= a.H) {
-            if (L.view == 0) count_oob(a.grad_oob);
+            if (L.view == 0) atomicAdd(&g_grad_oob, 1u);
             on = false;
         }
     }
@@ -321,7 +317,7 @@ __global__ void __launch_bounds__(kGradThreads) k_gn_refine(const __grid_constan
     bool on = L.pixel < L.per_warp && i < n_px;
     const int x = on ? (int)(i % a.W) : 0, y = on ? (int)(i / a.W) : 0;
     if (y >= a.H) {  // more pixels than the image has
-        if (L.view == 0) count_oob(a.grad_oob);
+        if (L.view == 0) atomicAdd(&g_grad_oob, 1u);
         on = false;
     }
     const hpm_camera& c0 = a.cams[0];
@@ -426,19 +422,19 @@ static int grad_blocks(size_t n, int S) {
     return (int)((n + per_block - 1) / per_block);
 }
 
-}  // namespace
-
-// The counter of the self-check, zero for the next launch: every call waits for its kernel, so none is
-// using it.
-cudaError_t Ctx::grad_oob_reset(RunArgs& a) {
-    if (!grad_oob) {
-        const cudaError_t e = cudaHostAlloc((void**)&grad_oob, sizeof(*grad_oob), cudaHostAllocDefault);
-        if (e != cudaSuccess) return e;
-    }
-    *grad_oob = 0;
-    a.grad_oob = grad_oob;
-    return cudaSuccess;
+// Resets the self-check counter before a launch and reads it after one.
+static cudaError_t grad_oob_reset(cudaStream_t st) {
+    const unsigned int zero = 0;
+    return cudaMemcpyToSymbolAsync(g_grad_oob, &zero, sizeof(zero), 0, cudaMemcpyHostToDevice, st);
 }
+
+static cudaError_t grad_oob_read(cudaStream_t st, unsigned int* n) {
+    cudaError_t e = cudaMemcpyFromSymbolAsync(n, g_grad_oob, sizeof(*n), 0, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    return e;
+}
+
+}  // namespace
 
 int Ctx::fill_src_images(const int32_t* srcs, int n_src, SrcImages& si) {
     for (int j = 0; j < n_src; ++j) {
@@ -474,13 +470,12 @@ int Ctx::eval_cost_grad(int ref, const int32_t* srcs, int n_src, const hpm_param
     e = cudaMemcpyAsync(d_px, px, (size_t)n * 8, cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_th, theta, (size_t)n * 12, cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return cuda_fail(e, "upload hypotheses");
-    if ((e = grad_oob_reset(a)) != cudaSuccess) return cuda_fail(e, "self-check reset");
+    if ((e = grad_oob_reset(stream)) != cudaSuccess) return cuda_fail(e, "self-check reset");
     k_cost_grad<<<grad_blocks(n, a.S), kGradThreads, grad_smem(a.S), stream>>>(a, si, n, d_px, d_th, d_c,
                                                                               grad ? d_g : nullptr);
     ++launches;
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "cost gradient launch");
-    if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_fail(e, "cost gradient");
-    const unsigned int oob = *grad_oob;
+    unsigned int oob = 0;
+    if ((e = grad_oob_read(stream, &oob)) != cudaSuccess) return cuda_fail(e, "cost gradient");
     if (oob) return fail(HPM_E_CUDA, "cost gradient: %u out-of-range accesses skipped", oob);
     e = cudaMemcpyAsync(cost, d_c, (size_t)n * n_src * 4, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess && grad) e = cudaMemcpyAsync(grad, d_g, (size_t)n * n_src * 12, cudaMemcpyDeviceToHost, stream);
@@ -501,14 +496,14 @@ int Ctx::eval_cost_grad_device(int ref, const int32_t* srcs, int n_src, const hp
     if ((rc = fill_src_images(srcs, n_src, si))) return rc;
     if (n == 0) return HPM_OK;
     cudaError_t e;
-    if ((e = grad_oob_reset(a)) != cudaSuccess) return cuda_fail(e, "self-check reset");
+    if ((e = grad_oob_reset(stream)) != cudaSuccess) return cuda_fail(e, "self-check reset");
     // pixels outside the reference image are skipped and counted by the kernel (no host copy to check them)
     k_cost_grad<<<grad_blocks(n, a.S), kGradThreads, grad_smem(a.S), stream>>>(a, si, n, d_px, d_theta, d_cost,
                                                                               d_grad);
     ++launches;
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "cost gradient launch");
-    if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_fail(e, "cost gradient");
-    const unsigned int oob = *grad_oob;
+    unsigned int oob = 0;
+    if ((e = grad_oob_read(stream, &oob)) != cudaSuccess) return cuda_fail(e, "cost gradient");
     if (oob) return fail(HPM_E_INVALID, "cost gradient: %u pixels or samples outside their images skipped", oob);
     return HPM_OK;
 }
@@ -530,14 +525,14 @@ int Ctx::gn_refine(int ref, const int32_t* srcs, int n_src, const hpm_params* pa
         return fail(HPM_E_STATE, "view %d needs depth and normal maps of its size", ref);
     cudaError_t e = ensure_map(ref, HPM_MAP_COST, v.w, v.h);
     if (e != cudaSuccess) return cuda_fail(e, "alloc cost map");
-    if ((e = grad_oob_reset(a)) != cudaSuccess) return cuda_fail(e, "self-check reset");
+    if ((e = grad_oob_reset(stream)) != cudaSuccess) return cuda_fail(e, "self-check reset");
     k_gn_refine<<<grad_blocks((size_t)v.w * v.h, a.S), kGradThreads, grad_smem(a.S), stream>>>(
         a, si, steps, dm.ptr, nm.ptr, v.maps[HPM_MAP_COST].ptr, (size_t)v.w * v.h);
     ++launches;
     e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    unsigned int oob = 0;
+    if (e == cudaSuccess) e = grad_oob_read(stream, &oob);
     if (e != cudaSuccess) return cuda_fail(e, "gauss-newton refinement");
-    const unsigned int oob = *grad_oob;
     if (oob) return fail(HPM_E_CUDA, "gauss-newton refinement: %u out-of-range accesses skipped", oob);
     return HPM_OK;
 }

@@ -59,7 +59,6 @@ struct RunArgs {
     // (ComputeMultiViewCostVector, HPM.cu:490-495); [2] the half-sweeps' NCCs
     // that sampled the source (36 filtered fetches each)
     unsigned long long* hyp_count;
-    unsigned int* grad_oob;  // skipped accesses of the gradient kernels (grad.cu), in host memory
 };
 
 constexpr int kWeightTable = 6 * 256;  // six patch distances x level differences 0..255
