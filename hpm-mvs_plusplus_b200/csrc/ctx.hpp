@@ -171,6 +171,8 @@ struct Ctx {
     cudaError_t ensure_run(size_t n);
     int bind_texture(int view);
     int bind_bytes(int view);
+    bool capturing() const;
+    int no_bytes(int view);
     int take_whole_levels(int ref, const int32_t* srcs, float* weights, RunArgs& a);
     int look_at_levels(int ref, const int32_t* srcs, int n_src);
     int fill_run_args(int ref, const int32_t* srcs, int n_src, const hpm_params* params, RunArgs& a);

@@ -50,17 +50,20 @@ __global__ void k_whole_levels(const float* __restrict__ gray, int n, int* __res
     }
 }
 
+bool Ctx::capturing() const {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+}
+
 // Finds out which of a run's images hold whole levels 0..255 only, as every image made by
-// hpm_prepare_level does.  Images from hpm_set_view are looked at once, when a run first uses them;
-// under stream capture, where their contents can still change, they are taken as they are.
+// hpm_prepare_level does.  Images from hpm_set_view are looked at once, when a run first uses them.
+// Not under stream capture: a replay reads the images of its time.
 int Ctx::look_at_levels(int ref, const int32_t* srcs, int n_src) {
     bool unknown = views[ref].whole_levels < 0;
     for (int j = 0; j < n_src; ++j) unknown = unknown || views[srcs[j]].whole_levels < 0;
     if (!unknown) return HPM_OK;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    cudaError_t e = cudaStreamIsCapturing(stream, &cap);
-    if (e != cudaSuccess) return cuda_fail(e, "capture status");
-    if (cap != cudaStreamCaptureStatusNone) return HPM_OK;
+    if (capturing()) return HPM_OK;
+    cudaError_t e;
     if ((e = ensure_buf(level_flags, level_flags_cap, HPM_MAX_VIEWS)) != cudaSuccess) return cuda_fail(e, "alloc level flags");
     int flags[HPM_MAX_VIEWS];
     e = cudaMemsetAsync(level_flags, 0xff, sizeof(flags), stream);
@@ -103,6 +106,14 @@ static cudaError_t make_texture(cudaArray_t arr, int addr_mode, cudaTextureReadM
     return cudaCreateTextureObject(tex, &rd, &td, nullptr);
 }
 
+// Where there is no memory for the copy below, the view stays on its float image.
+int Ctx::no_bytes(int view) {
+    cudaGetLastError();
+    views[view].whole_levels = 0;
+    views[view].bytes_bound = false;
+    return HPM_OK;
+}
+
 // 8-bit copy of a view's image of whole levels.  The unit filters with weights of 1/256, so an F32
 // fetch is a whole multiple N of 1/256 level, N <= 255 * 256, and an 8-bit fetch is N / 65280 rounded
 // to a multiple of 1/65535: fetch * 65280 lies within 0.4999 of N, and rounding it to the nearest
@@ -112,7 +123,7 @@ int Ctx::bind_bytes(int view) {
     ViewState& v = views[view];
     const size_t n = (size_t)v.w * v.h;
     cudaError_t e = ensure_buf(v.bytes, v.bytes_cap, n);
-    if (e != cudaSuccess) return cuda_fail(e, "alloc byte image");
+    if (e != cudaSuccess) return no_bytes(view);
     k_to_u8<<<(int)((n + 255) / 256), 256, 0, stream>>>(v.gray, (int)n, v.bytes);
     ++launches;
     if (v.arr_fmt != HPM_TEX_F32) return HPM_OK;
@@ -124,11 +135,11 @@ int Ctx::bind_bytes(int view) {
         }
         if (!v.arr8) {
             const cudaChannelFormatDesc fd = cudaCreateChannelDesc(8, 0, 0, 0, cudaChannelFormatKindUnsigned);
-            if ((e = cudaMallocArray(&v.arr8, &fd, v.w, v.h)) != cudaSuccess) return cuda_fail(e, "alloc byte image array");
+            if ((e = cudaMallocArray(&v.arr8, &fd, v.w, v.h)) != cudaSuccess) return no_bytes(view);
             v.arr8_w = v.w; v.arr8_h = v.h;
         }
         if ((e = make_texture(v.arr8, v.arr_mode, cudaReadModeNormalizedFloat, &v.tex8)) != cudaSuccess)
-            return cuda_fail(e, "create byte texture");
+            return no_bytes(view);
         v.arr8_mode = v.arr_mode;
     }
     e = cudaMemcpy2DToArrayAsync(v.arr8, 0, 0, v.bytes, (size_t)v.w, (size_t)v.w, v.h, cudaMemcpyDeviceToDevice, stream);
@@ -343,8 +354,10 @@ int Ctx::prepare_run_into(int ref, const int32_t* srcs, int n_src, const hpm_par
 }
 
 // What a run gains from images of whole levels: the reference's bytes and weight table (pm_kernels.cu,
-// build_patch), and the sources' 8-bit textures when every source has one.
+// build_patch), and the sources' 8-bit textures when every source has one.  A captured run takes neither:
+// its replays have to see images that hpm_set_view brings later, whatever their levels.
 int Ctx::take_whole_levels(int ref, const int32_t* srcs, float* weights, RunArgs& a) {
+    if (capturing()) return HPM_OK;
     if (views[ref].whole_levels == 1) {
         cudaError_t e = launch_weight_table(a.prm, weights, stream);
         if (e != cudaSuccess) return cuda_fail(e, "weight table");
@@ -409,6 +422,7 @@ int Ctx::launch_schedule(const RunArgs& a0, int n_half_sweeps) {
 bool Ctx::ensure_bands() {
     cudaError_t e = cudaSuccess;
     if (band_start) return true;
+    if (capturing()) return false;
     for (int b = 0; b < kBands && e == cudaSuccess; ++b) {
         if (b && !band_stream[b]) e = cudaStreamCreateWithFlags(&band_stream[b], cudaStreamNonBlocking);
         for (auto& parity : band_done)
