@@ -231,6 +231,12 @@ int Ctx::run_batch(int n, const int32_t* refs, const int32_t* src_off, const int
         }
     }
     cudaError_t e;
+    if ((size_t)n > d_bargs_cap || (size_t)3 * (n + 1) > d_btiles_cap) {
+        // captured launches hold the addresses of the tables that are about to move
+        if (!batch_graphs.empty() && (e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_fail(e, "batch graphs");
+        for (auto& g : batch_graphs) cudaGraphExecDestroy(g.exec);
+        batch_graphs.clear();
+    }
     if ((e = ensure_dev(b_planes, b_cap_planes, total)) != cudaSuccess ||
         (e = ensure_dev(b_costs, b_cap_costs, total)) != cudaSuccess ||
         (e = ensure_dev(b_pre, b_cap_pre, total)) != cudaSuccess ||

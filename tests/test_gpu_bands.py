@@ -70,3 +70,25 @@ def test_groups_equal_single_runs(heights):
     for a, b in zip(*out):
         for x, y in zip(a, b):
             assert _same(x, y)
+
+
+def test_graph_replay_after_a_larger_batch():
+    """A batch shape replayed after a batch that needed larger tables."""
+    from hpm_b200 import synth
+    scene = synth.make_scene(n_views=5, width=96, height=72, n_src=2, seed=24, supersample=1)
+    srcs = [[j for j, _ in p] for p in scene.pairs]
+    with hpm_b200.Context(0) as ctx:
+        ctx.set_batch_options(hpm_b200.BATCH_GRAPH)
+        cams = _load(ctx, scene)
+
+        def run(n):
+            params = [hpm_b200.Params.make(3, *hpm_b200.widened_range(cams[r]), mode=0) for r in range(n)]
+            ctx.run_batch(list(range(n)), srcs[:n], params, list(range(60, 60 + n)))
+            return _maps(ctx, range(n), hpm_b200.MAP_DEPTH)
+
+        first = run(2)
+        run(2)
+        run(5)
+        for a, b in zip(first, run(2)):
+            for x, y in zip(a, b):
+                assert _same(x, y)
