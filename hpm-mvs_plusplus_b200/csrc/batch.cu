@@ -7,7 +7,8 @@
 // (HPM.cu:2987-3035).  Here the runs' RunArgs go to device memory and each
 // stage is one launch whose blocks are the tiles of all views (pm_kernels.cu,
 // k_random_init_batch / k_half_sweep_batch), so the last wave of one view no
-// longer idles the GPU.  Per-run setup (hypothesis reload, packing) and the
+// longer idles the GPU; the half-sweeps go as two such launches, of half the
+// runs each, on two streams (launch_batch_sweeps).  Per-run setup (hypothesis reload, packing) and the
 // hand-off of the results are the single-run code paths of run.cu, applied to
 // per-run slices of resident batch buffers.
 //
