@@ -1136,7 +1136,8 @@ __device__ __forceinline__ void sweep_pixel(const RunArgs& a, float* smem_column
     }
 }
 
-// The views' geometry into shared memory, behind the threads' columns; every thread of the block calls it.
+// The views' geometry into shared memory, behind the threads' columns.  Every thread of the block calls it,
+// before any returns: the geometric modes (a prior run may be one) end it with a barrier.
 template <int NS, int BLK>
 __device__ __forceinline__ GeomView* load_geom_views(const RunArgs& a, float* smem, int tid) {
     GeomView* views = reinterpret_cast<GeomView*>(smem + Scratch<NS, BLK>::kWords * BLK);
@@ -1177,13 +1178,14 @@ __global__ void __launch_bounds__(BLK, kSweepBlocks) k_half_sweep_listed(const _
                                                                          int color, int iter, int first_pair,
                                                                          int last_pair) {
     extern __shared__ float smem[];
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    const GeomView* views = load_geom_views<NS, BLK>(a, smem, tid);
     const int pair = first_pair + blockIdx.y * blockDim.y + threadIdx.y;
     if (pair >= last_pair) return;
     const int k = color * a.cover_pairs + pair;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= a.active_n[k]) return;
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    sweep_pixel<NS, BLK, false, CNT>(a, smem + tid, nullptr, a.active_px[(size_t)k * a.W + x], pair, color, iter);
+    sweep_pixel<NS, BLK, false, CNT>(a, smem + tid, views, a.active_px[(size_t)k * a.W + x], pair, color, iter);
 }
 
 #ifndef HPM_NS
@@ -1230,12 +1232,14 @@ __global__ void __launch_bounds__(BLK, kSweepBlocks)
         const RunArgs& a = args[k];
         const int t = b - __ldg(tile_start + k);
         const int tx = (a.W + blockDim.x - 1) / blockDim.x;
+        if (a.prm.mode & HPM_MODE_GEOM) __syncthreads();  // the tile before may still read its views
+        const GeomView* views = load_geom_views<NS, BLK>(a, smem, tid);
         const int x = (t % tx) * blockDim.x + threadIdx.x;
         const int pair = (t / tx) * blockDim.y + threadIdx.y;
         if (pair >= a.cover_pairs) continue;
         const int r = color * a.cover_pairs + pair;
         if (x >= a.active_n[r]) continue;
-        sweep_pixel<NS, BLK, false, CNT>(a, smem + tid, nullptr, a.active_px[(size_t)r * a.W + x], pair, color, iter);
+        sweep_pixel<NS, BLK, false, CNT>(a, smem + tid, views, a.active_px[(size_t)r * a.W + x], pair, color, iter);
     }
 }
 
