@@ -237,7 +237,7 @@ int hpm_set_view(hpm_ctx* ctx, int view, const float* gray, int w, int h, const 
     if (e != cudaSuccess) return c->cuda_fail(e, "alloc grey image");
     e = cudaMemcpyAsync(v.gray, gray, sizeof(float) * w * h, cudaMemcpyHostToDevice, c->stream);
     if (e != cudaSuccess) return c->cuda_fail(e, "upload grey image");
-    v.whole_levels = -1;
+    c->new_image(view, -1);
     v.w = w; v.h = h; v.cam = *cam;
     v.cam.width = w; v.cam.height = h;
     return c->bind_texture(view);

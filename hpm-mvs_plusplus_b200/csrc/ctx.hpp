@@ -30,6 +30,7 @@ struct ViewState {
     float* gray = nullptr;
     size_t gray_cap = 0;
     int whole_levels = 0;  // the grey image holds whole levels 0..255 only (-1: not looked at yet)
+    bool captured = false;  // a stream capture holds an upload of this view: see Ctx::new_image
     cudaArray_t arr = nullptr;
     cudaTextureObject_t tex = 0;
     int arr_w = 0, arr_h = 0, arr_mode = -1, arr_fmt = -1;
@@ -172,6 +173,7 @@ struct Ctx {
     int bind_texture(int view);
     int bind_bytes(int view);
     bool capturing() const;
+    void new_image(int view, int whole_levels);
     int no_bytes(int view);
     int take_whole_levels(int ref, const int32_t* srcs, float* weights, RunArgs& a);
     int look_at_levels(int ref, const int32_t* srcs, int n_src);

@@ -187,7 +187,7 @@ int Ctx::prepare_level_image(int view, int w, int h, const hpm_camera& cam) {
     if (e != cudaSuccess) return cuda_fail(e, "alloc grey");
     k_gray<<<(int)((n + 255) / 256), 256, 0, stream>>>(v.color, (int)n, v.gray);
     ++launches;
-    v.whole_levels = 1;
+    new_image(view, 1);
     v.w = w;
     v.h = h;
     v.cam = cam;

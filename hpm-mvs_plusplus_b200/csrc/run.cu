@@ -55,6 +55,15 @@ bool Ctx::capturing() const {
     return cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
 }
 
+// A view's grey image has been replaced by one whose levels are whole (1) or not looked at (-1).  Once a
+// capture holds such an upload, a replay may bring another image at any time without a call that the host
+// sees, so the view stays on its float image (0), which every replay brings up to date.
+void Ctx::new_image(int view, int whole_levels) {
+    ViewState& v = views[view];
+    v.captured = v.captured || capturing();
+    v.whole_levels = v.captured ? 0 : whole_levels;
+}
+
 // Finds out which of a run's images hold whole levels 0..255 only, as every image made by
 // hpm_prepare_level does.  Images from hpm_set_view are looked at once, when a run first uses them.
 // Not under stream capture: a replay reads the images of its time.
