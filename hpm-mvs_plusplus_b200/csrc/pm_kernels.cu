@@ -41,6 +41,7 @@
 #include "pm_kernels.cuh"
 
 #include <float.h>
+#include <limits.h>
 
 namespace hpm {
 
@@ -93,6 +94,7 @@ constexpr int kWeightRows = 6;
 static_assert(kWeightRows * 256 == kWeightTable, "RunArgs::weights");
 
 constexpr int kSweepThreads = 128;
+constexpr int kEvalThreads = 128;
 constexpr int kSweepBlocks = 3;  // resident blocks per SM: at most 168 registers a thread
 
 // Statistics of a pixel's reference patch (the view-independent part of the NCC).
@@ -166,9 +168,12 @@ __global__ void k_weight_table(float two_ss, float two_sc, float* __restrict__ o
 
 // The patch in two ways with the same bits.  A reference of whole levels reads bytes and takes its
 // weights from the table: 36 loads of each, all in flight, instead of 36 exponentials and 72 divisions.
-// Any other forms the weights in a loop, through kPatchWords words of the thread's local memory.
+// Any other forms the weights: in a loop, through kPatchWords words of the thread's local memory, where
+// code size counts (half-sweeps), and UNROLLED elsewhere: the 36 chains side by side take 13 us less
+// (hpm_eval_costs of one pixel: 50 and 37 us a call, of 10,000: 88 and 74).
 constexpr int kPatchWords = 2 * kPatchSamples;
 
+template <bool UNROLLED>
 __device__ __forceinline__ void build_patch(const RunArgs& a, int px, int py, Patch& P, float* tmp) {
     const int W = a.W, H = a.H;
     const int at = clampi(py, 0, H - 1) * W + clampi(px, 0, W - 1);
@@ -196,17 +201,23 @@ __device__ __forceinline__ void build_patch(const RunArgs& a, int px, int py, Pa
         center = __ldg(a.ref_img + at);
         const float two_ss = 2.0f * a.prm.sigma_spatial * a.prm.sigma_spatial;
         const float two_sc = 2.0f * a.prm.sigma_color * a.prm.sigma_color;
-#pragma unroll 1
-        for (int k = 0; k < kPatchSamples; ++k) {
+        auto sample = [&](int k, float& texel, float& weight) {
             const int dx = -kPatchRadius + kPatchStep * (k / 6), dy = -kPatchRadius + kPatchStep * (k % 6);
             const float t = __ldg(a.ref_img + (size_t)clampi(py + dy, 0, H - 1) * W + clampi(px + dx, 0, W - 1));
-            tmp[k] = t;
-            tmp[kPatchSamples + k] = bilateral_weight(dx, dy, fabsf(t - center), two_ss, two_sc);
-        }
+            texel = t;
+            weight = bilateral_weight(dx, dy, fabsf(t - center), two_ss, two_sc);
+        };
+        if (UNROLLED) {
 #pragma unroll
-        for (int k = 0; k < kPatchSamples; ++k) {
-            r[k] = tmp[k];
-            w[k] = tmp[kPatchSamples + k];
+            for (int k = 0; k < kPatchSamples; ++k) sample(k, r[k], w[k]);
+        } else {
+#pragma unroll 1
+            for (int k = 0; k < kPatchSamples; ++k) sample(k, tmp[k], tmp[kPatchSamples + k]);
+#pragma unroll
+            for (int k = 0; k < kPatchSamples; ++k) {
+                r[k] = tmp[k];
+                w[k] = tmp[kPatchSamples + k];
+            }
         }
     }
     // shifted moments (precision form): the patch relative to its centre texel; shift 0 is the plain arithmetic
@@ -477,9 +488,8 @@ __device__ __forceinline__ void init_pixel(const RunArgs& a, const InitScratch<N
     a.rng[center] = rng.draw;
     if (!cost) return;
 
-    float tmp[kPatchWords];
     Patch P;
-    build_patch(a, px, py, P, tmp);
+    build_patch<true>(a, px, py, P, nullptr);
     uint32_t sel = 0;
     // upsample mode costs the pre-cost plane first: zero normal, upsampled depth as offset (HPM.cu:689,
     // HPM.cpp:894-901)
@@ -798,7 +808,7 @@ __device__ __forceinline__ void sweep_pixel(const RunArgs& a, float* smem_column
     float4 cand[8];
     const Scratch<NS, BLK> s{ smem_column, rows, cand, views };
     Patch P;
-    build_patch(a, px, py, P, rows);
+    build_patch<false>(a, px, py, P, rows);
     const uint32_t all_views = (S >= 32) ? 0xffffffffu : ((1u << S) - 1u);
 
     const uint32_t flags = direction_search(a, px, py, s);
@@ -1273,17 +1283,19 @@ __global__ void k_export(const __grid_constant__ RunArgs a) {
     a.planes[center] = rotate_to_world(a.cams[0], pl);
 }
 
-__global__ void k_eval_costs(const __grid_constant__ RunArgs a, int n, const int32_t* __restrict__ px,
-                             const float4* __restrict__ planes, float* __restrict__ out) {
+// Thread x of grid row y costs pixel x against the views y, y + gridDim.y, ...  Three blocks to an SM: at
+// the 183 registers of two, 100,000 pixels x 10 views took 614 us a call, with three 577.
+__global__ void __launch_bounds__(kEvalThreads, kSweepBlocks)
+    k_eval_costs(const __grid_constant__ RunArgs a, int n, const int32_t* __restrict__ px,
+                 const float4* __restrict__ planes, float* __restrict__ out) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int x = px[2 * k], y = px[2 * k + 1];
     Patch P;
-    float tmp[kPatchWords];
-    build_patch(a, x, y, P, tmp);
+    build_patch<true>(a, x, y, P, nullptr);
     const float4 pl = planes[k];
     const PlaneM pm = plane_m(a, pl);
-    for (int j = 0; j < a.S; ++j) out[(size_t)k * a.S + j] = ncc_view<false>(a, P, x, y, pm, j);
+    for (int j = blockIdx.y; j < a.S; j += gridDim.y) out[(size_t)k * a.S + j] = ncc_view<false>(a, P, x, y, pm, j);
 }
 #endif
 
@@ -1447,7 +1459,12 @@ cudaError_t launch_export(const RunArgs& a, cudaStream_t st) {
 cudaError_t launch_eval_costs(const RunArgs& a, int n, const int32_t* px, const float4* planes, float* out,
                               cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    k_eval_costs<<<(n + 127) / 128, 128, 0, st>>>(a, n, px, planes, out);
+    // A thread per pixel and view while they are resident together: one after the other, 31 views of one
+    // pixel took 78 us a call and take 41, of 64 pixels 92 and 54.  Past that a thread goes through its
+    // pixel's views, which share the patch (100,000 pixels x 31 views: 1200 us).
+    const int blocks = (n + kEvalThreads - 1) / kEvalThreads;
+    const bool apart = one_wave(blocks <= INT_MAX / HPM_MAX_SRC ? blocks * a.S : blocks);
+    k_eval_costs<<<dim3(blocks, apart ? a.S : 1), kEvalThreads, 0, st>>>(a, n, px, planes, out);
     return cudaGetLastError();
 }
 
