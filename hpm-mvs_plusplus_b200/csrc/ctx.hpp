@@ -34,9 +34,11 @@ struct ViewState {
     cudaArray_t arr = nullptr;
     cudaTextureObject_t tex = 0;
     int arr_w = 0, arr_h = 0, arr_mode = -1, arr_fmt = -1;
-    uint8_t* bytes = nullptr;  // an image of whole levels as bytes (whole_levels == 1)
+    uint8_t* bytes = nullptr;  // an image of whole levels as bytes (Ctx::bring_bytes)
     size_t bytes_cap = 0;
-    // 8-bit texture of an F32 image of whole levels, which the half-sweeps sample (Ctx::bind_bytes)
+    bool bytes_current = false;  // they are those of the current image
+    int64_t bytes_credit = 0;    // work of its runs as the reference since the image came
+    // 8-bit texture of an F32 image of whole levels, which the half-sweeps sample
     cudaArray_t arr8 = nullptr;
     cudaTextureObject_t tex8 = 0;
     int arr8_w = 0, arr8_h = 0, arr8_mode = -1;
@@ -90,7 +92,7 @@ struct Ctx {
     int addr_mode = 0;
     int tex_format = 0;  // HPM_TEX_F32, HPM_TEX_F16 or HPM_TEX_U8: texel type of the source-image textures
     int ncc_mode = 0;    // HPM_NCC_PLAIN or HPM_NCC_SHIFTED
-    int* level_flags = nullptr; size_t level_flags_cap = 0;  // per view, results of k_whole_levels
+    int* level_flags = nullptr; size_t level_flags_cap = 0;  // per view, results of k_bytes
     uint16_t* half_stage = nullptr; size_t half_stage_cap = 0;
     int64_t launches = 0;
 
@@ -176,7 +178,7 @@ struct Ctx {
     void new_image(int view, int whole_levels);
     int no_bytes(int view);
     int take_whole_levels(int ref, const int32_t* srcs, float* weights, RunArgs& a);
-    int look_at_levels(int ref, const int32_t* srcs, int n_src);
+    int bring_bytes(int ref, const int32_t* srcs, int n_src, int n_half_sweeps);
     int fill_run_args(int ref, const int32_t* srcs, int n_src, const hpm_params* params, RunArgs& a);
     int prepare_run(int ref, const int32_t* srcs, int n_src, const hpm_params* params, int texture_level,
                     uint64_t seed, RunArgs& a);

@@ -43,10 +43,23 @@ __global__ void k_to_u8(const float* __restrict__ src, int n, uint8_t* __restric
     if (i < n) dst[i] = (uint8_t)fminf(255.0f, fmaxf(0.0f, rintf(src[i])));
 }
 
-__global__ void k_whole_levels(const float* __restrict__ gray, int n, int* __restrict__ whole) {
+// Images for Ctx::bring_bytes, one to a grid row.
+struct ByteCopies {
+    const float* gray[HPM_MAX_SRC + 1];
+    uint8_t* bytes[HPM_MAX_SRC + 1];
+    int* whole[HPM_MAX_SRC + 1];  // cleared where a level is not a whole number 0..255; null: known to be
+    int n[HPM_MAX_SRC + 1];
+};
+
+__global__ void k_bytes(const __grid_constant__ ByteCopies c) {
+    const float* __restrict__ gray = c.gray[blockIdx.y];
+    uint8_t* __restrict__ bytes = c.bytes[blockIdx.y];
+    int* whole = c.whole[blockIdx.y];
+    const int n = c.n[blockIdx.y];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float v = gray[i];
-        if (!(v >= 0.0f && v <= 255.0f && v == rintf(v))) *whole = 0;
+        if (whole && !(v >= 0.0f && v <= 255.0f && v == rintf(v))) *whole = 0;
+        bytes[i] = (uint8_t)fminf(255.0f, fmaxf(0.0f, rintf(v)));
     }
 }
 
@@ -62,43 +75,8 @@ void Ctx::new_image(int view, int whole_levels) {
     ViewState& v = views[view];
     v.captured = v.captured || capturing();
     v.whole_levels = v.captured ? 0 : whole_levels;
-}
-
-// Finds out which of a run's images hold whole levels 0..255 only, as every image made by
-// hpm_prepare_level does.  Images from hpm_set_view are looked at once, when a run first uses them.
-// Not under stream capture: a replay reads the images of its time.
-int Ctx::look_at_levels(int ref, const int32_t* srcs, int n_src) {
-    bool unknown = views[ref].whole_levels < 0;
-    for (int j = 0; j < n_src; ++j) unknown = unknown || views[srcs[j]].whole_levels < 0;
-    if (!unknown) return HPM_OK;
-    if (capturing()) return HPM_OK;
-    cudaError_t e;
-    if ((e = ensure_buf(level_flags, level_flags_cap, HPM_MAX_VIEWS)) != cudaSuccess) return cuda_fail(e, "alloc level flags");
-    int flags[HPM_MAX_VIEWS];
-    e = cudaMemsetAsync(level_flags, 0xff, sizeof(flags), stream);
-    if (e != cudaSuccess) return cuda_fail(e, "grey levels");
-    for (int j = -1; j < n_src; ++j) {
-        const int view = j < 0 ? ref : srcs[j];
-        const ViewState& v = views[view];
-        if (v.whole_levels >= 0) continue;
-        const int n = v.w * v.h;
-        k_whole_levels<<<std::min((n + 255) / 256, 1184), 256, 0, stream>>>(v.gray, n, level_flags + view);
-        ++launches;
-    }
-    e = cudaMemcpyAsync(flags, level_flags, sizeof(flags), cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) return cuda_fail(e, "grey levels");
-    for (int j = -1; j < n_src; ++j) {
-        const int view = j < 0 ? ref : srcs[j];
-        ViewState& v = views[view];
-        if (v.whole_levels >= 0) continue;
-        v.whole_levels = flags[view] ? 1 : 0;
-        if (v.whole_levels == 1) {
-            const int rc = bind_bytes(view);
-            if (rc) return rc;
-        }
-    }
-    return HPM_OK;
+    v.bytes_current = v.bytes_bound = false;
+    v.bytes_credit = 0;
 }
 
 static cudaError_t make_texture(cudaArray_t arr, int addr_mode, cudaTextureReadMode read, cudaTextureObject_t* tex) {
@@ -115,28 +93,91 @@ static cudaError_t make_texture(cudaArray_t arr, int addr_mode, cudaTextureReadM
     return cudaCreateTextureObject(tex, &rd, &td, nullptr);
 }
 
-// Where there is no memory for the copy below, the view stays on its float image.
-int Ctx::no_bytes(int view) {
-    cudaGetLastError();
-    views[view].whole_levels = 0;
-    views[view].bytes_bound = false;
-    return HPM_OK;
-}
-
-// 8-bit copy of a view's image of whole levels.  The unit filters with weights of 1/256, so an F32
+// 8-bit copies of a run's images of whole levels 0..255, as every image made by hpm_prepare_level is:
+// bytes of the reference, and 8-bit textures of the sources that have float ones.  Images from hpm_set_view
+// are looked at once for it, for which the host waits.  The unit filters with weights of 1/256, so an F32
 // fetch is a whole multiple N of 1/256 level, N <= 255 * 256, and an 8-bit fetch is N / 65280 rounded
 // to a multiple of 1/65535: fetch * 65280 lies within 0.4999 of N, and rounding it to the nearest
 // integer gives N, hence the F32 fetch times 256, for every N (tests/test_gpu_whole_levels.py).  A
 // quarter of the bytes puts neighbouring samples of a warp on fewer lines.
+//
+// Not under stream capture: a replay reads the images of its time.  Not before the reference's runs have
+// work for it either: the copies take COPY_FIGURES, and save a half-sweep some 13 us of its latency and
+// 0.8 ns a pixel, the initialisation a quarter of that.  Until then its runs stay on the float images.
+int Ctx::bring_bytes(int ref, const int32_t* srcs, int n_src, int n_half_sweeps) {
+    if (capturing()) return HPM_OK;
+    int todo[HPM_MAX_SRC + 1], n_todo = 0, n_copies = 0, max_px = 0;
+    for (int j = -1; j < n_src; ++j) {
+        const int view = j < 0 ? ref : srcs[j];
+        const ViewState& v = views[view];
+        if (v.whole_levels == 0 || (j >= 0 && v.arr_fmt != HPM_TEX_F32)) continue;
+        if (v.bytes_current && (j < 0 || v.bytes_bound)) continue;
+        if (std::find(todo, todo + n_todo, view) == todo + n_todo) todo[n_todo++] = view;
+    }
+    if (!n_todo) return HPM_OK;
+    ViewState& rv = views[ref];
+    const int64_t px = (int64_t)rv.w * rv.h;
+    rv.bytes_credit += n_half_sweeps * (16384 + px) + px / 4;
+    if (rv.bytes_credit <= 32768 + 8192 * (int64_t)n_todo) return HPM_OK;
+
+    ByteCopies c;
+    bool unknown = false;
+    cudaError_t e = ensure_buf(level_flags, level_flags_cap, HPM_MAX_VIEWS);
+    if (e != cudaSuccess) return cuda_fail(e, "alloc level flags");
+    for (int k = 0; k < n_todo; ++k) {
+        ViewState& v = views[todo[k]];
+        if (v.bytes_current) continue;
+        if (ensure_buf(v.bytes, v.bytes_cap, (size_t)v.w * v.h) != cudaSuccess) {
+            no_bytes(todo[k]);
+            continue;
+        }
+        c.gray[n_copies] = v.gray;
+        c.bytes[n_copies] = v.bytes;
+        c.n[n_copies] = v.w * v.h;
+        c.whole[n_copies] = v.whole_levels < 0 ? level_flags + todo[k] : nullptr;
+        unknown = unknown || v.whole_levels < 0;
+        max_px = std::max(max_px, c.n[n_copies++]);
+    }
+    int flags[HPM_MAX_VIEWS];
+    if (unknown && (e = cudaMemsetAsync(level_flags, 0xff, sizeof(flags), stream)) != cudaSuccess)
+        return cuda_fail(e, "grey levels");
+    if (n_copies) {
+        k_bytes<<<dim3(std::min((max_px + 255) / 256, 1184), n_copies), 256, 0, stream>>>(c);
+        ++launches;
+    }
+    if (unknown) {
+        e = cudaMemcpyAsync(flags, level_flags, sizeof(flags), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) return cuda_fail(e, "grey levels");
+    }
+    for (int k = 0; k < n_todo; ++k) {
+        ViewState& v = views[todo[k]];
+        if (v.whole_levels < 0) v.whole_levels = flags[todo[k]] ? 1 : 0;
+        v.bytes_current = v.whole_levels == 1;
+    }
+    for (int j = 0; j < n_src; ++j) {
+        const ViewState& v = views[srcs[j]];
+        if (!v.bytes_current || v.bytes_bound || v.arr_fmt != HPM_TEX_F32) continue;
+        const int rc = bind_bytes(srcs[j]);
+        if (rc) return rc;
+    }
+    return HPM_OK;
+}
+
+// Where there is no memory for a copy, the view stays on its float image.
+int Ctx::no_bytes(int view) {
+    cudaGetLastError();
+    ViewState& v = views[view];
+    v.whole_levels = 0;
+    v.bytes_current = v.bytes_bound = false;
+    return HPM_OK;
+}
+
+// The 8-bit texture of a view whose bytes are current.
 int Ctx::bind_bytes(int view) {
     ViewState& v = views[view];
-    const size_t n = (size_t)v.w * v.h;
-    cudaError_t e = ensure_buf(v.bytes, v.bytes_cap, n);
-    if (e != cudaSuccess) return no_bytes(view);
-    k_to_u8<<<(int)((n + 255) / 256), 256, 0, stream>>>(v.gray, (int)n, v.bytes);
-    ++launches;
-    if (v.arr_fmt != HPM_TEX_F32) return HPM_OK;
-    if (!v.arr8 || v.arr8_w != v.w || v.arr8_h != v.h || v.arr8_mode != v.arr_mode) {
+    cudaError_t e;
+    if (!v.arr8 || !v.tex8 || v.arr8_w != v.w || v.arr8_h != v.h || v.arr8_mode != v.arr_mode) {
         if (v.tex8) { cudaDestroyTextureObject(v.tex8); v.tex8 = 0; }
         if (v.arr8 && (v.arr8_w != v.w || v.arr8_h != v.h)) {
             cudaFreeArray(v.arr8);
@@ -206,8 +247,7 @@ int Ctx::bind_texture(int view) {
                                      cudaMemcpyDeviceToDevice, stream);
     }
     if (e != cudaSuccess) return cuda_fail(e, "copy image to array");
-    v.bytes_bound = false;
-    return v.whole_levels == 1 ? bind_bytes(view) : HPM_OK;
+    return HPM_OK;
 }
 
 int Ctx::fill_run_args(int ref, const int32_t* srcs, int n_src, const hpm_params* params, RunArgs& a) {
@@ -351,7 +391,7 @@ int Ctx::prepare_run_into(int ref, const int32_t* srcs, int n_src, const hpm_par
     } else {
         a.prm.mode &= ~HPM_MODE_UPSAMPLE;
     }
-    if ((rc = look_at_levels(ref, srcs, n_src))) return rc;
+    if ((rc = bring_bytes(ref, srcs, n_src, 2 * std::max(0, params->max_iterations)))) return rc;
     const bool want_texture = !prior && !mand;
     if (want_texture) {
         e = ensure_map(ref, HPM_MAP_TEXTURE0 + texture_level, W, H);
@@ -367,7 +407,7 @@ int Ctx::prepare_run_into(int ref, const int32_t* srcs, int n_src, const hpm_par
 // its replays have to see images that hpm_set_view brings later, whatever their levels.
 int Ctx::take_whole_levels(int ref, const int32_t* srcs, float* weights, RunArgs& a) {
     if (capturing()) return HPM_OK;
-    if (views[ref].whole_levels == 1) {
+    if (views[ref].bytes_current) {
         cudaError_t e = launch_weight_table(a.prm, weights, stream);
         if (e != cudaSuccess) return cuda_fail(e, "weight table");
         ++launches;
