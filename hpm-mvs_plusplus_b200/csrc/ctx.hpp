@@ -37,7 +37,7 @@ struct ViewState {
     uint8_t* bytes = nullptr;  // an image of whole levels as bytes (Ctx::bring_bytes)
     size_t bytes_cap = 0;
     bool bytes_current = false;  // they are those of the current image
-    int64_t bytes_credit = 0;    // work of its runs as the reference since the image came
+    int64_t bytes_credit = 0;    // what its runs as the reference would have saved since the image came
     // 8-bit texture of an F32 image of whole levels, which the half-sweeps sample
     cudaArray_t arr8 = nullptr;
     cudaTextureObject_t tex8 = 0;

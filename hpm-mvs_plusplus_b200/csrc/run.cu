@@ -102,8 +102,11 @@ static cudaError_t make_texture(cudaArray_t arr, int addr_mode, cudaTextureReadM
 // quarter of the bytes puts neighbouring samples of a warp on fewer lines.
 //
 // Not under stream capture: a replay reads the images of its time.  Not before the reference's runs have
-// work for it either: the copies take COPY_FIGURES, and save a half-sweep some 13 us of its latency and
-// 0.8 ns a pixel, the initialisation a quarter of that.  Until then its runs stay on the float images.
+// work for it either.  With S sources on B200, the copies take about 20 + 5.5 (S + 1) us and save a half-sweep
+// 9 + 1.6 S us of its latency and (2 + S) / 16 ns a pixel, the initialisation 0.2 ns a pixel (0.125 here: an
+// image with other levels gains nothing).  Runs on new images, float and bytes: 64x48, S = 2, one iteration
+// 263 and 267 us, three 559 and 519; 160x120, S = 10, one iteration 762 and 715; 640x480, S = 10, none 1223
+// and 1236, three 9.5 and 7.5 ms.
 int Ctx::bring_bytes(int ref, const int32_t* srcs, int n_src, int n_half_sweeps) {
     if (capturing()) return HPM_OK;
     int todo[HPM_MAX_SRC + 1], n_todo = 0, n_copies = 0, max_px = 0;
@@ -117,8 +120,8 @@ int Ctx::bring_bytes(int ref, const int32_t* srcs, int n_src, int n_half_sweeps)
     if (!n_todo) return HPM_OK;
     ViewState& rv = views[ref];
     const int64_t px = (int64_t)rv.w * rv.h;
-    rv.bytes_credit += n_half_sweeps * (16384 + px) + px / 4;
-    if (rv.bytes_credit <= 32768 + 8192 * (int64_t)n_todo) return HPM_OK;
+    rv.bytes_credit += n_half_sweeps * (9000 + 1600 * n_src + px * (2 + n_src) / 16) + px / 8;  // in ns
+    if (rv.bytes_credit <= 20000 + 5500 * n_todo) return HPM_OK;
 
     ByteCopies c;
     bool unknown = false;
