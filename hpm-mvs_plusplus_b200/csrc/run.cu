@@ -318,6 +318,8 @@ int Ctx::prepare_run_into(int ref, const int32_t* srcs, int n_src, const hpm_par
     const bool geom = mode & HPM_MODE_GEOM, prior = mode & HPM_MODE_PRIOR, hier = mode & HPM_MODE_HIERARCHY;
     const bool mand = mode & HPM_MODE_MAND, multi = mode & HPM_MODE_MULTIGEOM;
     if (mand && !geom) return fail(HPM_E_INVALID, "mandatory consistency requires the geometric mode");
+    if (hier && geom && !prior)  // each would start the pixels from its own maps
+        return fail(HPM_E_INVALID, "the hierarchy mode and the geometric mode exclude each other");
     if (!rv.canny || rv.canny_w != W || rv.canny_h != H) return fail(HPM_E_STATE, "view %d has no Canny map of its size", ref);
     cudaError_t e;
     float4* const planes = b.planes;
