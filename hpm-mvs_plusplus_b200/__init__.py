@@ -39,7 +39,7 @@ MAP_TEXTURE0 = 8
 EXPORTED_SYMBOLS = (
     "hpm_create", "hpm_destroy", "hpm_last_error", "hpm_set_view", "hpm_set_map", "hpm_get_map",
     "hpm_set_canny", "hpm_set_prior", "hpm_run_patchmatch", "hpm_eval_costs", "hpm_set_address_mode",
-    "hpm_launch_count", "hpm_synchronize", "hpm_sample_view", "hpm_debug_run_partial", "hpm_set_color",
+    "hpm_launch_count", "hpm_synchronize", "hpm_sample_view", "hpm_debug_run_partial", "hpm_debug_scan_rounds", "hpm_set_color",
     "hpm_jbu", "hpm_jbu_maps", "hpm_confidence_eval", "hpm_fuse", "hpm_support_points", "hpm_delaunay",
     "hpm_prior_from_triangles", "hpm_build_prior", "hpm_get_prior", "hpm_set_image", "hpm_prepare_level",
     "hpm_get_level", "hpm_reconstruct", "hpm_get_points", "hpm_get_stream", "hpm_profile_enable",
@@ -238,6 +238,7 @@ def load_library(path: str = LIB_PATH) -> ctypes.CDLL:
     lib.hpm_confidence_eval.argtypes = [vp, ctypes.c_int, vp, vp, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]
     lib.hpm_fuse.argtypes = [vp, ctypes.c_int, vp, vp, ctypes.c_int, vp, vp, ctypes.c_int64,
                              ctypes.POINTER(ctypes.c_int64)]
+    lib.hpm_debug_scan_rounds.argtypes = [vp, ctypes.c_int]
     lib.hpm_debug_run_partial.argtypes = [vp, ctypes.c_int, vp, ctypes.c_int, ctypes.POINTER(Params), ctypes.c_int,
                                           ctypes.c_uint64, ctypes.c_int, vp, vp, vp, vp]
     lib.hpm_get_stream.argtypes = [vp, ctypes.POINTER(ctypes.c_void_p)]
@@ -452,6 +453,10 @@ class Context:
                                                    ctypes.c_uint64(seed), n_half_sweeps, _ptr(planes), _ptr(costs),
                                                    _ptr(sel), _ptr(draws)), "hpm_debug_run_partial")
         return {"planes": planes, "costs": costs, "selected_views": sel, "rng_draw": draws}
+
+    def debug_scan_rounds(self, rounds: int) -> None:
+        """Rounds a consistency scan spends on a view before its sequential pass (0..256, default 256)."""
+        self._check(self.lib.hpm_debug_scan_rounds(self.h, rounds), "hpm_debug_scan_rounds")
 
     def set_color(self, view: int, bgr: np.ndarray) -> None:
         c = np.ascontiguousarray(bgr, dtype=np.uint8)

@@ -544,6 +544,15 @@ int hpm_sample_view(hpm_ctx* ctx, int view, int n, const float* xy, float* out) 
     return reinterpret_cast<Ctx*>(ctx)->sample_view(view, n, xy, out);
 }
 
+int hpm_debug_scan_rounds(hpm_ctx* ctx, int rounds) {
+    if (!ctx) return HPM_E_INVALID;
+    Ctx* c = reinterpret_cast<Ctx*>(ctx);
+    if (rounds < 0 || rounds > kMaxScanIterations)
+        return c->fail(HPM_E_INVALID, "scan rounds must be 0..%d", kMaxScanIterations);
+    c->scan_rounds = rounds;
+    return HPM_OK;
+}
+
 int hpm_debug_run_partial(hpm_ctx* ctx, int ref, const int32_t* srcs, int n_src, const hpm_params* params,
                           int texture_level, uint64_t seed, int n_half_sweeps, float* planes, float* costs,
                           uint32_t* selected_views, uint32_t* draws) {

@@ -13,6 +13,7 @@
 namespace hpm {
 
 constexpr int kNumMaps = 16;
+constexpr int kMaxScanIterations = 256;  // rounds of a consistency scan before the sequential pass
 
 // Kinds of the profiling events (hpm_profile): PatchMatch launches and the other stages of hpm_reconstruct.
 enum { HPM_STAGE_INIT = 0, HPM_STAGE_SWEEP = 1, HPM_STAGE_CONFIDENCE = 2, HPM_STAGE_PRIOR = 3, HPM_STAGE_JBU = 4,
@@ -125,6 +126,7 @@ struct Ctx {
     short2* canny_grad = nullptr; size_t canny_grad_cap = 0;
     uint8_t* canny_state = nullptr; size_t canny_state_cap = 0;
     int64_t n_points = 0;
+    int scan_rounds = kMaxScanIterations;  // hpm_debug_scan_rounds
 
     // batching form (hpm_run_batch): per-run slices of these buffers, the runs'
     // RunArgs and tile prefix sums in device memory, and the tuned shapes

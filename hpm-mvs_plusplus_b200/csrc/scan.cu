@@ -50,7 +50,6 @@
 namespace hpm {
 
 constexpr int kScanBlock = 1024;  // pixels of a chunk: one word of summary bits
-constexpr int kMaxScanIterations = 256;
 constexpr uint32_t kAccepted = 1u << 31;  // in a pixel's word beside the eff bits of at most 31 sources
 
 // One source of the view being scanned.  slot: the mark buffers it uses (a source listed twice shares them).
@@ -427,7 +426,7 @@ __global__ void __launch_bounds__(256) k_conf_own(const __grid_constant__ ScanRu
 }
 
 // Exact sequential pass (the reference loop) over the precomputed candidates;
-// used when the fixed point has not settled within kMaxScanIterations.
+// used when the fixed point has not settled within Ctx::scan_rounds.
 __global__ void k_sequential(const __grid_constant__ ScanRun a, uint32_t round) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     int used[31];
@@ -690,8 +689,8 @@ int Ctx::consistency_scan(int mode, int n_views, const int32_t* src_off, const i
         if (e != cudaSuccess) return cuda_fail(e, "clear change flags");
         int launched = 0, it = 0;
         bool converged = a.n == 0;
-        while (!converged && launched < kMaxScanIterations) {
-            const int until = std::min(kMaxScanIterations, launched + expected);
+        while (!converged && launched < scan_rounds) {
+            const int until = std::min(scan_rounds, launched + expected);
             const int from = launched;
             for (; launched < until; ++launched) {
                 const int* before = launched ? d_changed + launched - 1 : nullptr;
@@ -720,7 +719,7 @@ int Ctx::consistency_scan(int mode, int n_views, const int32_t* src_off, const i
         } else {
             expected = std::min(16, std::max(2, it));
         }
-        max_iter = std::max(max_iter, converged ? it : kMaxScanIterations + 1);
+        max_iter = std::max(max_iter, converged ? it : scan_rounds + 1);
         if (a.n > 0) {
             if (mode == 0) {
                 k_settle<0><<<blocks, 256, 0, stream>>>(a, (uint32_t)i + 1);

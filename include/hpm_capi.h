@@ -281,6 +281,11 @@ int hpm_debug_run_partial(hpm_ctx *ctx, int ref, const int32_t *srcs, int n_src,
                           int texture_level, uint64_t seed, int n_half_sweeps, float *planes, float *costs,
                           uint32_t *selected_views, uint32_t *draws);
 
+/* Diagnostic: rounds (0..256, default 256) that hpm_confidence_eval and hpm_fuse spend on a view before
+ * they walk its pixels one after the other.  No reference counterpart: the results do not depend on it,
+ * and low values let the tests reach that walk. */
+int hpm_debug_scan_rounds(hpm_ctx *ctx, int rounds);
+
 /* Texture address mode of the source images: 0 = clamp (default), 1 = wrap
  * (what HPM.cpp:760-761 requests with unnormalised coordinates). */
 int hpm_set_address_mode(hpm_ctx *ctx, int mode);
