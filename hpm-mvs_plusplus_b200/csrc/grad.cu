@@ -78,7 +78,8 @@ struct Lane {
     int view;
     int base;   // first lane of the pixel
     int per_warp;
-    __device__ __forceinline__ explicit Lane(int S) {
+    int views;  // S
+    __device__ __forceinline__ explicit Lane(int S) : views(S) {
         const int lane = threadIdx.x & 31;
         per_warp = 32 / S;
         pixel = lane / S;
@@ -101,34 +102,39 @@ struct View {
 };
 static_assert(sizeof(View) == 72, "View stride");
 
-static size_t grad_smem(int S) {
-    return sizeof(View) * S + sizeof(float) * kPatchStride * (32 / S) * (kGradThreads / 32);
+static size_t grad_smem(int S, bool own) {
+    return sizeof(View) * S + (own ? 0 : sizeof(float) * kPatchStride * (32 / S) * (kGradThreads / 32));
 }
 
-// The block's views into shared memory; the patches follow them.
-__device__ __forceinline__ float* load_views(const RunArgs& a, const SrcImages& si, View* views) {
-    for (int j = threadIdx.x; j < a.S; j += blockDim.x) {
+// The block's views, n from the first, into shared memory; the patches follow them.
+__device__ __forceinline__ float* load_views(const RunArgs& a, const SrcImages& si, View* views, int first, int n) {
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        const int j = first + k + 1;
         View v{};
-        for (int k = 0; k < 9; ++k) v.A[k] = a.basis[j + 1].A[k];
-        for (int k = 0; k < 3; ++k) v.b[k] = a.basis[j + 1].b[k];
-        v.img = si.img[j + 1];
-        v.w = si.w[j + 1];
-        v.h = si.h[j + 1];
-        views[j] = v;
+        for (int q = 0; q < 9; ++q) v.A[q] = a.basis[j].A[q];
+        for (int q = 0; q < 3; ++q) v.b[q] = a.basis[j].b[q];
+        v.img = si.img[j];
+        v.w = si.w[j];
+        v.h = si.h[j];
+        views[k] = v;
     }
     __syncthreads();
-    return reinterpret_cast<float*>(views + a.S);
+    return reinterpret_cast<float*>(views + n);
+}
+
+// Where the lanes of a pixel keep its patch.
+__device__ __forceinline__ float* patch_of(const Lane& L, float* smem) {
+    return smem + ((threadIdx.x >> 5) * L.per_warp + (L.pixel < L.per_warp ? L.pixel : 0)) * kPatchStride;
 }
 
 struct RefPatch {
-    const float* w;  // shared memory
+    const float* w;  // shared memory, or local where every lane has a pixel of its own
     const float* r;
     float W, mean, var;
 };
 
 // The reference patch of a pixel, made by its lanes together.  Every lane of the warp calls it.
-__device__ __forceinline__ RefPatch ref_patch(const RunArgs& a, int px, int py, bool on, const Lane& L, float* smem) {
-    float* w = smem + ((threadIdx.x >> 5) * L.per_warp + (L.pixel < L.per_warp ? L.pixel : 0)) * kPatchStride;
+__device__ __forceinline__ RefPatch ref_patch(const RunArgs& a, int px, int py, bool on, const Lane& L, float* w) {
     float* r = w + 36;
     if (on) {
         auto texel = [&](int x, int y) {
@@ -139,7 +145,7 @@ __device__ __forceinline__ RefPatch ref_patch(const RunArgs& a, int px, int py, 
         const float center = texel(px, py);
         const float two_ss = 2.0f * a.prm.sigma_spatial * a.prm.sigma_spatial;
         const float two_sc = 2.0f * a.prm.sigma_color * a.prm.sigma_color;
-        for (int k = L.view; k < 36; k += a.S) {
+        for (int k = L.view; k < 36; k += L.views) {
             const int dx = -5 + 2 * (k / 6), dy = -5 + 2 * (k % 6);
             const float t = texel(px + dx, py + dy);
             r[k] = t;
@@ -257,14 +263,19 @@ __device__ __forceinline__ float cost_grad_view(const RunArgs& a, const View& vi
     return c;
 }
 
+// Grid row y takes the views from y * per on, `per` of them (fewer in the last row).  OWN: one view, every
+// lane a pixel of its own, whose patch is in local memory.  32 patches a warp in shared memory left 30 KB of
+// an SM's L1 to the images: 1,000,000 pixels took 1773 us a call and take 961, 100,000 284 and 172.
+template <bool OWN>
 __global__ void __launch_bounds__(kGradThreads) k_cost_grad(const __grid_constant__ RunArgs a,
-                                                            const __grid_constant__ SrcImages si, int n,
+                                                            const __grid_constant__ SrcImages si, int per, int n,
                                                             const int32_t* __restrict__ px,
                                                             const float* __restrict__ theta, float* __restrict__ cost,
                                                             float* __restrict__ grad) {
     extern __shared__ View views[];
-    float* smem = load_views(a, si, views);
-    const Lane L(a.S);
+    const int first = blockIdx.y * per, count = min(per, a.S - first);
+    float* smem = load_views(a, si, views, first, count);
+    const Lane L(per);
     const int k = (blockIdx.x * (kGradThreads / 32) + (threadIdx.x >> 5)) * L.per_warp + L.pixel;
     bool on = L.pixel < L.per_warp && k < n;
     int x = 0, y = 0;
@@ -272,14 +283,15 @@ __global__ void __launch_bounds__(kGradThreads) k_cost_grad(const __grid_constan
         x = px[2 * k];
         y = px[2 * k + 1];
         if (x < 0 || x >= a.W || y < 0 || y >= a.H) {
-            if (L.view == 0) atomicAdd(&g_grad_oob, 1u);
+            if (first + L.view == 0) atomicAdd(&g_grad_oob, 1u);
             on = false;
         }
     }
-    const RefPatch P = ref_patch(a, x, y, on, L, smem);
-    if (!on) return;
+    float own[OWN ? 72 : 1];
+    const RefPatch P = ref_patch(a, x, y, on, L, OWN ? own : patch_of(L, smem));
+    if (!on || L.view >= count) return;
     const float th[3] = { theta[3 * k], theta[3 * k + 1], theta[3 * k + 2] };
-    const size_t at = (size_t)k * a.S + L.view;
+    const size_t at = (size_t)k * a.S + first + L.view;
     float g[3];
     cost[at] = cost_grad_view(a, views[L.view], P, x, y, th, grad != nullptr, g);
     if (grad)
@@ -311,7 +323,7 @@ __global__ void __launch_bounds__(kGradThreads) k_gn_refine(const __grid_constan
                                                             float* __restrict__ depth, float* __restrict__ normal,
                                                             float* __restrict__ cost_out, size_t n_px) {
     extern __shared__ View views[];
-    float* smem = load_views(a, si, views);
+    float* smem = load_views(a, si, views, 0, a.S);
     const Lane L(a.S);
     const size_t i = ((size_t)blockIdx.x * (kGradThreads / 32) + (threadIdx.x >> 5)) * L.per_warp + L.pixel;
     bool on = L.pixel < L.per_warp && i < n_px;
@@ -334,7 +346,7 @@ __global__ void __launch_bounds__(kGradThreads) k_gn_refine(const __grid_constan
         th[0] = d0; th[1] = n[0] / len; th[2] = n[1] / len;
     }
     if (!__any_sync(0xffffffffu, on)) return;
-    const RefPatch P = ref_patch(a, x, y, on, L, smem);
+    const RefPatch P = ref_patch(a, x, y, on, L, patch_of(L, smem));
     enum { kStart, kGradient, kTrial };
     int turn = kStart, it = 0, attempt = 0;
     bool active = on, mine = on, refined = false;
@@ -422,6 +434,22 @@ static int grad_blocks(size_t n, int S) {
     return (int)((n + per_block - 1) / per_block);
 }
 
+// Views that the lanes of a warp take side by side.  More than 16 go in two rows of blocks: a warp that
+// gathers from more images of over a megabyte each takes up to three times as long (10,000 x 100 pairs, 16
+// images 22 ns a warp, 17 lanes of one pixel 17, 20 lanes 34, 31 lanes 78), and 17 to 31 lanes of one pixel
+// leave the others idle.  100,000 pixels with 17 views took 1632 us a call and take 1202, with 31 views 7467
+// and 2009.
+static int grad_views(int S) { return S <= 16 ? S : (S + 1) / 2; }
+
+static void launch_cost_grad(const RunArgs& a, const SrcImages& si, int n, const int32_t* px, const float* theta,
+                             float* cost, float* grad, cudaStream_t st) {
+    const int per = grad_views(a.S);
+    const dim3 grid(grad_blocks(n, per), (a.S + per - 1) / per);
+    const bool own = per == 1;
+    auto k = own ? k_cost_grad<true> : k_cost_grad<false>;
+    k<<<grid, kGradThreads, grad_smem(per, own), st>>>(a, si, per, n, px, theta, cost, grad);
+}
+
 // Resets the self-check counter before a launch and reads it after one.
 static cudaError_t grad_oob_reset(cudaStream_t st) {
     const unsigned int zero = 0;
@@ -471,8 +499,7 @@ int Ctx::eval_cost_grad(int ref, const int32_t* srcs, int n_src, const hpm_param
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_th, theta, (size_t)n * 12, cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return cuda_fail(e, "upload hypotheses");
     if ((e = grad_oob_reset(stream)) != cudaSuccess) return cuda_fail(e, "self-check reset");
-    k_cost_grad<<<grad_blocks(n, a.S), kGradThreads, grad_smem(a.S), stream>>>(a, si, n, d_px, d_th, d_c,
-                                                                              grad ? d_g : nullptr);
+    launch_cost_grad(a, si, n, d_px, d_th, d_c, grad ? d_g : nullptr, stream);
     ++launches;
     unsigned int oob = 0;
     if ((e = grad_oob_read(stream, &oob)) != cudaSuccess) return cuda_fail(e, "cost gradient");
@@ -498,8 +525,7 @@ int Ctx::eval_cost_grad_device(int ref, const int32_t* srcs, int n_src, const hp
     cudaError_t e;
     if ((e = grad_oob_reset(stream)) != cudaSuccess) return cuda_fail(e, "self-check reset");
     // pixels outside the reference image are skipped and counted by the kernel (no host copy to check them)
-    k_cost_grad<<<grad_blocks(n, a.S), kGradThreads, grad_smem(a.S), stream>>>(a, si, n, d_px, d_theta, d_cost,
-                                                                              d_grad);
+    launch_cost_grad(a, si, n, d_px, d_theta, d_cost, d_grad, stream);
     ++launches;
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "cost gradient launch");
     unsigned int oob = 0;
@@ -526,7 +552,7 @@ int Ctx::gn_refine(int ref, const int32_t* srcs, int n_src, const hpm_params* pa
     cudaError_t e = ensure_map(ref, HPM_MAP_COST, v.w, v.h);
     if (e != cudaSuccess) return cuda_fail(e, "alloc cost map");
     if ((e = grad_oob_reset(stream)) != cudaSuccess) return cuda_fail(e, "self-check reset");
-    k_gn_refine<<<grad_blocks((size_t)v.w * v.h, a.S), kGradThreads, grad_smem(a.S), stream>>>(
+    k_gn_refine<<<grad_blocks((size_t)v.w * v.h, a.S), kGradThreads, grad_smem(a.S, false), stream>>>(
         a, si, steps, dm.ptr, nm.ptr, v.maps[HPM_MAP_COST].ptr, (size_t)v.w * v.h);
     ++launches;
     e = cudaGetLastError();
