@@ -78,8 +78,10 @@ Ctx::~Ctx() {
         if (v.tex) cudaDestroyTextureObject(v.tex);
         if (v.arr) cudaFreeArray(v.arr);
         if (v.bytes) cudaFree(v.bytes);
-        if (v.tex8) cudaDestroyTextureObject(v.tex8);
-        if (v.arr8) cudaFreeArray(v.arr8);
+        for (auto& b : v.arr8) {
+            if (b.tex) cudaDestroyTextureObject(b.tex);
+            if (b.arr) cudaFreeArray(b.arr);
+        }
         if (v.gray) cudaFree(v.gray);
         for (auto& m : v.maps) if (m.ptr) cudaFree(m.ptr);
         if (v.canny) cudaFree(v.canny);

@@ -25,6 +25,16 @@ struct DevMap {
     int w = 0, h = 0, ch = 1;
 };
 
+// An 8-bit array of one size and its texture.  A view keeps those of its last sizes, since a reconstruction
+// takes every view through its levels again and again and an allocation takes as long as the rest of a level.
+struct ByteArray {
+    cudaArray_t arr = nullptr;
+    cudaTextureObject_t tex = 0;
+    int w = 0, h = 0, mode = -1;
+    uint32_t used = 0;  // ViewState::arr8_uses at the last use
+};
+constexpr int kByteArrays = 4;
+
 struct ViewState {
     int w = 0, h = 0;
     hpm_camera cam{};
@@ -40,9 +50,9 @@ struct ViewState {
     bool bytes_current = false;  // they are those of the current image
     int64_t bytes_credit = 0;    // what its runs as the reference would have saved since the image came
     // 8-bit texture of an F32 image of whole levels, which the half-sweeps sample
-    cudaArray_t arr8 = nullptr;
+    ByteArray arr8[kByteArrays];
+    uint32_t arr8_uses = 0;
     cudaTextureObject_t tex8 = 0;
-    int arr8_w = 0, arr8_h = 0, arr8_mode = -1;
     bool bytes_bound = false;  // tex8 holds the current image
     DevMap maps[kNumMaps];
     uint8_t* canny = nullptr;

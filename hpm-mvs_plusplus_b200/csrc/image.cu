@@ -52,11 +52,15 @@ __global__ void k_resize_u8c3(const uint8_t* __restrict__ src, int sw, int sh, u
     }
 }
 
-__global__ void k_gray(const uint8_t* __restrict__ bgr, int n, float* __restrict__ gray) {
+// The grey levels as floats and, where a copy is wanted, as bytes.
+__global__ void k_gray(const uint8_t* __restrict__ bgr, int n, float* __restrict__ gray,
+                       uint8_t* __restrict__ bytes) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int b = bgr[3 * (size_t)i], g = bgr[3 * (size_t)i + 1], r = bgr[3 * (size_t)i + 2];
-    gray[i] = (float)((b * 7470 + g * 38470 + r * 19596 + (1 << 15)) >> 16);
+    const int level = (b * 7470 + g * 38470 + r * 19596 + (1 << 15)) >> 16;
+    gray[i] = (float)level;
+    if (bytes) bytes[i] = (uint8_t)level;
 }
 
 // Sobel 3x3 (replicated border), strongest channel by |dx|+|dy| (first on ties),
@@ -185,15 +189,18 @@ int Ctx::prepare_level_image(int view, int w, int h, const hpm_camera& cam) {
     v.color_h = h;
     e = ensure_i(v.gray, v.gray_cap, n);
     if (e != cudaSuccess) return cuda_fail(e, "alloc grey");
-    k_gray<<<(int)((n + 255) / 256), 256, 0, stream>>>(v.color, (int)n, v.gray);
-    ++launches;
     new_image(view, 1);
+    if (v.whole_levels == 1 && ensure_i(v.bytes, v.bytes_cap, n) != cudaSuccess) no_bytes(view);
+    v.bytes_current = v.whole_levels == 1;
+    k_gray<<<(int)((n + 255) / 256), 256, 0, stream>>>(v.color, (int)n, v.gray, v.bytes_current ? v.bytes : nullptr);
+    ++launches;
     v.w = w;
     v.h = h;
     v.cam = cam;
     v.cam.width = w;
     v.cam.height = h;
     int rc = bind_texture(view);
+    if (!rc && v.bytes_current && v.arr_fmt == HPM_TEX_F32) rc = bind_bytes(view);
     if (rc) return rc;
     return canny_view(view);
 }

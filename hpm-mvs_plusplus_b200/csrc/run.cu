@@ -93,9 +93,9 @@ static cudaError_t make_texture(cudaArray_t arr, int addr_mode, cudaTextureReadM
     return cudaCreateTextureObject(tex, &rd, &td, nullptr);
 }
 
-// 8-bit copies of a run's images of whole levels 0..255, as every image made by hpm_prepare_level is:
-// bytes of the reference, and 8-bit textures of the sources that have float ones.  Images from hpm_set_view
-// are looked at once for it, for which the host waits.  The unit filters with weights of 1/256, so an F32
+// 8-bit copies of a run's images of whole levels 0..255: bytes of the reference, and 8-bit textures of the
+// sources that have float ones.  hpm_prepare_level makes them with the level's image; images from
+// hpm_set_view are looked at once, for which the host waits.  The unit filters with weights of 1/256, so an F32
 // fetch is a whole multiple N of 1/256 level, N <= 255 * 256, and an 8-bit fetch is N / 65280 rounded
 // to a multiple of 1/65535: fetch * 65280 lies within 0.4999 of N, and rounding it to the nearest
 // integer gives N, hence the F32 fetch times 256, for every N (tests/test_gpu_whole_levels.py).  A
@@ -179,24 +179,39 @@ int Ctx::no_bytes(int view) {
 // The 8-bit texture of a view whose bytes are current.
 int Ctx::bind_bytes(int view) {
     ViewState& v = views[view];
-    cudaError_t e;
-    if (!v.arr8 || !v.tex8 || v.arr8_w != v.w || v.arr8_h != v.h || v.arr8_mode != v.arr_mode) {
-        if (v.tex8) { cudaDestroyTextureObject(v.tex8); v.tex8 = 0; }
-        if (v.arr8 && (v.arr8_w != v.w || v.arr8_h != v.h)) {
-            cudaFreeArray(v.arr8);
-            v.arr8 = nullptr;
-        }
-        if (!v.arr8) {
-            const cudaChannelFormatDesc fd = cudaCreateChannelDesc(8, 0, 0, 0, cudaChannelFormatKindUnsigned);
-            if ((e = cudaMallocArray(&v.arr8, &fd, v.w, v.h)) != cudaSuccess) return no_bytes(view);
-            v.arr8_w = v.w; v.arr8_h = v.h;
-        }
-        if ((e = make_texture(v.arr8, v.arr_mode, cudaReadModeNormalizedFloat, &v.tex8)) != cudaSuccess)
-            return no_bytes(view);
-        v.arr8_mode = v.arr_mode;
+    cudaError_t e = cudaSuccess;
+    ByteArray* b = v.arr8;
+    for (auto& other : v.arr8) {  // the one of this size, or the longest unused
+        if (other.arr && other.w == v.w && other.h == v.h) { b = &other; break; }
+        if (other.used < b->used) b = &other;
     }
-    e = cudaMemcpy2DToArrayAsync(v.arr8, 0, 0, v.bytes, (size_t)v.w, (size_t)v.w, v.h, cudaMemcpyDeviceToDevice, stream);
+    const bool sized = b->arr && b->w == v.w && b->h == v.h;
+    if (b->tex && (!sized || b->mode != v.arr_mode)) {
+        if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_fail(e, "byte image");  // runs may sample it
+        cudaDestroyTextureObject(b->tex);
+        b->tex = 0;
+    }
+    if (!sized) {
+        if (b->arr) cudaFreeArray(b->arr);
+        b->arr = nullptr;
+        const cudaChannelFormatDesc fd = cudaCreateChannelDesc(8, 0, 0, 0, cudaChannelFormatKindUnsigned);
+        if (cudaMallocArray(&b->arr, &fd, v.w, v.h) != cudaSuccess) {
+            b->arr = nullptr;
+            return no_bytes(view);
+        }
+        b->w = v.w; b->h = v.h;
+    }
+    if (!b->tex) {
+        if (make_texture(b->arr, v.arr_mode, cudaReadModeNormalizedFloat, &b->tex) != cudaSuccess) {
+            b->tex = 0;
+            return no_bytes(view);
+        }
+        b->mode = v.arr_mode;
+    }
+    e = cudaMemcpy2DToArrayAsync(b->arr, 0, 0, v.bytes, (size_t)v.w, (size_t)v.w, v.h, cudaMemcpyDeviceToDevice, stream);
     if (e != cudaSuccess) return cuda_fail(e, "copy byte image to array");
+    b->used = ++v.arr8_uses;
+    v.tex8 = b->tex;
     v.bytes_bound = true;
     return HPM_OK;
 }

@@ -48,3 +48,34 @@ def test_runs_in_turn_match_oracle(turns, upload, batched):
                 for name, a, b in zip(("depth", "normal", "cost"), got,
                                       _oracle(cams, grays, own, ref, srcs, params, k)):
                     assert _same(a, np.ascontiguousarray(b)), (image, k, name)
+
+
+@pytest.mark.parametrize("address_mode", [0, 1])
+def test_views_through_more_sizes_than_are_kept(address_mode):
+    """Level images of six sizes in turn, twice: a view keeps the 8-bit arrays of its last four sizes."""
+    sc, cams, _ = _views(3, 96, 72, seed=92)
+    sizes = [(96, 72), (48, 36), (64, 48), (33, 25), (80, 60), (41, 52)]
+    want = {}
+    with hpm_b200.Context(0) as kept:
+        kept.set_address_mode(address_mode)
+        for i, v in enumerate(sc.views):
+            kept.set_image(i, v.image)
+        for turn, (w, h) in enumerate(sizes + sizes[::-1] + sizes[:2] * 2):
+            for fresh in (True, False):
+                if fresh and (w, h) in want:
+                    continue
+                ctx = hpm_b200.Context(0) if fresh else kept
+                if fresh:
+                    ctx.set_address_mode(address_mode)
+                    for i, v in enumerate(sc.views):
+                        ctx.set_image(i, v.image)
+                for i, c in enumerate(cams):
+                    ctx.prepare_level(i, w, h, c.scaled(w, h, 96, 72))
+                params = hpm_b200.Params.make(3, *hpm_b200.widened_range(cams[0]))
+                ctx.run_patchmatch(0, [1, 2], params, seed=3)
+                maps = [ctx.get_map(0, m) for m in (hpm_b200.MAP_DEPTH, hpm_b200.MAP_NORMAL, hpm_b200.MAP_COST)]
+                if fresh:
+                    ctx.close()
+                    want[(w, h)] = maps
+                else:
+                    assert all(_same(a, b) for a, b in zip(maps, want[(w, h)])), (turn, w, h)
