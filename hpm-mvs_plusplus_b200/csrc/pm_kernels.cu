@@ -506,7 +506,7 @@ __device__ __forceinline__ void init_pixel(const RunArgs& a, const InitScratch<N
 // byte textures and the weight table, against 1.50 with an inlined copy of the NCC per mode
 template <int NS, int BLK, bool CNT>
 __global__ void __launch_bounds__(BLK, kSweepBlocks) k_random_init(const __grid_constant__ RunArgs a) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const InitScratch<NS, BLK> s{ smem + tid };
     init_pixel<NS, BLK, CNT>(a, s, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y);
@@ -538,7 +538,7 @@ __device__ __forceinline__ int batch_run_of(const int* __restrict__ tile_start, 
 template <int NS, int BLK, bool CNT>
 __global__ void __launch_bounds__(BLK, kSweepBlocks) k_random_init_batch(const RunArgs* __restrict__ args,
                                                            const int* __restrict__ tile_start, int n) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const InitScratch<NS, BLK> s{ smem + tid };
     const int total = __ldg(tile_start + n);
@@ -1150,6 +1150,7 @@ __device__ __forceinline__ void sweep_pixel(const RunArgs& a, float* smem_column
 // before any returns: the geometric modes (a prior run may be one) end it with a barrier.
 template <int NS, int BLK>
 __device__ __forceinline__ GeomView* load_geom_views(const RunArgs& a, float* smem, int tid) {
+    static_assert(Scratch<NS, BLK>::kWords * BLK % 4 == 0, "GeomView's alignment");
     GeomView* views = reinterpret_cast<GeomView*>(smem + Scratch<NS, BLK>::kWords * BLK);
     if (a.prm.mode & HPM_MODE_GEOM) {
         for (int j = tid; j < a.S; j += blockDim.x * blockDim.y) {
@@ -1171,7 +1172,7 @@ __device__ __forceinline__ GeomView* load_geom_views(const RunArgs& a, float* sm
 template <int NS, int BLK, bool MAND, bool CNT>
 __global__ void __launch_bounds__(BLK, kSweepBlocks) k_half_sweep(const __grid_constant__ RunArgs a, int color, int iter,
                                                                     int first_pair, int last_pair) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const GeomView* views = load_geom_views<NS, BLK>(a, smem, tid);
     const int pair = first_pair + blockIdx.y * blockDim.y + threadIdx.y;
@@ -1187,7 +1188,7 @@ template <int NS, int BLK, bool CNT>
 __global__ void __launch_bounds__(BLK, kSweepBlocks) k_half_sweep_listed(const __grid_constant__ RunArgs a,
                                                                          int color, int iter, int first_pair,
                                                                          int last_pair) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const GeomView* views = load_geom_views<NS, BLK>(a, smem, tid);
     const int pair = first_pair + blockIdx.y * blockDim.y + threadIdx.y;
@@ -1234,7 +1235,7 @@ template <int NS, int BLK, bool CNT>
 __global__ void __launch_bounds__(BLK, kSweepBlocks)
     k_half_sweep_batch_listed(const RunArgs* __restrict__ args, const int* __restrict__ tile_start, int n,
                               int color, int iter) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const int total = __ldg(tile_start + n);
     for (int b = __ldg(tile_start) + blockIdx.x; b < total; b += gridDim.x) {
@@ -1257,7 +1258,7 @@ template <int NS, int BLK, bool MAND, bool CNT>
 __global__ void __launch_bounds__(BLK, kSweepBlocks)
     k_half_sweep_batch(const RunArgs* __restrict__ args, const int* __restrict__ tile_start, int n, int color,
                        int iter) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const int total = __ldg(tile_start + n);
     for (int b = __ldg(tile_start) + blockIdx.x; b < total; b += gridDim.x) {
