@@ -589,7 +589,7 @@ class Context:
         return int(self.lib.hpm_launch_count(self.h))
 
     def stream_handle(self) -> int:
-        """The cudaStream_t all of this context's work runs on."""
+        """The cudaStream_t that orders this context's work (half-sweeps also use streams joined to it)."""
         s = ctypes.c_void_p()
         self._check(self.lib.hpm_get_stream(self.h, ctypes.byref(s)), "hpm_get_stream")
         return int(s.value or 0)

@@ -8,18 +8,19 @@
 // stage is one launch whose blocks are the tiles of all views (pm_kernels.cu,
 // k_random_init_batch / k_half_sweep_batch), so the last wave of one view no
 // longer idles the GPU; the half-sweeps go as two such launches, of half the
-// runs each, on two streams (launch_batch_sweeps).  Per-run setup (hypothesis reload, packing) and the
-// hand-off of the results are the single-run code paths of run.cu, applied to
-// per-run slices of resident batch buffers.
+// runs each, on two streams (launch_batch_sweeps).  Per-run setup (hypothesis
+// reload, packing) and the hand-off of the results are the single-run code
+// paths of run.cu, applied to per-run slices of resident batch buffers.
 //
 // Launch shapes of the half-sweep (block width 32, 16 or 8 pixels; one block
 // per tile or a persistent grid; or, for views large enough to fill the GPU
 // alone, one single-view launch per run, stage by stage) give the same
 // results; the autotuner times them once per (source count, mode, size class)
 // on a snapshot of the batch's state and restores the state before the real
-// run.  With HPM_BATCH_GRAPH the
-// initialisation and the half-sweeps are captured once per batch shape in a
-// CUDA graph and replayed.
+// run.  It times one half-sweep of all runs on one stream; the shape it picks
+// then runs in two groups (launch_batch_sweeps), except the single-view shape.
+// With HPM_BATCH_GRAPH the initialisation and the half-sweeps are captured
+// once per batch shape in a CUDA graph and replayed.
 #include "ctx.hpp"
 
 #include <algorithm>
@@ -131,7 +132,8 @@ int Ctx::tune_batch(const BatchLaunch& base, int n, size_t total_px, uint64_t ke
     if (!rc) {
         cudaEventRecord(t0, stream);
         for (int k = 0; k < n && !rc; ++k) {
-            if ((e = launch_half_sweep(h_bargs[k], 0, 0, 0, h_bargs[k].cover_pairs, stream)) != cudaSuccess) rc = cuda_fail(e, "autotuner launch");
+            e = launch_half_sweep(h_bargs[k], 0, 0, 0, h_bargs[k].cover_pairs, stream);
+            if (e != cudaSuccess) rc = cuda_fail(e, "autotuner launch");
             ++launches;
         }
         cudaEventRecord(t1, stream);

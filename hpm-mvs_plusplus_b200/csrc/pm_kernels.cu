@@ -24,7 +24,7 @@
 // in registers, and the warps stand at different places), and the latency of
 // the serial parts around the NCCs.  Six half-sweeps of one run, ms, S = 10,
 // before and after each change, all with the same bits:
-//   code size 291 -> 105 KB (loops and calls outside the NCC):
+//   code size 291 -> 130 KB, 124 since (loops and calls outside the NCC):
 //                      1600x1200 mandatory 48.5 -> 42.0, prior 31.2 -> 22.8
 //   8-bit textures:    800x600 photometric 13.4 -> 11.0 (2.2 -> 1.4 passes a quad)
 //   pairs of samples in one instruction (f32x2):  mandatory 42.0 -> 39.0
@@ -64,12 +64,12 @@ struct alignas(16) GeomView {
 };
 static_assert(sizeof(GeomView) == 112, "seven 16-byte loads");
 
-// Per-thread scratch of a half-sweep, in blocks of at most BLK threads.  The cost rows of the eight directions are written once, an NCC
-// apart, and read once, by view selection: they stream through the thread's local memory, so that
-// shared memory (view weights, final costs, candidate positions) leaves the L1 to the textures and
-// the registers alone bound the resident warps.  After view selection the rows' words hold the
-// refinement's candidates and the state they are tested against, which would otherwise sit in
-// registers across every NCC.
+// Per-thread scratch of a half-sweep, in blocks of at most BLK threads.  The cost rows of the eight
+// directions are written once, an NCC apart, and read once, by view selection: they stream through the
+// thread's local memory, so that shared memory (view weights, final costs, candidate positions) leaves
+// the L1 to the textures and the registers alone bound the resident warps.  After view selection the
+// rows' words hold the refinement's candidates and the state they are tested against, which would
+// otherwise sit in registers across every NCC.
 template <int NS, int BLK>
 struct Scratch {
     float* base;   // smem + threadIdx linear
@@ -1337,9 +1337,9 @@ static bool one_wave(int blocks) {
 }
 
 // Row pairs of a block, one warp each.  An image of less than one wave of four-warp blocks runs in
-// two-warp blocks, which spread over the SMs more evenly: 320x240 has 300 blocks of four warps for
+// two-warp blocks, which spread over the SMs more evenly: 320x240 has 320 blocks of four warps for
 // 3 x 148 places, and its half-sweeps take 142 instead of 155 us (photometric, 4 sources), 297 instead
-// of 313 (prior, 10 sources).  From 400x300 on (494 blocks) four warps are as fast or faster, since the
+// of 313 (prior, 10 sources).  From 400x300 on (520 blocks) four warps are as fast or faster, since the
 // warps of a block share what they fetch.
 static int block_pairs(const RunArgs& a) { return one_wave(blocks_of_four(a)) ? 2 : 4; }
 

@@ -19,8 +19,8 @@ struct ViewBasis {
 // as a __grid_constant__ kernel parameter (about 6 KB).
 struct RunArgs {
     hpm_camera cams[32];            // 0 = reference
-    ViewBasis basis[32];
-    ViewBasis fwd[32], bwd[32];     // geometric cost: point transfer reference -> source j+1 and back            // homography basis of source j+1 w.r.t. the reference
+    ViewBasis basis[32];            // homography basis of source j+1 w.r.t. the reference
+    ViewBasis fwd[32], bwd[32];     // geometric cost: point transfer reference -> source j+1 and back
     float kinv[4];                  // 1/fx, 1/fy, cx/fx, cy/fy of the reference camera
     float var_s_min;                // flat-source threshold: 1e-5 (HPM.cu:434) in the textures' grey units
     int ncc_shift;                  // 1: shifted NCC moments (precision form); 0: the plain arithmetic

@@ -507,9 +507,9 @@ bool Ctx::ensure_bands() {
 // rows or more can start half-sweep k + 1 when it and its two neighbours have finished half-sweep k.
 // With four bands on streams of their own, one half-sweep's last, partly filled wave runs beside the
 // next one's first, which six launches in a row cannot.  One half-sweep on B200, 10 sources, one launch
-// and in bands: photometric 400x300 (494 blocks, 444 places) 92 and 85 us, 800x600 (1875 blocks) 281 and
-// 255, 1600x1200 (7500) 1106 and 1077; mandatory 259 and 231 at 800x600; prior 157 and 131.  Three to
-// eight bands differ by less than 3 %.  An image of one wave has no such tail: bands cost 320x240 (300
+// and in bands: photometric 400x300 (520 blocks, 444 places) 92 and 85 us, 800x600 (1900 blocks) 281 and
+// 255, 1600x1200 (7600) 1106 and 1077; mandatory 259 and 231 at 800x600; prior 157 and 131.  Three to
+// eight bands differ by less than 3 %.  An image of one wave has no such tail: bands cost 320x240 (320
 // blocks) 4 %, so it keeps one launch, as does a context without streams to spare.
 int Ctx::launch_sweeps(const RunArgs& a, int n_half_sweeps) {
     constexpr int kBandPairs = 16;  // shortest band, in row pairs

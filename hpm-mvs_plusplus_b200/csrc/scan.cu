@@ -26,10 +26,11 @@
 // first of them counts for the rounds and the last for the confidence.  A
 // counted pixel is nearly always accepted itself, so the first is q; the other
 // ends are looked up in bitmaps (one per source, one of accepted pixels), 32
-// pixels at a time, and 1024 at a time where a summary word shows nothing set.  (Prefix maxima of the last counted pixel for every
-// pixel and source, ten words a pixel written and read again in every round,
-// took two thirds of a scan: 11 views of 1600x1200 with 10 sources took 33.9 ms
-// and take 11.4.  A further summary level of 32 chunks changed nothing.)
+// pixels at a time, and 1024 at a time where a summary word shows nothing set.
+// (Prefix maxima of the last counted pixel for every pixel and source, ten
+// words a pixel written and read again in every round, took two thirds of a
+// scan: 11 views of 1600x1200 with 10 sources took 33.9 ms and take 11.4.  A
+// further summary level of 32 chunks changed nothing.)
 // Marks carry the round that set them, so no round clears them.
 //
 // Rounds are launched as many as the previous view needed; each kernel returns
@@ -622,7 +623,8 @@ int Ctx::consistency_scan(int mode, int n_views, const int32_t* src_off, const i
     const size_t mark_stride = (max_pix + 3) & ~size_t(3);
     const size_t mark_bytes = al(8 * mark_stride * ng);
     const size_t wbytes = 2 * al(4 * stride_max * ng) + 3 * al(4 * stride_max) + al(4 * stride_max / kScanBlock) +
-                          al(4 * stride_max / kScanBlock) + al(4 * (ng + 1) * (stride_max / 32)) + (mode == 0 ? 2 : 1) * mark_bytes + al(64) +
+                          al(4 * stride_max / kScanBlock) + al(4 * (ng + 1) * (stride_max / 32)) +
+                          (mode == 0 ? 2 : 1) * mark_bytes + al(64) +
                           al(4 * kMaxScanIterations);
     e = ensure_dev(scan_work, scan_work_cap, wbytes);
     if (e != cudaSuccess) return cuda_fail(e, "alloc scan work");

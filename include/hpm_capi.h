@@ -12,8 +12,8 @@
  * Conventions: plain pointers and sizes, host memory unless a name says
  * `_device`; every function returns 0 on success or a positive HPM_E* code and
  * never exits or throws (the reference calls exit(EXIT_FAILURE), HPM.cpp:68-76);
- * hpm_last_error() describes the last failure.  One CUDA stream per context;
- * calls on one context are not thread-safe.
+ * hpm_last_error() describes the last failure.  Each context has one CUDA stream
+ * (hpm_get_stream) that orders its work; calls on one context are not thread-safe.
  */
 #ifndef HPM_CAPI_H
 #define HPM_CAPI_H
@@ -103,7 +103,12 @@ int hpm_set_prior(hpm_ctx *ctx, int view, const float *planes, const uint8_t *ma
  * Outputs: DEPTH (DEPTH_GEOM in geom/mandatory passes), NORMAL, COST and, when
  * neither prior nor mandatory, TEXTURE0 + texture_level.
  * depth_min/max in params are the widened range of HPM.cpp:685-686.  `seed`
- * keys the counter-based random stream of this run. */
+ * keys the counter-based random stream of this run.
+ * The call queues the run and returns.  A run on images from hpm_set_view may
+ * look once whether their grey levels are whole numbers, which it then samples
+ * as bytes with the same result: it waits for that.  Not under stream capture.
+ * GEOM with HIERARCHY and without PRIOR is refused: each starts from maps of
+ * its own. */
 int hpm_run_patchmatch(hpm_ctx *ctx, int ref, const int32_t *srcs, int n_src, const hpm_params *params,
                        int texture_level, uint64_t seed);
 
@@ -162,8 +167,8 @@ int hpm_eval_costs_noalloc(hpm_ctx *ctx, int ref, const int32_t *srcs, int n_src
  * ny) in the reference camera frame with nz = -sqrt(1 - nx^2 - ny^2):
  * cost[k*n_src + j] and, when grad is not null, grad[(k*n_src + j)*3 + a] =
  * d cost / d theta_a.  Costs of 2 (out-of-image centre, flat patch) and
- * clamped costs have zero gradient.  The warped samples are recomputed, not
- * stored. */
+ * clamped costs have zero gradient.  A view's 36 warped samples are kept for
+ * its gradient, whose image derivatives sample it once more. */
 int hpm_eval_cost_grad(hpm_ctx *ctx, int ref, const int32_t *srcs, int n_src, const hpm_params *params, int n,
                        const int32_t *px, const float *theta, float *cost, float *grad);
 
@@ -321,11 +326,14 @@ int hpm_synchronize(hpm_ctx *ctx);
 /* ---- measurement (no reference counterpart; the reference has only its
  * wall-clock timer, main.cpp:10-23) ---- */
 
-/* The CUDA stream all work of the context is issued on (a cudaStream_t), so a
- * caller can record its own events around calls. */
+/* The CUDA stream that orders the context's work (a cudaStream_t), so a caller
+ * can record its own events around calls.  Half-sweeps also run on streams of
+ * the context's own, which wait for this one before them and which this one
+ * waits for after them. */
 int hpm_get_stream(hpm_ctx *ctx, void **stream);
 
-#define HPM_PROFILE_TIMING 1 /* CUDA events around every PatchMatch kernel launch */
+#define HPM_PROFILE_TIMING 1 /* CUDA events around the initialisation, and around the half-sweeps of a run
+                                or batch: together where they overlap, each one otherwise */
 #define HPM_PROFILE_COUNT 2  /* count (hypothesis, source view) cost evaluations */
 
 typedef struct hpm_profile {
@@ -346,7 +354,7 @@ typedef struct hpm_profile {
 } hpm_profile;
 
 /* Turns profiling on (flags) or off (0).  Timing adds two event records per
- * launch; counting adds one atomic per costed hypothesis. */
+ * timed part; counting adds one atomic per costed hypothesis. */
 int hpm_profile_enable(hpm_ctx *ctx, int flags);
 
 /* Waits for the context's work, returns what was gathered since the last read
